@@ -612,8 +612,7 @@ StepArgs<R> make_args(grains_gpu_ctx* c) {
   a.res_t = (typename Vec4<R>::type*)c->res_t;
   a.work = c->work;
   a.work_n = c->work_n;
-  // the signed-volume GJK keeps its runs in the pair kernel
-  a.gjk_out = c->gjk_sv ? nullptr : c->gjk_out;
+  a.gjk_out = c->gjk_out;
   a.gjk_next = c->gjk_next;
   a.gjk_order = c->gjk_order;
   a.gjk_bins = c->gjk_bins;
@@ -2441,7 +2440,7 @@ int grains_gpu_launches_per_step(grains_gpu_ctx* c, int64_t* launches) {
   // (the GJK kernel of convex scenarios,) pairs, sums with the kick, and the
   // obstacle move when obstacles move; the gather runs one step in
   // gather_every on top
-  *launches = launches_per_middle_step() + (c->has_convex && !c->gjk_sv ? 3 : 0) + (c->n_moving > 0 ? 1 : 0) +
+  *launches = launches_per_middle_step() + (c->has_convex ? 3 : 0) + (c->n_moving > 0 ? 1 : 0) +
                (c->n_force_obs > 0 ? 1 : 0);
   return 0;
 }

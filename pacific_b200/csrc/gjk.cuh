@@ -42,6 +42,13 @@
 #include "device_state.h"
 #include "sphere_contact.cuh"
 
+// rare paths, kept out of the registers of the code around them
+#if defined(__CUDACC__)
+#define GG_COLD static __host__ __device__ __noinline__
+#else
+#define GG_COLD inline
+#endif
+
 namespace gg {
 
 struct BodyRef {
@@ -221,142 +228,150 @@ GG_HD V3<T> gjk_direction(bool accel, int k, V3<T> d, V3<T> v, V3<T> w) {
   return v;
 }
 
-// The arrays of a Johnson GJK run, as a view of kGjkWords numbers `stride`
-// apart: the sub-determinants of every subset s of the 4-point simplex for
-// each of its points i (32 values, packed by subset: the entries of s start at
-// the number of point slots of the subsets below it), the dot products of the
-// simplex points (16), the points of A - B, and the support points of A and B
-// in their local frames (3 x 4 x 3).  A run on its own keeps them in a local
-// array (stride 1); the GJK kernel keeps those of its 64 threads interleaved
-// in shared memory (stride 64), so that a warp's accesses fall in distinct
-// banks.
-constexpr int kGjkWords = 32 + 16 + 36;
+// Johnson's sub-algorithm on a simplex of up to four points in fixed slots.
+// The subsets of the four slots are written out (masks known at compile time)
+// and selected by predicates, so that the points and sub-determinants stay in
+// registers and the lanes of a warp, whose simplexes differ in size and slots,
+// run the same instructions.  The subset loops it replaces kept the
+// sub-determinants in shared memory, walked the subsets by their bits and left
+// 10 of 32 lanes active.
+//
+// Every value is the one of the published recurrence with cached
+// sub-determinants, to the bit: a subset's determinants depend on the order in
+// which its points came only for three points (the reference point of the
+// difference is the lower of the two older points for the newest one, and the
+// other older point for these), so the three-point subsets with the newest
+// point are formed here, and the one without it, when the kept simplex has
+// three points, is that simplex (its determinants are kept with it); pairs are
+// symmetric, and all four points take slot order.
 template <typename T>
-struct GjkState {
-  T* base;
-  int stride;
-  GG_HD static int at(unsigned s, unsigned i) {
-    // sum of the sizes of the subsets 0 .. s-1, bytes of two constants
-    const unsigned long long lo = 0x0907050402010000ull, hi = 0x1C191614110F0D0Cull;
-    const unsigned start = unsigned((s < 8 ? lo >> (8 * s) : hi >> (8 * (s - 8))) & 0xffu);
-#if defined(__CUDA_ARCH__)
-    return int(start + __popc(s & ((1u << i) - 1u)));
-#else
-    return int(start + __builtin_popcount(s & ((1u << i) - 1u)));
-#endif
-  }
-  GG_HD T& det(unsigned s, unsigned i) const { return base[at(s, i) * stride]; }
-  GG_HD T& dp(unsigned i, unsigned j) const { return base[(32 + 4 * i + j) * stride]; }
-  GG_HD V3<T> vec(int k) const {  // k: 0-3 y, 4-7 p, 8-11 q
-    const T* b = base + (48 + 3 * k) * stride;
-    return v3<T>(b[0], b[stride], b[2 * stride]);
-  }
-  GG_HD void set_vec(int k, V3<T> v) const {
-    T* b = base + (48 + 3 * k) * stride;
-    b[0] = v.x;
-    b[stride] = v.y;
-    b[2 * stride] = v.z;
-  }
-  GG_HD V3<T> y(unsigned i) const { return vec(int(i)); }
-  GG_HD V3<T> p(unsigned i) const { return vec(4 + int(i)); }
-  GG_HD V3<T> q(unsigned i) const { return vec(8 + int(i)); }
+struct GjkSimplex {
+  unsigned bits;      // slots of the current simplex
+  unsigned all_bits;  // slots of the last iteration's candidate simplex
+  V3<T> y[4];         // points of A - B
+  T det[4];           // determinants of the current simplex by slot
 };
 
+// det[s][i]: the determinant of subset s for its slot i, of every subset of the
+// current simplex and the new point (slot `last`, already in y)
 template <typename T>
-GG_HD void gjk_det(unsigned bits, unsigned last, unsigned last_bit, unsigned all_bits, const GjkState<T>& g) {
-  const V3<T> yl = g.y(last);
-  for (unsigned i = 0, bit = 1; i < 4; ++i, bit <<= 1)
-    if (bits & bit) g.dp(i, last) = g.dp(last, i) = dot(g.y(i), yl);
-  g.dp(last, last) = dot(yl, yl);
-  g.det(last_bit, last) = T(1);
-  for (unsigned j = 0, sj = 1; j < 4; ++j, sj <<= 1) {
-    if (!(bits & sj)) continue;
-    unsigned s2 = sj | last_bit;
-    g.det(s2, j) = g.dp(last, last) - g.dp(last, j);
-    g.det(s2, last) = g.dp(j, j) - g.dp(j, last);
-    for (unsigned k = 0, sk = 1; k < j; ++k, sk <<= 1) {
-      if (!(bits & sk)) continue;
-      unsigned s3 = sk | s2;
-      g.det(s3, k) = g.det(s2, j) * (g.dp(j, j) - g.dp(j, k)) + g.det(s2, last) * (g.dp(last, j) - g.dp(last, k));
-      g.det(s3, j) = g.det(sk | last_bit, k) * (g.dp(k, k) - g.dp(k, j)) +
-                     g.det(sk | last_bit, last) * (g.dp(last, k) - g.dp(last, j));
-      g.det(s3, last) = g.det(sk | sj, k) * (g.dp(k, k) - g.dp(k, last)) +
-                        g.det(sk | sj, j) * (g.dp(j, k) - g.dp(j, last));
+GG_HD void gjk_dets(const GjkSimplex<T>& S, unsigned last, T (&det)[16][4]) {
+  T dp[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = i; j < 4; ++j) dp[i][j] = dp[j][i] = dot(S.y[i], S.y[j]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) det[1 << i][i] = T(1);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i != j) det[(1 << i) | (1 << j)][i] = dp[j][j] - dp[i][j];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {  // the triple without slot t: a < b < c
+    const int a = t == 0 ? 1 : 0, b = t <= 1 ? 2 : 1, c = t == 3 ? 2 : 3;
+    const int m = 15 ^ (1 << t), ab = (1 << a) | (1 << b), ac = (1 << a) | (1 << c), bc = (1 << b) | (1 << c);
+    // reference points: of a: b, or c when b is the newest; of b: a, or c when a is; of c: a, or b when a is
+    const bool bn = (int)last == b, an = (int)last == a;
+    const T ra_b = bn ? dp[b][c] : dp[b][b], ra_c = bn ? dp[c][c] : dp[c][b];
+    const T rb_a = an ? dp[a][c] : dp[a][a], rb_c = an ? dp[c][c] : dp[c][a];
+    const T rc_a = an ? dp[a][b] : dp[a][a], rc_b = an ? dp[b][b] : dp[b][a];
+    det[m][a] = det[bc][b] * (ra_b - dp[b][a]) + det[bc][c] * (ra_c - dp[c][a]);
+    det[m][b] = det[ac][a] * (rb_a - dp[a][b]) + det[ac][c] * (rb_c - dp[c][b]);
+    det[m][c] = det[ab][a] * (rc_a - dp[a][c]) + det[ab][b] * (rc_b - dp[b][c]);
+    if (S.bits == (unsigned)m) {
+      det[m][a] = S.det[a];
+      det[m][b] = S.det[b];
+      det[m][c] = S.det[c];
     }
   }
-  if (all_bits == 15) {
-    g.det(15, 0) = g.det(14, 1) * (g.dp(1, 1) - g.dp(1, 0)) + g.det(14, 2) * (g.dp(2, 1) - g.dp(2, 0)) +
-                   g.det(14, 3) * (g.dp(3, 1) - g.dp(3, 0));
-    g.det(15, 1) = g.det(13, 0) * (g.dp(0, 0) - g.dp(0, 1)) + g.det(13, 2) * (g.dp(2, 0) - g.dp(2, 1)) +
-                   g.det(13, 3) * (g.dp(3, 0) - g.dp(3, 1));
-    g.det(15, 2) = g.det(11, 0) * (g.dp(0, 0) - g.dp(0, 2)) + g.det(11, 1) * (g.dp(1, 0) - g.dp(1, 2)) +
-                   g.det(11, 3) * (g.dp(3, 0) - g.dp(3, 2));
-    g.det(15, 3) = g.det(7, 0) * (g.dp(0, 0) - g.dp(0, 3)) + g.det(7, 1) * (g.dp(1, 0) - g.dp(1, 3)) +
-                   g.det(7, 2) * (g.dp(2, 0) - g.dp(2, 3));
+  det[15][0] = det[14][1] * (dp[1][1] - dp[1][0]) + det[14][2] * (dp[2][1] - dp[2][0]) +
+               det[14][3] * (dp[3][1] - dp[3][0]);
+  det[15][1] = det[13][0] * (dp[0][0] - dp[0][1]) + det[13][2] * (dp[2][0] - dp[2][1]) +
+               det[13][3] * (dp[3][0] - dp[3][1]);
+  det[15][2] = det[11][0] * (dp[0][0] - dp[0][2]) + det[11][1] * (dp[1][0] - dp[1][2]) +
+               det[11][3] * (dp[3][0] - dp[3][2]);
+  det[15][3] = det[7][0] * (dp[0][0] - dp[0][3]) + det[7][1] * (dp[1][0] - dp[1][3]) +
+               det[7][2] * (dp[2][0] - dp[2][3]);
+}
+
+// The backup procedure: the closest of all proper subsets.  It ends a run, so
+// gjk_end calls it, out of the registers of the iteration.
+template <typename T>
+GG_COLD void gjk_backup(GjkSimplex<T>& S, unsigned last, V3<T>& v) {
+  T det[16][4];
+  gjk_dets(S, last, det);
+  const unsigned all = S.all_bits;
+  T least = T(INFINITY);
+#pragma unroll 1
+  for (int s = 15; s > 0; --s) {
+    bool proper = !(s & ~all);
+    T sum = T(0);
+    V3<T> u = v3<T>(T(0), T(0), T(0));
+    for (int i = 0; i < 4; ++i)
+      if (s & (1 << i)) {
+        if (s != (1 << i)) proper = proper && !(det[s][i] <= T(kEpsilon3));
+        sum += det[s][i];
+        u = u + sc(S.y[i], det[s][i]);
+      }
+    if (!proper) continue;
+    u = sc(u, T(1) / sum);
+    const T d2 = norm2(u);
+    if (d2 < least) {
+      least = d2;
+      S.bits = s;
+      v = u;
+      for (int i = 0; i < 4; ++i) S.det[i] = (s & (1 << i)) ? det[s][i] : T(0);
+    }
   }
 }
 
+// Finds the subset of the current simplex and the new point (slot `last`,
+// already in y) closest to the origin; false when none is valid (the backup
+// procedure then gives the answer).
 template <typename T>
-GG_HD bool gjk_valid(unsigned s, unsigned all_bits, const GjkState<T>& g) {
-  for (unsigned i = 0, bit = 1; i < 4; ++i, bit <<= 1) {
-    if (!(all_bits & bit)) continue;
-    if (s & bit) {
-      if (g.det(s, i) <= T(kEpsilon3)) return false;
-    } else if (g.det(s | bit, i) > T(0)) {
-      return false;
-    }
-  }
-  return true;
-}
-
-template <typename T>
-GG_HD V3<T> gjk_vector(unsigned bits, const GjkState<T>& g) {
-  T sum = T(0);
-  V3<T> v = v3<T>(T(0), T(0), T(0));
-  for (unsigned i = 0, bit = 1; i < 4; ++i, bit <<= 1)
-    if (bits & bit) {
-      sum += g.det(bits, i);
-      v = v + sc(g.y(i), g.det(bits, i));
-    }
-  return sc(v, T(1) / sum);
-}
-
-template <typename T>
-GG_HD bool gjk_proper(unsigned s, const GjkState<T>& g) {
-  for (unsigned i = 0, bit = 1; i < 4; ++i, bit <<= 1)
-    if ((s & bit) && g.det(s, i) <= T(kEpsilon3)) return false;
-  return true;
-}
-
-template <typename T>
-GG_HD bool gjk_closest(unsigned& bits, unsigned last, unsigned last_bit, unsigned all_bits, const GjkState<T>& g,
-                       V3<T>& v) {
-  gjk_det(bits, last, last_bit, all_bits, g);
-  // the non-empty subsets of bits in decreasing order (s = (s - 1) & bits
-  // steps from one subset to the next smaller one)
-  for (unsigned s = bits; s; s = (s - 1) & bits) {
-    if (gjk_valid(s | last_bit, all_bits, g)) {
-      bits = s | last_bit;
-      v = gjk_vector(bits, g);
-      return true;
-    }
-  }
-  if (gjk_valid(last_bit, all_bits, g)) {
-    bits = last_bit;
-    v = g.y(last);
-    return true;
-  }
-  T best = T(INFINITY);
-  for (unsigned s = all_bits; s; s = (s - 1) & all_bits) {  // backup procedure
-    if (gjk_proper(s, g)) {
-      V3<T> u = gjk_vector(s, g);
-      T d2 = norm2(u);
-      if (d2 < best) {
-        best = d2;
-        bits = s;
-        v = u;
+GG_HD bool gjk_closest(GjkSimplex<T>& S, unsigned last, V3<T>& v) {
+  const unsigned last_bit = 1u << last, all = S.bits | last_bit;
+  S.all_bits = all;
+  T det[16][4];
+  gjk_dets(S, last, det);
+  // the largest subset (as a number) with the newest point that is valid: its
+  // determinants are positive, and adding any other candidate point gives that
+  // point a determinant that is not
+  unsigned best = 0;
+#pragma unroll
+  for (int s = 1; s < 16; ++s) {
+    bool ok = (s & last_bit) && !(s & ~all);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (s & (1 << i)) {
+        if (s != (1 << i)) ok = ok && !(det[s][i] <= T(kEpsilon3));
+      } else {
+        ok = ok && !((all & (1u << i)) && det[s | (1 << i)][i] > T(0));
       }
     }
+    if (ok) best = s;
+  }
+  if (best) {
+    T sum = T(0);
+    V3<T> u = v3<T>(T(0), T(0), T(0)), ylast = u;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      T d = T(0);
+#pragma unroll
+      for (int s = 1; s < 16; ++s)
+        if ((s & (1 << i)) && best == (unsigned)s) d = det[s][i];
+      S.det[i] = d;
+      if (best & (1u << i)) {
+        sum += d;
+        u = u + sc(S.y[i], d);
+      }
+      if (last == (unsigned)i) ylast = S.y[i];
+    }
+    S.bits = best;
+    v = best == last_bit ? ylast : sc(u, T(1) / sum);
+    return true;
   }
   return false;
 }
@@ -379,19 +394,38 @@ struct GjkResult {
 // kernel interleaves the passes of different pairs on one thread.
 template <typename T>
 struct GjkRun {
-  unsigned bits, last, last_bit, all_bits;
-  GjkState<T> g;  // the run's arrays (the caller's storage)
+  GjkSimplex<T> S;
+  // the support points of A and B in their local frames by slot (2 x 4 x 3
+  // numbers, `stride` apart): storage of the caller's
+  T* points;
+  int stride;
   V3<T> v, w, d;
   T dist, lower, rel_error, abs_error;
   int num, exit_reason;
   bool accel;
+
+  GG_HD V3<T> point(int body, int slot) const {
+    const T* b = points + (12 * body + 3 * slot) * stride;
+    return v3<T>(b[0], b[stride], b[2 * stride]);
+  }
+  GG_HD void set_point(int body, int slot, V3<T> p) const {
+    T* b = points + (12 * body + 3 * slot) * stride;
+    b[0] = p.x;
+    b[stride] = p.y;
+    b[2 * stride] = p.z;
+  }
 };
+constexpr int kGjkWords = 24;  // numbers of GjkRun::points
 
 template <typename T>
 GG_HD void gjk_begin(GjkRun<T>& r, const LocalBody<T>& A, const LocalBody<T>& B, T rel_error,
                      const GjkStart<T>& st) {
-  r.bits = r.last = r.last_bit = r.all_bits = 0;
-  for (int i = 0; i < kGjkWords; ++i) r.g.base[i * r.g.stride] = T(0);
+  r.S.bits = r.S.all_bits = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    r.S.y[i] = v3<T>(T(0), T(0), T(0));
+    r.S.det[i] = T(0);
+  }
   r.rel_error = rel_error;
   r.abs_error = T(1.e-4) * rel_error;
   r.dist = gjk_first(A, B, st, r.v, r.w);
@@ -402,18 +436,17 @@ GG_HD void gjk_begin(GjkRun<T>& r, const LocalBody<T>& A, const LocalBody<T>& B,
   r.lower = -r.dist;
 }
 
+// the lowest free slot of a simplex of up to three points
+GG_HD unsigned gjk_free_slot(unsigned bits) {
+  return !(bits & 1) ? 0u : (!(bits & 2) ? 1u : (!(bits & 4) ? 2u : 3u));
+}
+
 // one pass of the loop; true when the run has ended
 template <typename T>
 GG_HD bool gjk_iterate(GjkRun<T>& r, const LocalBody<T>& A, const LocalBody<T>& B) {
-  if (!(r.bits < 15 && r.dist > T(kEpsilon2) && r.num < 1000)) return true;
+  if (!(r.S.bits < 15 && r.dist > T(kEpsilon2) && r.num < 1000)) return true;
   ++r.num;
-  r.last = 0;
-  r.last_bit = 1;
-  while (r.bits & r.last_bit) {
-    ++r.last;
-    r.last_bit <<= 1;
-  }
-  const unsigned last = r.last;
+  const unsigned last = gjk_free_slot(r.S.bits);
   r.d = gjk_direction(r.accel, r.num, r.d, r.v, r.w);
   V3<T> pl = support_local(A, lb_vecmat(-r.d, A));
   V3<T> ql = support_local(B, lb_vecmat(r.d, B));
@@ -423,8 +456,6 @@ GG_HD bool gjk_iterate(GjkRun<T>& r, const LocalBody<T>& A, const LocalBody<T>& 
   T mu = r.dist - sep;
   if (mu < r.dist * r.rel_error || mu < r.abs_error) {
     if (!r.accel || norm(r.d - r.v) < T(kEpsilon)) {
-      r.g.set_vec(4 + int(last), pl);
-      r.g.set_vec(8 + int(last), ql);
       r.exit_reason = 0;
       return true;
     }
@@ -434,22 +465,24 @@ GG_HD bool gjk_iterate(GjkRun<T>& r, const LocalBody<T>& A, const LocalBody<T>& 
     ql = support_local(B, lb_vecmat(r.v, B));
     r.w = lb_apply(A, pl) - lb_apply(B, ql);
   }
-  r.g.set_vec(4 + int(last), pl);
-  r.g.set_vec(8 + int(last), ql);
   bool degen = false;
-  for (unsigned i = 0, bit = 1; i < 4; ++i, bit <<= 1)
-    if (r.all_bits & bit) {
-      const V3<T> yi = r.g.y(i);
+#pragma unroll
+  for (unsigned i = 0; i < 4; ++i)
+    if (r.S.all_bits & (1u << i)) {
+      const V3<T> yi = r.S.y[i];
       if (yi.x == r.w.x && yi.y == r.w.y && yi.z == r.w.z) degen = true;
     }
   if (degen) {
     r.exit_reason = 1;
     return true;
   }
-  r.g.set_vec(int(last), r.w);
-  r.all_bits = r.bits | r.last_bit;
-  if (!gjk_closest(r.bits, last, r.last_bit, r.all_bits, r.g, r.v)) {
-    r.exit_reason = 2;
+  r.set_point(0, int(last), pl);
+  r.set_point(1, int(last), ql);
+#pragma unroll
+  for (unsigned i = 0; i < 4; ++i)
+    if (last == i) r.S.y[i] = r.w;
+  if (!gjk_closest(r.S, last, r.v)) {
+    r.exit_reason = 2;  // gjk_end runs the backup procedure
     return true;
   }
   r.dist = norm(r.v);
@@ -457,17 +490,25 @@ GG_HD bool gjk_iterate(GjkRun<T>& r, const LocalBody<T>& A, const LocalBody<T>& 
 }
 
 template <typename T>
-GG_HD GjkResult<T> gjk_end(const GjkRun<T>& r, const LocalBody<T>& A, const LocalBody<T>& B) {
+GG_HD GjkResult<T> gjk_end(GjkRun<T>& r, const LocalBody<T>& A, const LocalBody<T>& B) {
   GjkResult<T> out;
+  if (r.exit_reason == 2) {
+    GjkSimplex<T> S = r.S;  // the call's memory, not the run's registers
+    V3<T> v = r.v;
+    gjk_backup(S, gjk_free_slot(S.bits), v);
+    r.S = S;
+    r.v = v;
+  }
   T sum = T(0);
   const V3<T> zero = v3<T>(T(0), T(0), T(0));
   V3<T> pa = zero, pb = zero;
-  for (unsigned i = 0, bit = 1; i < 4; ++i, bit <<= 1)
-    if (r.bits & bit) {
-      const T di = r.g.det(r.bits, i);
+#pragma unroll
+  for (unsigned i = 0; i < 4; ++i)
+    if (r.S.bits & (1u << i)) {
+      const T di = r.S.det[i];
       sum += di;
-      pa = pa + sc(r.g.p(i), di);
-      pb = pb + sc(r.g.q(i), di);
+      pa = pa + sc(r.point(0, int(i)), di);
+      pb = pb + sc(r.point(1, int(i)), di);
     }
   T s = T(1) / sum;
   out.pa = lb_apply(A, sc(pa, s));
@@ -485,8 +526,8 @@ GG_HD GjkResult<T> gjk_distance(const LocalBody<T>& A, const LocalBody<T>& B, T 
                                 const GjkStart<T>& st = GjkStart<T>()) {
   T words[kGjkWords];
   GjkRun<T> r;
-  r.g.base = words;
-  r.g.stride = 1;
+  r.points = words;
+  r.stride = 1;
   gjk_begin(r, A, B, rel_error, st);
   while (!gjk_iterate(r, A, B)) {
   }
@@ -534,6 +575,7 @@ GG_HD double sv_triple(V3<double> a, V3<double> b, V3<double> c) { return dot(a,
 
 GG_HD void sv_finish(const V3<double>* y, SvPick& r) {
   V3<double> pt = v3<double>(0., 0., 0.);
+#pragma unroll
   for (int k = 0; k < 4; ++k)
     if (r.keep & (1u << k)) pt = pt + sc(y[k], r.lam[k]);
   r.d2 = dot(pt, pt);
@@ -573,11 +615,13 @@ GG_HD SvPick sv_pick_triangle(const V3<double>* y, int a, int b, int c) {
   if (area[0] > 0. && area[1] > 0. && area[2] > 0.) {
     const double total = area[0] + area[1] + area[2];
     SvPick r{(1u << a) | (1u << b) | (1u << c), {0., 0., 0., 0.}, 0.};
+#pragma unroll
     for (int k = 0; k < 3; ++k) r.lam[vx[k]] = area[k] / total;
     sv_finish(y, r);
     return r;
   }
   SvPick best{0u, {0., 0., 0., 0.}, INFINITY};
+#pragma unroll
   for (int k = 0; k < 3; ++k) {
     if (area[k] > 0.) continue;  // the projection is on y_k's side of the opposite edge
     const SvPick e = sv_pick_segment(y, vx[(k + 1) % 3], vx[(k + 2) % 3]);
@@ -591,6 +635,7 @@ GG_HD SvPick sv_pick_tetrahedron(const V3<double>* y) {
                          sv_triple(y[0], y[1] - y[0], y[3] - y[0]), -sv_triple(y[0], y[1] - y[0], y[2] - y[0])};
   const double total = sv_triple(y[1] - y[0], y[2] - y[0], y[3] - y[0]);
   bool same[4];
+#pragma unroll
   for (int k = 0; k < 4; ++k) same[k] = vol[k] != 0. && ((vol[k] > 0.) == (total > 0.));
   if (total != 0. && same[0] && same[1] && same[2] && same[3]) {
     const double sum = (vol[0] + vol[1]) + (vol[2] + vol[3]);
@@ -598,6 +643,7 @@ GG_HD SvPick sv_pick_tetrahedron(const V3<double>* y) {
     return r;  // the origin is inside: distance zero
   }
   SvPick best{0u, {0., 0., 0., 0.}, INFINITY};
+#pragma unroll
   for (int k = 0; k < 4; ++k) {
     if (same[k] && total != 0.) continue;
     const SvPick f = sv_pick_triangle(y, (k + 1) & 3, (k + 2) & 3, (k + 3) & 3);
@@ -612,92 +658,152 @@ GG_HD SvPick sv_pick_tetrahedron(const V3<double>* y) {
 // (relative rel_error or absolute 1e-4 rel_error), on a support point already
 // in the simplex, on a full simplex, at distance <= EPSILON2 or after 1000
 // iterations; the accelerated direction as in gjk_distance.
-GG_HD GjkResult<double> gjk_sv_distance(const LocalBody<double>& A, const LocalBody<double>& B, double rel_error,
-                                        const GjkStart<double>& st = GjkStart<double>()) {
-  const V3<double> zero = v3<double>(0., 0., 0.);
-  V3<double> y[4], p[4], q[4];
-  double lam[4] = {0., 0., 0., 0.};
-  for (int i = 0; i < 4; ++i) y[i] = p[i] = q[i] = zero;
-  int n = 0;  // vertices in the simplex
-  const double abs_error = 1.e-4 * rel_error;
-  V3<double> v, w;
-  double dist = gjk_first(A, B, st, v, w);
-  V3<double> d = v;
-  bool accel = st.accel;
-  int iters = 0, exit_reason = 3;
-  double lower = -dist;
-  while (n < 4 && dist > kEpsilon2 && iters < 1000) {
-    ++iters;
-    d = gjk_direction(accel, iters, d, v, w);
-    V3<double> pa = support_local(A, lb_vecmat(-d, A));
-    V3<double> qb = support_local(B, lb_vecmat(d, B));
-    w = lb_apply(A, pa) - lb_apply(B, qb);
-    const double sep = dot(v, w) / dist;
-    if (sep > lower) lower = sep;
-    const double gap = dist - sep;
-    if (gap < dist * rel_error || gap < abs_error) {
-      if (!accel || norm(d - v) < kEpsilon) {
-        exit_reason = 0;
-        break;
-      }
-      accel = false;
-      pa = support_local(A, lb_vecmat(-v, A));
-      qb = support_local(B, lb_vecmat(v, B));
-      w = lb_apply(A, pa) - lb_apply(B, qb);
-    }
-    bool repeated = false;
-    for (int k = 0; k < n; ++k) repeated = repeated || (y[k].x == w.x && y[k].y == w.y && y[k].z == w.z);
-    if (repeated) {
-      exit_reason = 1;
-      break;
-    }
-    y[n] = w;
-    p[n] = pa;
-    q[n] = qb;
-    ++n;
-    SvPick pick;
-    if (n == 1) pick = sv_pick_vertex(y, 0);
-    else if (n == 2) pick = sv_pick_segment(y, 0, 1);
-    else if (n == 3) pick = sv_pick_triangle(y, 0, 1, 2);
-    else pick = sv_pick_tetrahedron(y);
-    // In exact arithmetic the new support point is part of the answer whenever
-    // the optimality gap is still open; when rounding drops it, the next
-    // iteration would find the same point again and cycle: stop here, with the
-    // answer of the current simplex (like a support point already in it).
-    const bool dropped = !(pick.keep & (1u << (n - 1)));
-    // pack the kept vertices to the front, in their order
-    int m = 0;
-    v = zero;
-    for (int k = 0; k < n; ++k) {
-      if (!(pick.keep & (1u << k))) continue;
-      y[m] = y[k];
-      p[m] = p[k];
-      q[m] = q[k];
-      lam[m] = pick.lam[k];
-      v = v + sc(y[m], lam[m]);
-      ++m;
-    }
-    n = m;
-    dist = norm(v);
-    if (dropped) {
-      exit_reason = 1;
-      break;
-    }
+//
+// Like GjkRun a resumable state: sv_begin, sv_iterate, sv_end.  The simplex is in
+// registers (its moves to the front are written out for the four places), the
+// support points in the caller's storage.
+struct SvRun {
+  V3<double> y[4];
+  double lam[4];
+  int n;           // vertices in the simplex
+  double* points;  // support points of A and B by vertex, as GjkRun::points
+  int stride;
+  V3<double> v, w, d;
+  double dist, lower, rel_error, abs_error;
+  int num, exit_reason;
+  bool accel;
+
+  GG_HD V3<double> point(int body, int k) const {
+    const double* b = points + (12 * body + 3 * k) * stride;
+    return v3<double>(b[0], b[stride], b[2 * stride]);
   }
-  V3<double> wa = zero, wb = zero;
-  for (int k = 0; k < n; ++k) {
-    wa = wa + sc(p[k], lam[k]);
-    wb = wb + sc(q[k], lam[k]);
+  GG_HD void set_point(int body, int k, V3<double> p) const {
+    double* b = points + (12 * body + 3 * k) * stride;
+    b[0] = p.x;
+    b[stride] = p.y;
+    b[2 * stride] = p.z;
+  }
+};
+
+GG_HD void gjk_begin(SvRun& r, const LocalBody<double>& A, const LocalBody<double>& B, double rel_error,
+                     const GjkStart<double>& st) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    r.y[i] = v3<double>(0., 0., 0.);
+    r.lam[i] = 0.;
+  }
+  r.n = 0;
+  r.rel_error = rel_error;
+  r.abs_error = 1.e-4 * rel_error;
+  r.dist = gjk_first(A, B, st, r.v, r.w);
+  r.d = r.v;
+  r.accel = st.accel;
+  r.num = 0;
+  r.exit_reason = 3;
+  r.lower = -r.dist;
+}
+
+// one pass of the loop; true when the run has ended
+GG_HD bool gjk_iterate(SvRun& r, const LocalBody<double>& A, const LocalBody<double>& B) {
+  if (!(r.n < 4 && r.dist > kEpsilon2 && r.num < 1000)) return true;
+  ++r.num;
+  r.d = gjk_direction(r.accel, r.num, r.d, r.v, r.w);
+  V3<double> pa = support_local(A, lb_vecmat(-r.d, A));
+  V3<double> qb = support_local(B, lb_vecmat(r.d, B));
+  r.w = lb_apply(A, pa) - lb_apply(B, qb);
+  const double sep = dot(r.v, r.w) / r.dist;
+  if (sep > r.lower) r.lower = sep;
+  const double gap = r.dist - sep;
+  if (gap < r.dist * r.rel_error || gap < r.abs_error) {
+    if (!r.accel || norm(r.d - r.v) < kEpsilon) {
+      r.exit_reason = 0;
+      return true;
+    }
+    r.accel = false;
+    pa = support_local(A, lb_vecmat(-r.v, A));
+    qb = support_local(B, lb_vecmat(r.v, B));
+    r.w = lb_apply(A, pa) - lb_apply(B, qb);
+  }
+  bool repeated = false;
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    repeated = repeated || (k < r.n && r.y[k].x == r.w.x && r.y[k].y == r.w.y && r.y[k].z == r.w.z);
+  if (repeated) {
+    r.exit_reason = 1;
+    return true;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (r.n == k) r.y[k] = r.w;
+  r.set_point(0, r.n, pa);
+  r.set_point(1, r.n, qb);
+  ++r.n;
+  SvPick pick;
+  if (r.n == 1) pick = sv_pick_vertex(r.y, 0);
+  else if (r.n == 2) pick = sv_pick_segment(r.y, 0, 1);
+  else if (r.n == 3) pick = sv_pick_triangle(r.y, 0, 1, 2);
+  else pick = sv_pick_tetrahedron(r.y);
+  // In exact arithmetic the new support point is part of the answer whenever
+  // the optimality gap is still open; when rounding drops it, the next
+  // iteration would find the same point again and cycle: stop here, with the
+  // answer of the current simplex (like a support point already in it).
+  const bool dropped = !(pick.keep & (1u << (r.n - 1)));
+  // pack the kept vertices to the front, in their order
+  int m = 0;
+  r.v = v3<double>(0., 0., 0.);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (k >= r.n || !(pick.keep & (1u << k))) continue;
+    const V3<double> yk = r.y[k];
+    const double lk = pick.lam[k];
+#pragma unroll
+    for (int to = 0; to <= k; ++to)
+      if (m == to) {
+        r.y[to] = yk;
+        r.lam[to] = lk;
+      }
+    if (m != k) {
+      r.set_point(0, m, r.point(0, k));
+      r.set_point(1, m, r.point(1, k));
+    }
+    r.v = r.v + sc(yk, lk);
+    ++m;
+  }
+  r.n = m;
+  r.dist = norm(r.v);
+  if (dropped) r.exit_reason = 1;
+  return dropped;
+}
+
+GG_HD GjkResult<double> gjk_end(const SvRun& run, const LocalBody<double>& A, const LocalBody<double>& B) {
+  V3<double> wa = v3<double>(0., 0., 0.), wb = wa;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (k >= run.n) continue;
+    wa = wa + sc(run.point(0, k), run.lam[k]);
+    wb = wb + sc(run.point(1, k), run.lam[k]);
   }
   GjkResult<double> r;
   r.pa = lb_apply(A, wa);
   r.pb = lb_apply(B, wb);
-  r.dist = dist;
-  r.iters = iters;
-  r.exit = exit_reason;
-  r.lower = lower;
-  r.v = v;
+  r.dist = run.dist;
+  r.iters = run.num;
+  r.exit = run.exit_reason;
+  r.lower = run.lower;
+  r.v = run.v;
   return r;
+}
+
+GG_HD GjkResult<double> gjk_sv_distance(const LocalBody<double>& A, const LocalBody<double>& B, double rel_error,
+                                        const GjkStart<double>& st = GjkStart<double>()) {
+  double words[kGjkWords];
+  SvRun r;
+  r.points = words;
+  r.stride = 1;
+  gjk_begin(r, A, B, rel_error, st);
+  while (!gjk_iterate(r, A, B)) {
+  }
+  return gjk_end(r, A, B);
 }
 
 // The contact features of a finished distance run (RigidBodyWithCrust.cpp:
@@ -751,43 +857,11 @@ GG_HD ContactGeom convex_closest_point_t(const BodyRef& A, const BodyRef& B, dou
   return gjk_features(r, xadd(A.crust, B.crust), shift);
 }
 
-// RigidBodyWithCrust::ClosestPoint with the signed-volume GJK (the same
-// features as convex_closest_point_t)
-GG_HD ContactGeom convex_closest_point_sv(const BodyRef& A, const BodyRef& B, double tol, int* iters,
-                                         GjkStart<double>* st = nullptr) {
-  ContactGeom c = no_contact();
-  D3 g = xsub3(A.origin, B.origin);
-  if (!(xnorm(g) < xadd(A.radius, B.radius))) {
-    c.status = 2;
-    if (st) st->v0 = v3<double>(0., 0., 0.);
-    return c;
-  }
-  LocalBody<double> la = local_body<double>(A, d3(0., 0., 0.), A.scaling);
-  LocalBody<double> lb = local_body<double>(B, d3(0., 0., 0.), B.scaling);
-  GjkResult<double> r = st ? gjk_sv_distance(la, lb, tol, *st) : gjk_sv_distance(la, lb, tol);
-  if (st) st->v0 = r.v;
-  *iters = r.iters;
-  if (r.dist < kEpsilon) {
-    c.status = 1;
-    return c;
-  }
-  V3<double> ba = r.pa - r.pb;
-  V3<double> pc = dv(r.pa, 2.) + dv(r.pb, 2.);
-  double crust_sum = xadd(A.crust, B.crust);
-  V3<double> ov = round3(dv(ba, r.dist));
-  ov = sc(ov, crust_sum - r.dist);
-  c.point = d3(pc.x, pc.y, pc.z);
-  c.overlap_vector = d3(ov.x, ov.y, ov.z);
-  c.overlap = r.dist - crust_sum;
-  c.status = 0;
-  return c;
-}
-
 // RigidBodyWithCrust::ClosestPoint_ErreurHandling (RigidBodyWithCrust.cpp:532-588):
 // bodies shrunk by 'factor' crusts (scaling capped below at 0.5); the contact
 // is imposed with overlap = -(crust sum) along the witness direction B->A.
 // status 1 when even the shrunk bodies touch (fatal ContactError).
-GG_HD ContactGeom convex_error_handling(const BodyRef& A, const BodyRef& B, const double ext_a[3],
+GG_COLD ContactGeom convex_error_handling(const BodyRef& A, const BodyRef& B, const double ext_a[3],
                                         const double ext_b[3], double factor, double tol, bool accel = false) {
   double sa[3], sb[3];
   for (int i = 0; i < 3; ++i) {

@@ -21,6 +21,7 @@
 #pragma once
 
 #include <algorithm>
+#include <type_traits>
 
 #include <cooperative_groups.h>
 
@@ -570,12 +571,11 @@ __device__ __forceinline__ void make_obstacle_ref(const StepArgs<R>& a, int oidx
 // per step, 100,000 convex bodies).  Error handling (crust x10) on
 // ContactError.  st carries the accelerated-direction option and, for a
 // warm-started run, the pair's direction in and out.
-template <typename R, bool SV = false>
+template <typename R>
 __device__ ContactGeom convex_closest_point(const StepArgs<R>& a, const BodyRef& A, const BodyRef& B, int& iters,
                                             int& handled, GjkStart<double>& st) {
   handled = 0;
-  ContactGeom c = SV ? convex_closest_point_sv(A, B, a.gjk_tol, &iters, &st)
-                     : convex_closest_point_t<double>(A, B, a.gjk_tol, &iters, nullptr, nullptr, &st);
+  ContactGeom c = convex_closest_point_t<double>(A, B, a.gjk_tol, &iters, nullptr, nullptr, &st);
   if (c.status == 1) {
     c = convex_error_handling(A, B, A.lext, B.lext, 10., a.gjk_tol, st.accel);
     handled = 1;
@@ -879,7 +879,7 @@ __device__ __forceinline__ void put_memory(const StepArgs<R>& a, int row, int ra
 // or particle-obstacle candidate (p0 = the particle, p1 = the obstacle)
 // GEOM: the narrowphase of general convex pairs comes from the GJK kernel
 // (gjk_out) instead of running here
-template <typename R, bool DIAG, bool CONVEX, bool SV = false, bool GEOM = false>
+template <typename R, bool DIAG, bool CONVEX, bool GEOM = false>
 __device__ __forceinline__ void pair_one(const StepArgs<R>& a, int idx, int4 item, R dt, ForceStats& fs) {
   const ParticleArrays<R>& P = a.cur;
   const int s = item.x, e = item.y, q = item.z & 511, rank = item.z >> 9, oi = item.w;
@@ -953,7 +953,7 @@ __device__ __forceinline__ void pair_one(const StepArgs<R>& a, int idx, int4 ite
       bool known = false;
       if (st.history) known = find_gjk_dir(a, oi, mj.x, st.v0);
       const V3<double> v_before = st.v0;
-      g = convex_closest_point<R, SV>(a, ba, bb, it, handled, st);
+      g = convex_closest_point(a, ba, bb, it, handled, st);
       if (g.status != 2) {
         ++fs.ngjk;
         fs.ngjk_it += it;
@@ -1075,7 +1075,7 @@ __device__ __forceinline__ void pair_one(const StepArgs<R>& a, int idx, int4 ite
     int it = 0, handled = 0;
     GjkStart<double> st;  // no collision history for obstacles (SimpleObstacle.cpp:222-250)
     st.accel = a.gjk_accel != 0;
-    g = convex_closest_point<R, SV>(a, ba, bb, it, handled, st);
+    g = convex_closest_point(a, ba, bb, it, handled, st);
     if (g.status != 2) {
       ++fs.ngjk;
       fs.ngjk_it += it;
@@ -1137,7 +1137,8 @@ __device__ __forceinline__ void pair_one(const StepArgs<R>& a, int idx, int4 ite
 }
 
 // ---------------------------------------------------------------------------
-// B0. The GJK phase of convex scenarios (Johnson's GJK): every work item whose
+// B0. The GJK phase of convex scenarios (Johnson's GJK or the signed-volume one,
+// an instance each): every work item whose
 // pair needs the general narrowphase gets RigidBodyWithCrust::ClosestPoint's
 // features written to gjk_out[item]; the pair kernel then applies the law.
 //
@@ -1189,16 +1190,59 @@ __device__ __forceinline__ int take_item(int* counter) {
   return g.shfl(base, 0) + (int)g.thread_rank();
 }
 
-template <typename R>
+// A thread's GJK run in flight.  What an iteration needs of the two bodies (the
+// shrunk basis, the origin, three sizes: 15 numbers each) and the run's support
+// points (24) lie in shared memory, interleaved across the block's threads, so
+// that the registers hold the simplex and its determinants.
+constexpr int kBodyWords = 15;
+constexpr int kLaneWords = 2 * kBodyWords + kGjkWords;
+template <typename RUN>
 struct GjkLane {
-  int idx;        // work item in flight
-  int4 item;
-  double crust_sum;
-  bool known;     // the pair's history was found
-  V3<double> v_before;
-  LocalBody<double> la, lb;
-  GjkRun<double> run;
+  int idx;               // work item in flight
+  int type[2], nverts[2], verts[2];  // shape type, polyhedron vertices (first in the vertex table)
+  int vertex[2];         // the hill climb's current vertices
+  double* words;         // the lane's shared memory (stride kGjkBlock)
+  RUN run;               // GjkRun<double> (Johnson) or SvRun (signed volumes)
 };
+constexpr int kGjkBlock = 64;
+
+template <typename RUN>
+__device__ __forceinline__ void put_lane_body(GjkLane<RUN>& L, int w, const BodyRef& r, int vert_offset) {
+  const LocalBody<double> B = local_body<double>(r, d3(0., 0., 0.), r.scaling);
+  double* d = L.words + w * kBodyWords * kGjkBlock;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) d[i * kGjkBlock] = B.b[i];
+  d[9 * kGjkBlock] = B.o.x;
+  d[10 * kGjkBlock] = B.o.y;
+  d[11 * kGjkBlock] = B.o.z;
+  const bool box = B.type == GRAINS_GPU_BOX, cyl = B.type == GRAINS_GPU_CYLINDER;
+  d[12 * kGjkBlock] = box ? B.ext.x : (cyl ? B.cyl_r : B.radius);
+  d[13 * kGjkBlock] = box ? B.ext.y : B.cyl_hh;
+  d[14 * kGjkBlock] = B.ext.z;
+  L.type[w] = B.type;
+  L.nverts[w] = B.nverts;
+  L.verts[w] = vert_offset;
+  L.vertex[w] = 0;
+}
+
+template <typename R, typename RUN>
+__device__ __forceinline__ LocalBody<double> lane_body(const StepArgs<R>& a, const GjkLane<RUN>& L, int w) {
+  LocalBody<double> B;
+  const double* d = L.words + w * kBodyWords * kGjkBlock;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) B.b[i] = d[i * kGjkBlock];
+  B.o = v3<double>(d[9 * kGjkBlock], d[10 * kGjkBlock], d[11 * kGjkBlock]);
+  B.radius = B.cyl_r = B.ext.x = d[12 * kGjkBlock];
+  B.cyl_hh = B.ext.y = d[13 * kGjkBlock];
+  B.ext.z = d[14 * kGjkBlock];
+  B.type = L.type[w];
+  B.nverts = L.nverts[w];
+  B.verts = a.verts + 3 * L.verts[w];
+  B.adj_start = a.adj_start + L.verts[w];
+  B.adj = a.adj;
+  B.cur = L.vertex[w];
+  return B;
+}
 
 // the collision history of a particle pair (Particle.cpp:497-504): the run's
 // last iterate, or the entry as it was when a ContactError was handled, or a
@@ -1221,8 +1265,8 @@ __device__ __forceinline__ void store_gjk_dir(const StepArgs<R>& a, int4 item, i
 
 // takes work items until one needs a GJK run and starts it; items whose
 // bounding spheres are apart are finished on the way.  False when none is left.
-template <typename R>
-__device__ bool gjk_lane_start(const StepArgs<R>& a, int n_gjk, GjkLane<R>& L) {
+template <typename R, typename RUN>
+__device__ __forceinline__ bool gjk_lane_start(const StepArgs<R>& a, int n_gjk, GjkLane<RUN>& L) {
   for (;;) {
     const int j = take_item(a.gjk_next);
     if (j >= n_gjk) return false;
@@ -1235,45 +1279,37 @@ __device__ bool gjk_lane_start(const StepArgs<R>& a, int n_gjk, GjkLane<R>& L) {
     GjkStart<double> st;
     st.accel = a.gjk_accel != 0;
     st.history = pair && a.gjk_history != 0;
-    L.known = st.history && find_gjk_dir(a, item.w, partner, st.v0);
+    const bool known = st.history && find_gjk_dir(a, item.w, partner, st.v0);
     const D3 g = xsub3(ba.origin, bb.origin);
     if (!(xnorm(g) < xadd(ba.radius, bb.radius))) {  // RigidBodyWithCrust.cpp:278-282
       GjkOut& o = a.gjk_out[k];
       o.status = 2;
       o.handled = 0;
       o.overlap = 1.;
-      if (st.history) store_gjk_dir(a, item, partner, 2, 0, L.known, st.v0, st.v0);
+      if (st.history) store_gjk_dir(a, item, partner, 2, 0, known, st.v0, st.v0);
       continue;
     }
     L.idx = k;
-    L.item = item;
-    L.crust_sum = xadd(ba.crust, bb.crust);
-    L.v_before = st.v0;
-    L.la = local_body<double>(ba, d3(0., 0., 0.), ba.scaling);
-    L.lb = local_body<double>(bb, d3(0., 0., 0.), bb.scaling);
-    gjk_begin(L.run, L.la, L.lb, a.gjk_tol, st);  // L.run.g: the lane's shared-memory arrays
+    put_lane_body(L, 0, ba, (int)((ba.verts - a.verts) / 3));
+    put_lane_body(L, 1, bb, (int)((bb.verts - a.verts) / 3));
+    const LocalBody<double> A = lane_body(a, L, 0), B = lane_body(a, L, 1);
+    gjk_begin(L.run, A, B, a.gjk_tol, st);
+    L.vertex[0] = A.cur;
+    L.vertex[1] = B.cur;
     return true;
   }
 }
 
-// the features of a finished run, the crust-x10 retry on ContactError, the
-// history and the statistics
-template <typename R>
-__device__ void gjk_lane_finish(const StepArgs<R>& a, GjkLane<R>& L, unsigned long long& ngjk,
-                                unsigned long long& nit) {
-  const GjkResult<double> r = gjk_end(L.run, L.la, L.lb);
-  ContactGeom c = gjk_features(r, L.crust_sum, d3(0., 0., 0.));
-  ++ngjk;
-  nit += r.iters;
-  int handled = 0;
-  if (c.status == 1) {
-    BodyRef ba, bb;
-    item_bodies(a, L.item, ba, bb);
-    c = convex_error_handling(ba, bb, ba.lext, bb.lext, 10., a.gjk_tol, a.gjk_accel != 0);
-    handled = 1;
-    set_status(a.stats, c.status == 1 ? GRAINS_GPU_CONTACT_ERROR : GRAINS_GPU_CONTACT_HANDLED);
-  }
-  GjkOut& o = a.gjk_out[L.idx];
+template <typename R, typename RUN>
+__device__ __forceinline__ bool gjk_lane_iterate(const StepArgs<R>& a, GjkLane<RUN>& L) {
+  const LocalBody<double> A = lane_body(a, L, 0), B = lane_body(a, L, 1);
+  const bool ended = gjk_iterate(L.run, A, B);
+  L.vertex[0] = A.cur;
+  L.vertex[1] = B.cur;
+  return ended;
+}
+
+__device__ __forceinline__ void put_gjk_out(GjkOut& o, const ContactGeom& c, int handled) {
   o.point[0] = c.point.x;
   o.point[1] = c.point.y;
   o.point[2] = c.point.z;
@@ -1283,8 +1319,50 @@ __device__ void gjk_lane_finish(const StepArgs<R>& a, GjkLane<R>& L, unsigned lo
   o.overlap = c.overlap;
   o.status = c.status;
   o.handled = handled;
-  if (L.item.y >= 0 && a.gjk_history)
-    store_gjk_dir(a, L.item, a.cur.meta[entry_slot(L.item.y)].x, c.status, handled, L.known, L.v_before, r.v);
+}
+
+// the features of a finished run, the history and the statistics.  An item that
+// ended in a ContactError joins the thread's chain of such items (`errors`: its
+// head, linked through GjkOut::handled) for gjk_lane_retry.
+template <typename R, typename RUN>
+__device__ __forceinline__ void gjk_lane_finish(const StepArgs<R>& a, GjkLane<RUN>& L, int& errors,
+                                                unsigned long long& ngjk, unsigned long long& nit) {
+  const int4 item = a.work[L.idx];
+  const double crust_sum =
+      xadd(a.cur.md[item.x].y, item.y >= 0 ? a.cur.md[entry_slot(item.y)].y : a.obs[-1 - item.y].crust);
+  const GjkResult<double> r = gjk_end(L.run, lane_body(a, L, 0), lane_body(a, L, 1));
+  const ContactGeom c = gjk_features(r, crust_sum, d3(0., 0., 0.));
+  ++ngjk;
+  nit += r.iters;
+  put_gjk_out(a.gjk_out[L.idx], c, 0);
+  if (c.status == 1) {
+    a.gjk_out[L.idx].handled = errors;
+    errors = L.idx;
+  } else if (item.y >= 0 && a.gjk_history) {
+    store_gjk_dir(a, item, a.cur.meta[entry_slot(item.y)].x, c.status, 0, false, r.v, r.v);
+  }
+}
+
+// the crust-x10 retry of the thread's ContactErrors, after its runs: the call
+// and its bodies stay out of the registers of the run loop
+template <typename R>
+__device__ __forceinline__ void gjk_lane_retry(const StepArgs<R>& a, int errors) {
+  while (errors >= 0) {
+    const int idx = errors;
+    errors = a.gjk_out[idx].handled;
+    const int4 item = a.work[idx];
+    BodyRef ba, bb;
+    item_bodies(a, item, ba, bb);
+    const ContactGeom c = convex_error_handling(ba, bb, ba.lext, bb.lext, 10., a.gjk_tol, a.gjk_accel != 0);
+    set_status(a.stats, c.status == 1 ? GRAINS_GPU_CONTACT_ERROR : GRAINS_GPU_CONTACT_HANDLED);
+    put_gjk_out(a.gjk_out[idx], c, 1);
+    if (item.y >= 0 && a.gjk_history) {  // the history entry stays as it was
+      const int partner = a.cur.meta[entry_slot(item.y)].x;
+      V3<double> before = v3<double>(0., 0., 0.);
+      const bool known = find_gjk_dir(a, item.w, partner, before);
+      store_gjk_dir(a, item, partner, c.status, 1, known, before, before);
+    }
+  }
 }
 
 // The GJK items are grouped by the shape types of their pair first (a
@@ -1374,13 +1452,19 @@ __global__ void __launch_bounds__(256) gjk_place_kernel(StepArgs<R> a) {
 // Starting a run (the bodies, the history, the first iterate) costs about as
 // much as two GJK iterations and diverges across the shapes, so lanes whose
 // run has ended wait until GG_GJK_BATCH lanes of the warp are idle (by default
-// the whole warp) and start their next runs together (settled drum, pair phase
-// per step: 3.05 ms with batches of 16, 2.88 with 24, 2.75 with 32).
-// The arrays of each thread's run (sub-determinants, dot products, simplex and
-// support points: 672 bytes) live in shared memory, interleaved across the
-// block's 64 threads; in local memory they overflowed L1 and were written back
-// to DRAM (1.9 GB per launch on the settled drum).
-constexpr int kGjkBlock = 64;
+// the whole warp) and start their next runs together.
+// What bounds it: the instructions of an iteration, issued in order by few
+// warps (FP64 pipe 11 % busy, DRAM idle).  So the sub-algorithm is written out
+// with predicates (gjk_closest: 55 M instead of 85 M warp instructions for
+// 70,600 runs, 14.5 instead of 9.9 lanes active), the simplex stays in
+// registers (255, 8 warps per SM), the bodies and support points, 54 numbers a
+// thread, in shared memory, and the rare retry of a ContactError runs after the
+// loop: called inside it, its spills took 5 of 6 issue slots.  141,000 runs of
+// 10.3 iterations (40,000 bodies, pair phase): 0.626 -> 0.341 ms; 7,000 runs,
+// where one run's length is the time: 0.253 -> 0.145 ms.  Registers limited to
+// 168 for 12 warps: 0.389 ms; to 128 for 16: 0.554 ms; batches of 16: 0.403 ms.
+// The signed-volume runs ran in the pair kernel, one per thread, until they took
+// this kernel too (11,111 bodies, 38,000 runs, pair phase): 0.803 -> 0.306 ms.
 // idle lanes of a warp that wait before they write their results and start
 // their next runs together
 #ifndef GG_GJK_BATCH
@@ -1389,21 +1473,24 @@ constexpr int kGjkBlock = 64;
 #ifndef GG_GJK_MIN_BLOCKS
 #define GG_GJK_MIN_BLOCKS 1
 #endif
-template <typename R>
+template <typename R, bool SV>
 __global__ void __launch_bounds__(kGjkBlock, GG_GJK_MIN_BLOCKS) gjk_kernel(StepArgs<R> a) {
-  __shared__ double words[kGjkWords * kGjkBlock];
+  using Run = typename std::conditional<SV, SvRun, GjkRun<double>>::type;
+  __shared__ double words[kLaneWords * kGjkBlock];
   const unsigned full = 0xffffffffu;
   int n_items = 0;  // GJK items: the total of the shape-pair bins
   for (int b = 0; b < kGjkBins; ++b) n_items += a.gjk_bins[b];
   unsigned long long ngjk = 0, nit = 0;
-  GjkLane<R> L;
-  L.run.g.base = words + threadIdx.x;
-  L.run.g.stride = kGjkBlock;
+  int errors = -1;
+  GjkLane<Run> L;
+  L.words = words + threadIdx.x;
+  L.run.points = L.words + 2 * kBodyWords * kGjkBlock;
+  L.run.stride = kGjkBlock;
   bool busy = gjk_lane_start(a, n_items, L);
   bool ended = false;    // the lane's run has ended and waits for its results to be written
   bool drained = !busy;  // no work item is left for this lane
   for (;;) {
-    if (busy && gjk_iterate(L.run, L.la, L.lb)) {
+    if (busy && gjk_lane_iterate(a, L)) {
       busy = false;
       ended = true;
     }
@@ -1413,7 +1500,7 @@ __global__ void __launch_bounds__(kGjkBlock, GG_GJK_MIN_BLOCKS) gjk_kernel(StepA
     if (__popc(waiting) >= GG_GJK_BATCH || !running) {
       // the ended runs' results and the next runs' starts, together
       if (ended) {
-        gjk_lane_finish(a, L, ngjk, nit);
+        gjk_lane_finish(a, L, errors, ngjk, nit);
         ended = false;
       }
       if (!busy && !drained) {
@@ -1422,19 +1509,20 @@ __global__ void __launch_bounds__(kGjkBlock, GG_GJK_MIN_BLOCKS) gjk_kernel(StepA
       }
     }
   }
+  gjk_lane_retry(a, errors);
   warp_add(&a.stats->n_gjk_calls, ngjk);
   warp_add(&a.stats->n_gjk_iters, nit);
 }
 
 // work items [first, n_items) with the given stride; `padded`: a bound with a
 // uniform trip count for the warp reductions of the statistics
-template <typename R, bool DIAG, bool CONVEX, bool SV = false, bool GEOM = false>
+template <typename R, bool DIAG, bool CONVEX, bool GEOM = false>
 __device__ __forceinline__ void pairs_range(const StepArgs<R>& a, int first, int stride, R dt) {
   const int n_items = (int)min((long long)*(volatile int*)a.work_n, (long long)a.n * a.clist_cap);
   const int padded = (n_items + stride - 1) / stride * stride;
   ForceStats fs{0, 0, 0, 0, 0., 0.};
   for (int k = first; k < padded; k += stride)
-    if (k < n_items) pair_one<R, DIAG, CONVEX, SV, GEOM>(a, k, a.work[k], dt, fs);
+    if (k < n_items) pair_one<R, DIAG, CONVEX, GEOM>(a, k, a.work[k], dt, fs);
   flush_force_stats(a.stats, fs);
 }
 
@@ -1452,10 +1540,10 @@ __device__ __forceinline__ void pairs_range(const StepArgs<R>& a, int first, int
 #ifndef GG_PAIRS_CONVEX_MIN_BLOCKS
 #define GG_PAIRS_CONVEX_MIN_BLOCKS 3
 #endif
-template <typename R, bool DIAG, bool CONVEX, bool SV = false, bool GEOM = false>
+template <typename R, bool DIAG, bool CONVEX, bool GEOM = false>
 __global__ void __launch_bounds__(128, CONVEX ? (GEOM ? GG_PAIRS_CONVEX_MIN_BLOCKS : 1) : GG_PAIRS_MIN_BLOCKS)
     pairs_kernel(StepArgs<R> a, R dt) {
-  pairs_range<R, DIAG, CONVEX, SV, GEOM>(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, dt);
+  pairs_range<R, DIAG, CONVEX, GEOM>(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, dt);
 }
 
 // C. the torsor of particle s: InitializeForces(withWeight) (torsor = weight,
@@ -2043,7 +2131,7 @@ int launch_sort_and_gather(const StepArgs<R>& a, cudaStream_t s, int gather, int
 }
 
 // the GJK kernel keeps every SM full: its resident blocks per SM x the SMs
-template <typename R>
+template <typename R, bool SV>
 int gjk_grid() {
   static int grid = 0;
   if (!grid) {
@@ -2051,8 +2139,8 @@ int gjk_grid() {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // as much shared memory as the SM has, for the runs' arrays
-    cudaFuncSetAttribute(gjk_kernel<R>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gjk_kernel<R>, kGjkBlock, 0);
+    cudaFuncSetAttribute(gjk_kernel<R, SV>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gjk_kernel<R, SV>, kGjkBlock, 0);
     grid = (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1);
   }
   return grid;
@@ -2078,26 +2166,19 @@ int launch_forces(const StepArgs<R>& a, cudaStream_t s, double dt, int diag, int
   // about two work items per thread in a settled packing; the grid-stride
   // loop takes any count
   const int g = (int)std::min<long long>(grid_for(2ll * a.n, fb), 1ll << 20);
-  if (a.has_convex && a.gjk_sv) {  // the signed-volume GJK: a kernel of its own
-    if (diag)
-      pairs_kernel<R, true, true, true><<<g, fb, 0, s>>>(a, R(dt));
-    else
-      pairs_kernel<R, false, true, true><<<g, fb, 0, s>>>(a, R(dt));
-  } else if (a.has_convex && a.gjk_out) {  // the GJK items grouped by shape pair, the GJK kernel, the law
+  if (a.has_convex) {  // the GJK items grouped by shape pair, the GJK kernel, the law
     cudaMemsetAsync(a.gjk_bins, 0, 2 * kGjkBins * sizeof(int), s);
     const int gb = 2 * 148;
     gjk_count_kernel<R><<<gb, 256, 0, s>>>(a);
     gjk_place_kernel<R><<<gb, 256, 0, s>>>(a);
-    gjk_kernel<R><<<gjk_grid<R>(), kGjkBlock, 0, s>>>(a);
-    if (diag)
-      pairs_kernel<R, true, true, false, true><<<g, fb, 0, s>>>(a, R(dt));
+    if (a.gjk_sv)
+      gjk_kernel<R, true><<<gjk_grid<R, true>(), kGjkBlock, 0, s>>>(a);
     else
-      pairs_kernel<R, false, true, false, true><<<g, fb, 0, s>>>(a, R(dt));
-  } else if (a.has_convex) {
+      gjk_kernel<R, false><<<gjk_grid<R, false>(), kGjkBlock, 0, s>>>(a);
     if (diag)
-      pairs_kernel<R, true, true><<<g, fb, 0, s>>>(a, R(dt));
+      pairs_kernel<R, true, true, true><<<g, fb, 0, s>>>(a, R(dt));
     else
-      pairs_kernel<R, false, true><<<g, fb, 0, s>>>(a, R(dt));
+      pairs_kernel<R, false, true, true><<<g, fb, 0, s>>>(a, R(dt));
   } else {
     if (diag)
       pairs_kernel<R, true, false><<<g, fb, 0, s>>>(a, R(dt));
