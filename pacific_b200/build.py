@@ -30,7 +30,7 @@ UNITS = [
     ("noalloc.cu", []),
     ("io.cu", ["-fmad=false"]),
 ]
-HEADERS = ["common.cuh", "sphere_contact.cuh", "contact_law.cuh", "gjk.cuh", "kernels.cuh", "device_state.h",
+HEADERS = ["common.cuh", "sphere_contact.cuh", "contact_law.cuh", "gjk.cuh", "kernels.cuh", "resident.cuh", "device_state.h",
            "dual.cuh", "adjoint.cuh", "adjoint.h", "format.cuh", "io.h"]
 
 

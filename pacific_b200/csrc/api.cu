@@ -187,6 +187,16 @@ struct grains_gpu_ctx {
   unsigned* pbar = nullptr;  // grid-barrier state of the persistent launch
   int* psums = nullptr;      // its scan scratch (one int per block)
   int pblocks = 0;
+  // resident pair lists of the middle steps (resident.cuh)
+  char* res_buf = nullptr;   // per-particle and per-obstacle arrays
+  size_t res_bytes = 0;
+  int* cell_count2 = nullptr;  // cell counts of the steps of odd parity
+  int res_blocks = 0;          // blocks of the build's cooperative launch
+  double r_min = 0, r_max = 0; // radii of the uploaded particles
+  std::vector<double> sys_r_max;  // and the largest of each system
+  bool res_ok = false;         // the uploaded scene can run on resident lists
+  cudaGraphExec_t res_graph[4] = {nullptr, nullptr, nullptr, nullptr};  // by (cur, hcur)
+  double res_graph_dt[4] = {0, 0, 0, 0};
   // reload and RawData files (io.cu): particle names by upload index, sorted
   // (system, id) keys, obstacle ids, per-particle record attributes
   int* d_row_id = nullptr;
@@ -638,6 +648,78 @@ StepArgs<R> make_args(grains_gpu_ctx* c) {
   return a;
 }
 
+// The resident lists' buffers: entries, results and pairs in the contact-list
+// scratch (clist; res_f and res_t as one array of two R4 an entry; work), the
+// pair memories in the memory rows' buffer that is not the current one, the
+// rest in res_buf.  So the lists hold as many entries in all as the launched
+// pipeline's.
+constexpr size_t kResAlign = 256;
+constexpr int kResObsHost = 8;  // obstacles per system the state word holds
+size_t res_layout(int64_t cap, int obs_stride, int hist_cap, size_t rsize, size_t off[9]) {
+  size_t at = 0;
+  auto put = [&](int k, size_t bytes) {
+    off[k] = at;
+    at += (bytes + kResAlign - 1) / kResAlign * kResAlign;
+  };
+  const size_t n = (size_t)cap, m = n * (size_t)std::max(1, obs_stride);
+  put(0, 16 * sizeof(int) + 2 * sizeof(unsigned) + sizeof(double) + 4096 * sizeof(int));  // control, barrier, skin, sums
+  put(1, n * sizeof(double4));
+  put(2, n * sizeof(int2));
+  put(3, n * sizeof(int));
+  put(4, n * sizeof(unsigned long long));
+  put(5, m * 8 * rsize);
+  put(6, m * 9 * rsize);
+  put(7, 2 * m * sizeof(int));
+  put(8, n * (size_t)hist_cap);
+  return at;
+}
+
+int res_obs_stride(const grains_gpu_ctx* c) {
+  size_t m = 0;
+  for (const auto& s : c->sys) m = std::max(m, s.obs.size());
+  return (int)m;
+}
+
+template <typename R>
+ResArgs<R> make_res(grains_gpu_ctx* c) {
+  ResArgs<R> r{};
+  size_t off[9];
+  const int stride = res_obs_stride(c);
+  res_layout(c->cap, stride, c->hist_cap, c->rsize, off);
+  char* b = c->res_buf;
+  r.ctl = (int*)(b + off[0]);
+  r.bar = (unsigned*)(r.ctl + 16);
+  r.skin = (double*)(r.bar + 2);
+  r.block_sums = (int*)(r.skin + 1);
+  // a wide skin lasts longer but lists more pairs: 0.2 r_min (a tenth of a
+  // diameter) lists 8 to 9 partners a particle in a dense bed, of which 5 touch
+  r.skin0 = 0.2 * c->r_min;
+  r.r_max = c->r_max;
+  r.x0 = (double4*)(b + off[1]);
+  r.ent = (int2*)(b + off[2]);
+  r.pair_first = (int*)(b + off[3]);
+  r.obs_state = (unsigned long long*)(b + off[4]);
+  r.obs_res = (ResResult<R>*)(b + off[5]);
+  r.obs_mem = (R*)(b + off[6]);
+  const size_t m = (size_t)c->cap * std::max(1, stride);
+  r.obs_item[0] = (int*)(b + off[7]);
+  r.obs_item[1] = r.obs_item[0] + m;
+  r.obs_stride = std::max(1, stride);
+  r.nb = c->clist;
+  r.res = (ResResult<R>*)c->res_f;
+  r.pair = c->work;
+  r.state = (unsigned char*)(b + off[8]);
+  r.mem = (R*)c->hist[1 - c->hcur];
+  // capacities from the buffers' sizes
+  const int64_t ent = std::min<int64_t>(c->cap * (int64_t)c->clist_cap, 1ll << 30);
+  r.ent_cap = (int)ent;
+  r.pair_cap = (int)std::min<int64_t>(ent / 2, c->cap * (int64_t)c->hist_cap);
+  r.count[0] = c->cell_count;
+  r.count[1] = c->cell_count2;
+  r.rebuild_blocks = c->res_blocks;
+  return r;
+}
+
 // Runs f(args) with the StepArgs of the context's precision
 template <typename F>
 int with_args(grains_gpu_ctx* c, F f) {
@@ -772,6 +854,136 @@ int middle_step(grains_gpu_ctx* c, double dt) {
   return move_obstacles(c, dt);
 }
 
+// Runs f(StepArgs, ResArgs) in the context's precision
+template <typename F>
+int with_res(grains_gpu_ctx* c, F f) {
+  if (c->precision == GRAINS_GPU_FP64) return f(make_args<double>(c), make_res<double>(c));
+  return f(make_args<float>(c), make_res<float>(c));
+}
+
+// Whether the uploaded scene can run its middle steps on resident lists:
+// spheres among at most 8 static obstacles a system; cells no smaller than the
+// largest diameter of their system (so that every contact lies in adjacent
+// cells, as the launched broadphase needs); radii within a factor of 4 (the skin
+// is a share of the smallest); list and memory capacities no smaller than a dense
+// packing needs.
+bool res_scene(const grains_gpu_ctx* c) {
+  if (c->n < 1 || c->has_convex || c->n_moving > 0 || c->n_force_obs > 0 || c->clist_cap < 24 ||
+      2 * c->hist_cap < c->clist_cap)
+    return false;
+  if (!(c->r_min > 0) || c->r_max > 4. * c->r_min) return false;
+  for (size_t k = 0; k < c->sys.size(); ++k) {
+    const SysHost& s = c->sys[k];
+    if (s.obs.size() > (size_t)kResObsHost) return false;
+    if (2. * c->sys_r_max[k] > std::min(s.ex, std::min(s.ey, s.ez))) return false;
+  }
+  return true;
+}
+
+// after an upload or a change of the tuning: whether the scene runs on resident
+// lists, and their buffers (kept with the context)
+int ensure_resident(grains_gpu_ctx* c) {
+  c->res_ok = res_scene(c);
+  if (!c->res_ok) return 0;
+  size_t off[9];
+  const size_t need = res_layout(c->cap, res_obs_stride(c), c->hist_cap, c->rsize, off);
+  if (need > c->res_bytes) {
+    if (c->res_buf) cudaFree(c->res_buf);
+    c->res_buf = nullptr;
+    c->res_bytes = 0;
+    void* q = nullptr;
+    CK(cudaMalloc(&q, need));
+    c->res_buf = (char*)q;
+    c->res_bytes = need;
+  }
+  if (!c->res_blocks) {
+    c->res_blocks = c->precision == GRAINS_GPU_FP64 ? res_rebuild_blocks<double>((int)c->cap)
+                                                    : res_rebuild_blocks<float>((int)c->cap);
+    if (c->res_blocks <= 0 || c->res_blocks > 4096)
+      return fail(c, GRAINS_GPU_CUDA_ERROR, "resident lists: occupancy query failed");
+  }
+  return 0;
+}
+
+// The start of a resident run: key and cell_count hold the current positions
+int resident_begin(grains_gpu_ctx* c) {
+  const int rc = with_res(c, [&](auto a, auto r) { return launch_res_begin(a, r, c->stream); });
+  return rc ? fail(c, rc, "resident lists: start failed") : 0;
+}
+
+int resident_step(grains_gpu_ctx* c, double dt, int parity, int phases = 7) {
+  const int rc = with_res(c, [&](auto a, auto r) { return launch_res_step(a, r, c->stream, dt, parity, phases); });
+  return rc ? fail(c, rc, "resident step launch failed") : 0;
+}
+
+// the memories back into the rows, the counts and keys of the new positions
+// where the launched pipeline expects them
+int resident_end(grains_gpu_ctx* c, int parity) {
+  const int rc = with_res(c, [&](auto a, auto r) { return launch_res_end(a, r, c->stream); });
+  if (rc) return fail(c, rc, "resident lists: end failed");
+  if (parity) {
+    CK(cudaMemcpyAsync(c->cell_count, c->cell_count2, (size_t)c->n_cells * sizeof(int), cudaMemcpyDeviceToDevice,
+                       c->stream));
+    CK(cudaMemcpyAsync(c->buf[c->cur].key, c->buf[1 - c->cur].key, (size_t)c->n * sizeof(unsigned),
+                       cudaMemcpyDeviceToDevice, c->stream));
+  }
+  c->keys_valid = true;
+  c->sorted = false;
+  return 0;
+}
+
+// Steps between two gathers of the particle arrays into cell order within a
+// resident run (a gather moves the slots, so the lists are built anew)
+constexpr int kResGather = 512;
+constexpr int kResGraph = 16;  // steps of a graph (even: the parity comes back)
+// A resident run costs the build of its lists and the memories' way back, about
+// as much as two launched steps: shorter runs take those
+constexpr int kResMinSteps = 6;
+
+bool use_resident(const grains_gpu_ctx* c, int middle) {
+  return c->res_ok && !c->persistent && middle >= kResMinSteps;
+}
+
+// n middle steps on resident lists
+int resident_steps(grains_gpu_ctx* c, int n, double dt) {
+  while (n > 0) {
+    int k = std::min(n, kResGather), parity = 0;
+    n -= k;
+    if (int rc = resident_begin(c)) return rc;
+    for (; k >= kResGraph; k -= kResGraph) {
+      const int slot = 2 * c->cur + c->hcur;
+      if (!c->res_graph[slot] || c->res_graph_dt[slot] != dt) {
+        if (c->res_graph[slot]) {
+          cudaGraphExecDestroy(c->res_graph[slot]);
+          c->res_graph[slot] = nullptr;
+        }
+        cudaGraph_t g;
+        CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+        int rc = 0;
+        for (int q = 0; q < kResGraph && !rc; ++q) rc = resident_step(c, dt, q & 1);
+        cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+        if (rc) return rc;
+        if (e != cudaSuccess) return cuda_fail(c, e, "cudaStreamEndCapture");
+        e = cudaGraphInstantiate(&c->res_graph[slot], g, 0);
+        cudaGraphDestroy(g);
+        if (e != cudaSuccess) return cuda_fail(c, e, "cudaGraphInstantiate");
+        c->res_graph_dt[slot] = dt;
+      }
+      CK(cudaGraphLaunch(c->res_graph[slot], c->stream));
+    }
+    for (; k > 0; --k, parity ^= 1)
+      if (int rc = resident_step(c, dt, parity)) return rc;
+    if (int rc = resident_end(c, parity)) return rc;
+    if (n > 0) {  // into cell order, and the counts the next lists start from
+      if (int rc = sort_now(c, 0)) return rc;
+      CK(cudaMemsetAsync(c->cell_count, 0, (size_t)c->n_cells * sizeof(int), c->stream));
+      const int rc = with_args(c, [&](auto& a) { return launch_bin(a, c->stream); });
+      if (rc) return fail(c, rc, "bin kernel launch failed");
+    }
+  }
+  return 0;
+}
+
 // n middle steps in one cooperative launch (persistent_steps_kernel); the
 // host then follows the buffer selection the launch leaves
 int persistent_middle_steps(grains_gpu_ctx* c, int n, double dt) {
@@ -816,13 +1028,23 @@ int last_step(grains_gpu_ctx* c, double dt) {
   return 0;
 }
 
+// the step graphs: they hold buffer pointers, counts and options
+void drop_graphs(grains_gpu_ctx* c) {
+  for (cudaGraphExec_t* g : {c->graph, c->res_graph})
+    for (int k = 0; k < 4; ++k)
+      if (g[k]) {
+        cudaGraphExecDestroy(g[k]);
+        g[k] = nullptr;
+      }
+}
+
 // Contact-list scratch for cap_per entries per particle: the lists, the
 // result of each entry (two R4) and the work items; grown, never shrunk.
 int ensure_lists(grains_gpu_ctx* c, int cap_per) {
   const int64_t need = (int64_t)c->cap * cap_per;
   if (need > c->clist_alloc || (c->has_convex && !c->gjk_out)) {
-    for (void** p : {(void**)&c->clist, &c->res_f, &c->res_t, (void**)&c->work, (void**)&c->gjk_out,
-                     (void**)&c->gjk_order})
+    c->res_t = nullptr;  // the second half of res_f
+    for (void** p : {(void**)&c->clist, &c->res_f, (void**)&c->work, (void**)&c->gjk_out, (void**)&c->gjk_order})
       if (*p) {
         cudaFree(*p);
         *p = nullptr;
@@ -833,10 +1055,9 @@ int ensure_lists(grains_gpu_ctx* c, int cap_per) {
     void* q = nullptr;
     CK(cudaMalloc(&q, (size_t)need * sizeof(int)));
     c->clist = (int*)q;
-    CK(cudaMalloc(&q, (size_t)need * r4));
+    CK(cudaMalloc(&q, 2 * (size_t)need * r4));
     c->res_f = q;
-    CK(cudaMalloc(&q, (size_t)need * r4));
-    c->res_t = q;
+    c->res_t = (char*)q + (size_t)need * r4;
     CK(cudaMalloc(&q, (size_t)need * sizeof(int4)));
     c->work = (int4*)q;
     if (c->has_convex) {  // one narrowphase result per possible work item, their order
@@ -846,11 +1067,7 @@ int ensure_lists(grains_gpu_ctx* c, int cap_per) {
       c->gjk_order = (int*)q;
     }
     c->clist_alloc = need;
-    for (int k = 0; k < 4; ++k)  // graphs hold the old pointers
-      if (c->graph[k]) {
-        cudaGraphExecDestroy(c->graph[k]);
-        c->graph[k] = nullptr;
-      }
+    drop_graphs(c);  // they hold the old pointers
   }
   c->clist_cap = cap_per;
   return 0;
@@ -965,16 +1182,16 @@ int grains_gpu_create(const grains_gpu_config* cfg, grains_gpu_ctx** out) {
 int grains_gpu_destroy(grains_gpu_ctx* c) {
   if (!c) return 0;
   if (c->stream) cudaStreamSynchronize(c->stream);
-  for (int k = 0; k < 4; ++k)
-    if (c->graph[k]) cudaGraphExecDestroy(c->graph[k]);
+  drop_graphs(c);
   for (void* p : c->pool) cudaFree(p);
   for (void* p : c->table_pool) cudaFree(p);
   for (int k = 0; k < 2; ++k)
     if (c->buf[k].basis) cudaFree(c->buf[k].basis);
+  if (c->res_buf) cudaFree(c->res_buf);
   if (c->stage) cudaFree(c->stage);
   if (c->row_scratch) cudaFree(c->row_scratch);
   if (c->d_hydro) cudaFree(c->d_hydro);
-  for (void* p : {(void*)c->clist, (void*)c->ccount, c->res_f, c->res_t, (void*)c->work, (void*)c->gjk_out,
+  for (void* p : {(void*)c->clist, (void*)c->ccount, c->res_f, (void*)c->work, (void*)c->gjk_out,
                   (void*)c->gjk_order})
     if (p) cudaFree(p);
   if (c->pbar) cudaFree(c->pbar);
@@ -1090,16 +1307,6 @@ int grains_gpu_set_obstacles(grains_gpu_ctx* c, int32_t system, int32_t n, const
   c->tables_dirty = true;
   return 0;
 }
-
-namespace {
-void drop_graphs(grains_gpu_ctx* c) {
-  for (int k = 0; k < 4; ++k)
-    if (c->graph[k]) {
-      cudaGraphExecDestroy(c->graph[k]);
-      c->graph[k] = nullptr;
-    }
-}
-}  // namespace
 
 int grains_gpu_set_collision_algorithm(grains_gpu_ctx* c, int32_t algorithm) {
   if (!c) return GRAINS_GPU_INVALID_ARGUMENT;
@@ -1339,6 +1546,9 @@ int build_tables(grains_gpu_ctx* c) {
   CK(cudaMalloc(&p, (size_t)cells * sizeof(int)));
   c->table_pool.push_back(p);
   c->cell_count = (int*)p;
+  CK(cudaMalloc(&p, (size_t)cells * sizeof(int)));
+  c->table_pool.push_back(p);
+  c->cell_count2 = (int*)p;
   CK(cudaMalloc(&p, ((size_t)cells + 1) * sizeof(int)));
   c->table_pool.push_back(p);
   c->cell_start = (int*)p;
@@ -1350,11 +1560,7 @@ int build_tables(grains_gpu_ctx* c) {
   c->block_sums = (int*)p;
   CK(cudaMemsetAsync(c->cell_count, 0, (size_t)cells * sizeof(int), c->stream));
   if (((size_t)cells / 4096 + 1) > 4096) return fail(c, GRAINS_GPU_INVALID_ARGUMENT, "too many cells for the scan");
-  for (int k = 0; k < 4; ++k)
-    if (c->graph[k]) {
-      cudaGraphExecDestroy(c->graph[k]);
-      c->graph[k] = nullptr;
-    }
+  drop_graphs(c);
   return 0;
 }
 }  // namespace
@@ -1395,6 +1601,8 @@ int grains_gpu_upload_particles(grains_gpu_ctx* c, const grains_gpu_particles* p
     if (int rc = build_tables(c)) return rc;
     c->tables_dirty = false;
   }
+  const int64_t n_before = c->n;
+  const bool basis_before = c->has_basis, convex_before = c->has_convex;
   c->has_basis = basis_needed;
   c->has_convex = nonsphere;
   c->all_spheres = !nonsphere;
@@ -1563,6 +1771,21 @@ int grains_gpu_upload_particles(grains_gpu_ctx* c, const grains_gpu_particles* p
   c->sorted = false;
   c->pending_kick2 = false;
   c->uploaded = true;
+  double r_min = n > 0 ? p->radius[0] : 0., r_max = r_min;
+  c->sys_r_max.assign(c->sys.size(), 0.);
+  for (int64_t i = 0; i < n; ++i) {
+    r_min = std::min(r_min, p->radius[i]);
+    r_max = std::max(r_max, p->radius[i]);
+    double& b2 = c->sys_r_max[p->system ? p->system[i] : 0];
+    b2 = std::max(b2, p->radius[i]);
+  }
+  // what the step graphs hold of the last upload
+  if (n != n_before || basis_needed != basis_before || c->has_convex != convex_before || r_min != c->r_min ||
+      r_max != c->r_max)
+    drop_graphs(c);
+  c->r_min = r_min;
+  c->r_max = r_max;
+  if (int rc2 = ensure_resident(c)) return rc2;
   if (int e = sort_now(c, 1)) return e;
   return finish_call(c);
 }
@@ -2227,6 +2450,10 @@ int grains_gpu_step(grains_gpu_ctx* c, int32_t n_steps, double* time, double dt)
   // evaluation and leaves its second half kick pending
   if (int rc = first_move(c, dt, *time)) return rc;
   int middle = n_steps - 1;
+  if (use_resident(c, middle)) {
+    if (int rc = resident_steps(c, middle, dt)) return rc;
+    middle = 0;
+  }
   // the persistent kernel carries Johnson's GJK only: the signed-volume one runs from the graphs
   // (force-driven obstacles need the contact-force sums between the phases:
   // launched steps only)
@@ -2431,6 +2658,7 @@ int grains_gpu_set_barrier_test(grains_gpu_ctx* c, int64_t polls, int32_t skip_b
   if (!c || polls < 1) return GRAINS_GPU_INVALID_ARGUMENT;
   c->barrier_polls = polls;
   c->barrier_skip_block = skip_block < 0 ? -1 : skip_block;
+  drop_graphs(c);
   return 0;
 }
 
@@ -2440,6 +2668,10 @@ int grains_gpu_launches_per_step(grains_gpu_ctx* c, int64_t* launches) {
   // (the GJK kernel of convex scenarios,) pairs, sums with the kick, and the
   // obstacle move when obstacles move; the gather runs one step in
   // gather_every on top
+  if (use_resident(c, kResMinSteps)) {  // the rebuild's check, the pairs, the sums
+    *launches = 3;
+    return 0;
+  }
   *launches = launches_per_middle_step() + (c->has_convex ? 3 : 0) + (c->n_moving > 0 ? 1 : 0) +
                (c->n_force_obs > 0 ? 1 : 0);
   return 0;
@@ -2466,8 +2698,31 @@ int grains_gpu_profile_kernels(grains_gpu_ctx* c, int32_t n_steps, double* time,
   cudaEventElapsedTime(&m, ev[0], ev[1]);
   acc[0] += m;
   cnt[0] += 1;
+  const bool resident = use_resident(c, n_steps - 1);
+  if (resident)
+    if (int rc = resident_begin(c)) return rc;
   for (int k = 0; k < n_steps; ++k) {
     const bool last = (k == n_steps - 1);
+    if (resident && !last) {
+      // a step on resident lists: the rebuild (or its check) counts as the sort,
+      // the overlap tests and the law as the pairs
+      for (int q = 0; q < 3; ++q) {
+        CK(cudaEventRecord(ev[1 + q], c->stream));
+        if (int rc = resident_step(c, dt, k & 1, 1 << q)) return rc;
+      }
+      CK(cudaEventRecord(ev[4], c->stream));
+      CK(cudaEventSynchronize(ev[4]));
+      const int phase[3] = {1, 3, 4};
+      for (int q = 0; q < 3; ++q) {
+        float t = 0;
+        cudaEventElapsedTime(&t, ev[1 + q], ev[2 + q]);
+        acc[phase[q]] += t;
+        cnt[phase[q]] += 1;
+      }
+      if (k == n_steps - 2)
+        if (int rc = resident_end(c, (n_steps - 1) & 1)) return rc;
+      continue;
+    }
     CK(cudaEventRecord(ev[1], c->stream));
     if (int rc = last ? sort_now(c, 0) : sort_for_step(c)) return rc;
     CK(cudaEventRecord(ev[2], c->stream));
@@ -2552,11 +2807,7 @@ int grains_gpu_set_tuning(grains_gpu_ctx* c, const grains_gpu_tuning* t) {
     cudaFree(c->psums);
     c->psums = nullptr;
   }
-  for (int k = 0; k < 4; ++k)  // launch shapes and the gather period are baked into the step graphs
-    if (c->graph[k]) {
-      cudaGraphExecDestroy(c->graph[k]);
-      c->graph[k] = nullptr;
-    }
+  drop_graphs(c);  // launch shapes and the gather period are baked into the step graphs
   for (auto& s : c->sys)
     if (s.has_domain)
       if (int rc = apply_grid(c, s)) return rc;
@@ -2598,6 +2849,7 @@ int grains_gpu_set_tuning(grains_gpu_ctx* c, const grains_gpu_tuning* t) {
   const int cap_per = c->list_capacity > 0 ? c->list_capacity : (c->has_convex ? 64 : 32);
   CK(cudaStreamSynchronize(c->stream));
   if (int rc = ensure_lists(c, cap_per)) return rc;
+  if (int rc = ensure_resident(c)) return rc;
   CK(cudaStreamSynchronize(c->stream));
   return 0;
 }

@@ -243,6 +243,37 @@ struct StepArgs {
   int forces_block;      // threads per block of forces_kernel (<= 128)
 };
 
+// Resident pair lists (resident.cuh): the state of a run of middle steps of
+// spheres among static obstacles.  Lists, results and pair memories use the
+// buffers of the launched pipeline's lists and of the memory rows it is not
+// reading.
+template <typename R>
+struct ResResult;
+template <typename R>
+struct ResArgs {
+  int* ctl;              // control words (kResRequest ...)
+  double* skin;          // the skin of the present lists
+  double skin0, r_max;   // the skin asked for, the largest radius
+  double4* x0;           // positions at the build
+  int2* ent;             // per particle: first entry, entries
+  int* pair_first;       // per particle: its first owned pair
+  int* nb;               // entries: partner's slot, kOwnBit when this particle owns the pair
+  ResResult<R>* res;     // per entry: force and torque on this particle
+  int4* pair;            // pairs: owner's slot, partner's slot, their entries
+  unsigned char* state;  // per pair: contact and memory of the last evaluation
+  R* mem;                // pair memories, 9 arrays of pair_cap
+  int ent_cap, pair_cap;
+  int obs_stride;        // obstacles of the system that has most
+  unsigned long long* obs_state;  // per particle: a state byte per obstacle of its system
+  ResResult<R>* obs_res; // per particle and obstacle
+  R* obs_mem;            // per particle and obstacle: 9 numbers
+  int* obs_item[2];      // obstacle candidates (particle * kResObsMax + obstacle) by the step's parity
+  int* count[2];         // cell counts of the step's positions, by parity
+  int* block_sums;       // scan scratch of the build, one per block
+  unsigned* bar;         // its grid barrier
+  int rebuild_blocks;
+};
+
 // kernel launchers, instantiated for float and double
 template <typename R>
 int launch_kick_move(const StepArgs<R>& a, cudaStream_t s, int do_kick2, double dt_kick2, int do_move,
@@ -307,6 +338,15 @@ int persistent_blocks(const StepArgs<R>& a);
 template <typename R>
 int launch_persistent_steps(const StepArgs<R>& a, cudaStream_t s, int n_steps, double dt, int gather_every,
                             int since_gather, int n_moving, double* clock, unsigned* bar, int* sums, int blocks);
+// steps on resident pair lists; parity: of the step within the run
+template <typename R>
+int res_rebuild_blocks(int n);
+template <typename R>
+int launch_res_begin(const StepArgs<R>& a, const ResArgs<R>& r, cudaStream_t s);
+template <typename R>
+int launch_res_step(const StepArgs<R>& a, const ResArgs<R>& r, cudaStream_t s, double dt, int parity, int phases);
+template <typename R>
+int launch_res_end(const StepArgs<R>& a, const ResArgs<R>& r, cudaStream_t s);
 // number of kernel launches issued by one middle step of grains_gpu_step
 int launches_per_middle_step();
 

@@ -100,7 +100,8 @@ __device__ __forceinline__ V3<R> rk3(bool sphere, V3<R> I, V3<R> Tbf, V3<R> wbf,
 template <typename R>
 __device__ __forceinline__ void integrate(const StepArgs<R>& a, const ParticleArrays<R>& src,
                                           const ParticleArrays<R>& dst, int s, V3<R> F, V3<R> T, int do_kick2,
-                                          R dt_kick2, int do_move, R dt_v, double dt_x) {
+                                          R dt_kick2, int do_move, R dt_v, double dt_x, D3* x_out = nullptr,
+                                          unsigned* key_out = nullptr) {
   double4 xr = src.xr[s];
   const double4 qd = src.q[s];
   const int4 meta = src.meta[s];
@@ -153,6 +154,8 @@ __device__ __forceinline__ void integrate(const StepArgs<R>& a, const ParticleAr
     unsigned key = (unsigned)cell_index(S, ci, cj, ck);
     dst.key[s] = key;
     atomicAdd(&a.cell_count[key], 1);  // result unused: a fire-and-forget reduction
+    if (x_out) *x_out = d3(xr.x, xr.y, xr.z);
+    if (key_out) *key_out = key;
   } else if (a.has_basis && dst.basis != src.basis) {
     for (int t = 0; t < 9; ++t) dst.basis[9 * (size_t)s + t] = src.basis[9 * (size_t)s + t];
   }
@@ -304,11 +307,9 @@ __global__ void __launch_bounds__(256) scatter_kernel(StepArgs<R> a) {
   a.perm[slot] = s;
 }
 
-// order the slots [b, e) of cell c by particle id; resets the count for the
-// next step
+// order the slots [b, e) of a cell by particle id
 template <typename R>
-__device__ __forceinline__ void cell_sort_range(const StepArgs<R>& a, int c, int b, int e) {
-  a.cell_count[c] = 0;
+__device__ __forceinline__ void cell_order(const StepArgs<R>& a, int b, int e) {
   if (b < 0 || e > a.n || b > e) return;
   for (int i = b + 1; i < e; ++i) {
     int pi = a.perm[i];
@@ -320,6 +321,13 @@ __device__ __forceinline__ void cell_sort_range(const StepArgs<R>& a, int c, int
     }
     a.perm[j + 1] = pi;
   }
+}
+
+// order the slots [b, e) of cell c; resets the count for the next step
+template <typename R>
+__device__ __forceinline__ void cell_sort_range(const StepArgs<R>& a, int c, int b, int e) {
+  a.cell_count[c] = 0;
+  cell_order(a, b, e);
 }
 
 // the cell sort of a fully scanned cell list (the persistent kernel's)
@@ -875,6 +883,99 @@ __device__ __forceinline__ void put_memory(const StepArgs<R>& a, int row, int ra
   a.hist_next[(size_t)row * a.hist_cap + rank] = e;
 }
 
+// Contact features of two spheres, with the retry of ContactError; false when
+// they do not touch or the retry failed too.
+template <typename R>
+__device__ __forceinline__ bool sphere_pair_geometry(const StepArgs<R>& a, D3 Xi, double ri, double crust_i, D3 Xj,
+                                                     double rj, double crust_j, ContactGeom& g) {
+  D3 ab;
+  double nab;
+  const double dist = sphere_sphere_overlap(Xi, ri, Xj, rj, &ab, &nab);
+  if (!(dist < 0.)) return false;
+  g = sphere_sphere_features(Xi, ri, ab, nab, dist, xadd(crust_i, crust_j));
+  if (!g.status) return true;
+  bool fatal;
+  g = sphere_sphere_error_handling(Xi, ri, crust_i, Xj, rj, crust_j, fatal);
+  set_status(a.stats, fatal ? GRAINS_GPU_CONTACT_ERROR : GRAINS_GPU_CONTACT_HANDLED);
+  return !fatal;
+}
+
+// The law of a particle pair seen from p0 (i) at the contact features g: the
+// force on p0 and the torques of the contact force about both centres.
+template <typename R>
+__device__ __forceinline__ LawResult<R> particle_pair_law(const LawParams<R>& L, R dt, const ContactGeom& g, D3 Xi,
+                                                          D3 Xj, const double4& mdi, const double4& mdj, V3<R> vi,
+                                                          V3<R> wi, V3<R> vj, V3<R> wj, bool existed,
+                                                          PairMemory<R>& mem, V3<R>& t0, V3<R>& t1) {
+  const D3 lev0 = xsub3(g.point, Xi), lev1 = xsub3(g.point, Xj);
+  BodyAtContact<R> b0, b1;
+  b0.v = vi;
+  b0.w = wi;
+  b0.lever = from_d3<R>(lev0);
+  b0.pos_minus_contact = from_d3<R>(xsub3(Xi, g.point));
+  b0.mass = R(mdi.x);
+  b0.req = R(mdi.z);
+  b1.v = vj;
+  b1.w = wj;
+  b1.lever = from_d3<R>(lev1);
+  b1.pos_minus_contact = from_d3<R>(xsub3(Xj, g.point));
+  b1.mass = R(mdj.x);
+  b1.req = R(mdj.z);
+  PairFp64 pd;
+  if constexpr (sizeof(R) == 4) {
+    pd.v0 = widen(vi);
+    pd.w0 = widen(wi);
+    pd.lev0 = dvec(lev0);
+    pd.v1 = widen(vj);
+    pd.w1 = widen(wj);
+    pd.lev1 = dvec(lev1);
+    pd.m0 = mdi.x;
+    pd.m1 = mdj.x;
+    pd.req0 = mdi.z;
+    pd.req1 = mdj.z;
+  }
+  return pair_law(L, dt, g, b0, b1, pd, existed, mem, t0, t1);
+}
+
+// The law of a particle-obstacle contact: p0 = particle, p1 = obstacle (mass
+// 1e20, velocity at the point, Obstacle.cpp:128-133).
+template <typename R>
+__device__ __forceinline__ LawResult<R> obstacle_law(const LawParams<R>& L, R dt, const ContactGeom& g, D3 Xi,
+                                                     const ObstacleDev& O, const ShapeDev& sho, const double4& mdi,
+                                                     V3<R> vi, V3<R> wi, bool existed, PairMemory<R>& mem, V3<R>& t0,
+                                                     V3<R>& t1) {
+  const D3 oo = d3(O.o[0], O.o[1], O.o[2]);
+  BodyAtContact<R> b0, b1;
+  b0.v = vi;
+  b0.w = wi;
+  b0.lever = from_d3<R>(xsub3(g.point, Xi));
+  b0.pos_minus_contact = from_d3<R>(xsub3(Xi, g.point));
+  b0.mass = R(mdi.x);
+  b0.req = R(mdi.z);
+  // the law adds w x lever to the centre velocity (velocity_at)
+  const D3 olev = xsub3(g.point, oo);
+  b1.v = v3<R>(R(O.vel[0]), R(O.vel[1]), R(O.vel[2]));
+  b1.w = v3<R>(R(O.omega[0]), R(O.omega[1]), R(O.omega[2]));
+  b1.lever = from_d3<R>(olev);
+  b1.pos_minus_contact = from_d3<R>(xsub3(oo, g.point));
+  b1.mass = R(kObstacleMass);
+  b1.req = R(pow((0.75 / kPi) * sho.volume, 1. / 3.));
+  PairFp64 pd;
+  if constexpr (sizeof(R) == 4) {
+    pd.v0 = widen(vi);
+    pd.w0 = widen(wi);
+    pd.lev0 = dvec(xsub3(g.point, Xi));
+    pd.v1 = v3<double>(O.vel[0], O.vel[1], O.vel[2]);
+    pd.w1 = v3<double>(O.omega[0], O.omega[1], O.omega[2]);
+    pd.lev1 = dvec(olev);
+    pd.m0 = mdi.x;
+    pd.m1 = kObstacleMass;
+    pd.req0 = mdi.z;
+    pd.req1 = pow((0.75 / kPi) * sho.volume, 1. / 3.);
+  }
+  return pair_law(L, dt, g, b0, b1, pd, existed, mem, t0, t1);
+}
+
 // B. one owned list entry: particle pair (p0 = this particle, the lower id)
 // or particle-obstacle candidate (p0 = the particle, p1 = the obstacle)
 // GEOM: the narrowphase of general convex pairs comes from the GJK kernel
@@ -924,19 +1025,7 @@ __device__ __forceinline__ void pair_one(const StepArgs<R>& a, int idx, int4 ite
     bool contact = true;
     const double4 mdj = P.md[t];
     if (!CONVEX || (a.shapes[mi.z].type == GRAINS_GPU_SPHERE && a.shapes[mj.z].type == GRAINS_GPU_SPHERE)) {
-      D3 ab;
-      double nab;
-      const double dist = sphere_sphere_overlap(Xi, xi.w, Xj, xj.w, &ab, &nab);
-      contact = dist < 0.;
-      if (contact) {
-        g = sphere_sphere_features(Xi, xi.w, ab, nab, dist, xadd(mdi.y, mdj.y));
-        if (g.status) {
-          bool fatal;
-          g = sphere_sphere_error_handling(Xi, xi.w, mdi.y, Xj, xj.w, mdj.y, fatal);
-          set_status(a.stats, fatal ? GRAINS_GPU_CONTACT_ERROR : GRAINS_GPU_CONTACT_HANDLED);
-          contact = !fatal;
-        }
-      }
+      contact = sphere_pair_geometry(a, Xi, xi.w, mdi.y, Xj, xj.w, mdj.y, g);
     } else if constexpr (GEOM) {
       // the GJK kernel's result for this work item
       g = gjk_result(a.gjk_out[idx]);
@@ -985,39 +1074,12 @@ __device__ __forceinline__ void pair_one(const StepArgs<R>& a, int idx, int4 ite
     }
     if (qp < 0) set_status(a.stats, GRAINS_GPU_PAIR_OVERFLOW);  // the partner's list overflowed
     const V3<R> vj = ld3<R>(P.v[t]), wj = ld3<R>(P.w[t]);
-    const D3 lev0 = xsub3(g.point, Xi), lev1 = xsub3(g.point, Xj);
-    BodyAtContact<R> b0, b1;
-    b0.v = vi;
-    b0.w = wi;
-    b0.lever = from_d3<R>(lev0);
-    b0.pos_minus_contact = from_d3<R>(xsub3(Xi, g.point));
-    b0.mass = R(mdi.x);
-    b0.req = R(mdi.z);
-    b1.v = vj;
-    b1.w = wj;
-    b1.lever = from_d3<R>(lev1);
-    b1.pos_minus_contact = from_d3<R>(xsub3(Xj, g.point));
-    b1.mass = R(mdj.x);
-    b1.req = R(mdj.z);
     const LawParams<R> L = a.laws[S.law_offset + mi.y * S.n_mat + mj.y];
     PairMemory<R> mem;
     bool existed = false;
     if (law_has_memory(L.type)) existed = find_memory(a, oi, keys, mj.x, 0, mem);
-    PairFp64 pd;
-    if constexpr (sizeof(R) == 4) {
-      pd.v0 = widen(vi);
-      pd.w0 = widen(wi);
-      pd.lev0 = dvec(lev0);
-      pd.v1 = widen(vj);
-      pd.w1 = widen(wj);
-      pd.lev1 = dvec(lev1);
-      pd.m0 = mdi.x;
-      pd.m1 = mdj.x;
-      pd.req0 = mdi.z;
-      pd.req1 = mdj.z;
-    }
     V3<R> t0, t1;
-    LawResult<R> res = pair_law(L, dt, g, b0, b1, pd, existed, mem, t0, t1);
+    LawResult<R> res = particle_pair_law(L, dt, g, Xi, Xj, mdi, mdj, vi, wi, vj, wj, existed, mem, t0, t1);
     int flag = 1;
     if (law_has_memory(L.type)) {
       put_memory(a, oi, rank, mj.x, 0, mem);
@@ -1087,42 +1149,13 @@ __device__ __forceinline__ void pair_one(const StepArgs<R>& a, int idx, int4 ite
     put_no_contact(a, my_slot);
     return;
   }
-  // p0 = particle, p1 = obstacle (mass 1e20, velocity at the point, Obstacle.cpp:128-133)
-  BodyAtContact<R> b0, b1;
-  b0.v = vi;
-  b0.w = wi;
-  b0.lever = from_d3<R>(xsub3(g.point, Xi));
-  b0.pos_minus_contact = from_d3<R>(xsub3(Xi, g.point));
-  b0.mass = R(mdi.x);
-  b0.req = R(mdi.z);
-  // the law adds w x lever to the centre velocity (velocity_at)
-  const D3 olev = xsub3(g.point, oo);
-  b1.v = v3<R>(R(O.vel[0]), R(O.vel[1]), R(O.vel[2]));
-  b1.w = v3<R>(R(O.omega[0]), R(O.omega[1]), R(O.omega[2]));
-  b1.lever = from_d3<R>(olev);
-  b1.pos_minus_contact = from_d3<R>(xsub3(oo, g.point));
-  b1.mass = R(kObstacleMass);
-  b1.req = R(pow((0.75 / kPi) * sho.volume, 1. / 3.));
   const LawParams<R> L = a.laws[S.law_offset + mi.y * S.n_mat + O.material];
   PairMemory<R> mem;
   const int oloc = oidx - S.obs_offset;
   bool existed = false;
   if (law_has_memory(L.type)) existed = find_memory(a, oi, keys, oloc, 1, mem);
-  PairFp64 pd;
-  if constexpr (sizeof(R) == 4) {
-    pd.v0 = widen(vi);
-    pd.w0 = widen(wi);
-    pd.lev0 = dvec(xsub3(g.point, Xi));
-    pd.v1 = v3<double>(O.vel[0], O.vel[1], O.vel[2]);
-    pd.w1 = v3<double>(O.omega[0], O.omega[1], O.omega[2]);
-    pd.lev1 = dvec(olev);
-    pd.m0 = mdi.x;
-    pd.m1 = kObstacleMass;
-    pd.req0 = mdi.z;
-    pd.req1 = pow((0.75 / kPi) * sho.volume, 1. / 3.);
-  }
   V3<R> t0, t1;
-  LawResult<R> res = pair_law(L, dt, g, b0, b1, pd, existed, mem, t0, t1);
+  LawResult<R> res = obstacle_law(L, dt, g, Xi, O, sho, mdi, vi, wi, existed, mem, t0, t1);
   int flag = 1;
   if (law_has_memory(L.type)) {
     put_memory(a, oi, rank, oloc, 1, mem);
@@ -1546,6 +1579,17 @@ __global__ void __launch_bounds__(128, CONVEX ? (GEOM ? GG_PAIRS_CONVEX_MIN_BLOC
   pairs_range<R, DIAG, CONVEX, GEOM>(a, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, dt);
 }
 
+// AppPRSHydroFT::ComputeForces (Fluid/src/AppPRSHydroFT.cpp:29-45): the
+// fluid's force and torque, after the contacts (the collision App comes first
+// in Grains::m_allApp)
+template <typename R>
+__device__ __forceinline__ void add_hydro(const StepArgs<R>& a, int row, V3<R>& F, V3<R>& T) {
+  if (!a.hydro) return;
+  const double* h = a.hydro + 6 * (size_t)row;
+  F = F + v3<R>(R(h[0]), R(h[1]), R(h[2]));
+  T = T + v3<R>(R(h[3]), R(h[4]), R(h[5]));
+}
+
 // C. the torsor of particle s: InitializeForces(withWeight) (torsor = weight,
 // Particle.cpp:1409-1416) then every contact in list order; the coordination
 // number; the owner's next memory row packed: an owned entry whose result flag
@@ -1597,14 +1641,7 @@ __device__ __forceinline__ void sum_one(const StepArgs<R>& a, int s, V3<R>* f_ou
       ++ncontact;
     }
   }
-  if (a.hydro) {
-    // AppPRSHydroFT::ComputeForces (Fluid/src/AppPRSHydroFT.cpp:29-45): the
-    // fluid's force and torque, after the contacts (the collision App comes
-    // first in Grains::m_allApp)
-    const double* h = a.hydro + 6 * (size_t)row;
-    F = F + v3<R>(R(h[0]), R(h[1]), R(h[2]));
-    T = T + v3<R>(R(h[3]), R(h[4]), R(h[5]));
-  }
+  add_hydro(a, row, F, T);
   a.coord[s] = ncontact;
   a.hist_n_next[row] = kept;
   if (a.gjk_history) a.gdir_n_next[row] = owned < a.hist_cap ? owned : a.hist_cap;
@@ -2464,6 +2501,8 @@ int launch_persistent_steps(const StepArgs<R>& a, cudaStream_t s, int n_steps, d
   return e == cudaSuccess ? 0 : GRAINS_GPU_CUDA_ERROR;
 }
 
+#include "resident.cuh"
+
 #define GG_INSTANTIATE(R)                                                                                  \
   template int launch_kick_move<R>(const StepArgs<R>&, cudaStream_t, int, double, int, double, double);    \
   template int launch_bin<R>(const StepArgs<R>&, cudaStream_t);                                            \
@@ -2480,6 +2519,10 @@ int launch_persistent_steps(const StepArgs<R>& a, cudaStream_t s, int n_steps, d
   template int launch_candidate_pairs<R>(const StepArgs<R>&, cudaStream_t, int, int, int*, int,           \
                                          unsigned long long*);                                            \
   template int persistent_blocks<R>(const StepArgs<R>&);                                                   \
+  template int res_rebuild_blocks<R>(int);                                                                 \
+  template int launch_res_begin<R>(const StepArgs<R>&, const ResArgs<R>&, cudaStream_t);                   \
+  template int launch_res_end<R>(const StepArgs<R>&, const ResArgs<R>&, cudaStream_t);                     \
+  template int launch_res_step<R>(const StepArgs<R>&, const ResArgs<R>&, cudaStream_t, double, int, int);  \
   template int launch_persistent_steps<R>(const StepArgs<R>&, cudaStream_t, int, double, int, int, int, double*, \
                                           unsigned*, int*, int);
 

@@ -1,0 +1,731 @@
+// resident.cuh -- the middle steps of a run of spheres among static obstacles on
+// resident pair lists (included by kernels.cuh, in namespace gg).
+//
+// The launched pipeline lists every particle's contacts anew in every step:
+// three sort kernels, the 27-cell walk, the search of the partner's list entry
+// and of the pair's memory row.  Here the pairs whose surfaces are closer than a
+// skin are listed once and kept until a particle has moved half the skin, so a
+// pair that is not listed cannot have met.  A step is then three launches:
+//
+//   res_rebuild_kernel  (returns at once unless a particle has moved half the
+//                       skin) cell lists of the current positions, pair lists,
+//                       contact memory carried over
+//   res_pairs_kernel    every listed pair's exact overlap test, the contact law
+//                       of those in contact with the memory in the pair's slot,
+//                       both sides' results; the obstacle candidates; the
+//                       candidate-pair count of the step
+//   res_sums_kernel     per-particle sums in the order of the launched pipeline
+//                       (cell of the partner, then id; obstacles last), kicks,
+//                       drift, cell key and count, the obstacle candidates of
+//                       the new position, the displacement check
+//
+// The results are those of the launched pipeline to the bit: the same contacts
+// (the exact test runs on every listed pair in every step), the same law with
+// the same operands, the same order of sums, the same status bits and counts.
+// The last step of every call runs the launched pipeline, which leaves contact
+// lists, memory rows and coordination as before.
+
+// control words
+enum { kResRequest = 0, kResEntries = 1, kResPairs = 2, kResValid = 3, kResObs = 4, kResWords = 8 };
+// kResRequest: 0 lists are good, 1 a particle has moved half the skin, other
+// values: first build of a run (the memory rows are current)
+// kResEntries, kResPairs: reservations of a build; kResValid: pairs of a
+// complete build, else -1; kResObs, kResObs + 1: obstacle items of the steps of
+// even and odd parity
+
+constexpr int kResObsMax = 8;   // obstacles per system (a byte each in a particle's state word)
+// the state of a listed pair or of a particle's obstacle
+enum { kResContact = 1, kResMemory = 2, kResCandidate = 4 };
+
+// force and torque of one side of a listed pair: one 32-byte sector in mixed precision
+template <typename R>
+struct ResResult {
+  typename Vec4<R>::type f;  // w: 0 no contact, 1 contact, 3 contact whose owner stored a memory
+  typename Vec4<R>::type t;
+};
+
+template <typename R>
+__device__ __forceinline__ PairMemory<R> res_load_memory(const R* m, size_t stride, bool rolling) {
+  PairMemory<R> x;
+  x.kdelta = v3<R>(m[0], m[stride], m[2 * stride]);
+  x.prev_normal = v3<R>(m[3 * stride], m[4 * stride], m[5 * stride]);
+  // without a rolling spring the stored one stays where it is
+  x.spring = rolling ? v3<R>(m[6 * stride], m[7 * stride], m[8 * stride]) : v3<R>(R(0), R(0), R(0));
+  return x;
+}
+template <typename R>
+__device__ __forceinline__ void res_store_memory(R* m, size_t stride, const PairMemory<R>& x, bool spring) {
+  m[0] = x.kdelta.x;
+  m[stride] = x.kdelta.y;
+  m[2 * stride] = x.kdelta.z;
+  m[3 * stride] = x.prev_normal.x;
+  m[4 * stride] = x.prev_normal.y;
+  m[5 * stride] = x.prev_normal.z;
+  if (spring) {
+    m[6 * stride] = x.spring.x;
+    m[7 * stride] = x.spring.y;
+    m[8 * stride] = x.spring.z;
+  }
+}
+
+// ---- the lists ------------------------------------------------------------------
+
+// f(slot, own) for every particle whose surface is closer than `skin` to that of
+// particle s, in the order of (cell, id).  The cells that hold such particles:
+// every centre within r_s + r_max + skin.
+template <typename R, typename F>
+__device__ __forceinline__ void res_walk(const StepArgs<R>& a, const ResArgs<R>& r, int s, double skin, F f) {
+  const double4 xi = a.cur.xr[s];
+  const int4 mi = a.cur.meta[s];
+  const SysDev& S = a.sys[mi.w];
+  const double reach = (xi.w + r.r_max + skin) * (1. + 1.e-9);
+  auto cell = [](double x, double o, double e, int n) { return min(max((int)floor((x - o) / e), 0), n - 1); };
+  const int i0 = cell(xi.x - reach, S.ox, S.ex, S.nbi), i1 = cell(xi.x + reach, S.ox, S.ex, S.nbi);
+  const int j0 = cell(xi.y - reach, S.oy, S.ey, S.nbj), j1 = cell(xi.y + reach, S.oy, S.ey, S.nbj);
+  const int k0 = cell(xi.z - reach, S.oz, S.ez, S.nbk), k1 = cell(xi.z + reach, S.oz, S.ez, S.nbk);
+  for (int j = j0; j <= j1; ++j)
+    for (int k = k0; k <= k1; ++k) {
+      const int b = a.cell_start[cell_index(S, i0, j, k)], e = a.cell_start[cell_index(S, i1, j, k) + 1];
+      for (int q = b; q < e; ++q) {
+        const int t = a.perm[q];
+        const double4 xj = a.cur.xr[t];
+        const double dx = xj.x - xi.x, dy = xj.y - xi.y, dz = xj.z - xi.z;
+        const double rs = (xi.w + xj.w) + skin;  // symmetric: both sides list the pair
+        if (t != s && dx * dx + dy * dy + dz * dz < rs * rs) f(t, mi.x < a.cur.meta[t].x);
+      }
+    }
+}
+
+// the memory of the listed pairs of particle s back into its memory row
+template <typename R>
+__device__ __forceinline__ int res_flush_pairs(const StepArgs<R>& a, const ResArgs<R>& r, int s) {
+  const int2 en = r.ent[s];
+  const int row = a.cur.orig[s];
+  HistEntry<R>* h = a.hist_prev + (size_t)row * a.hist_cap;
+  int cnt = 0;
+  int p = r.pair_first[s];
+  for (int q = 0; q < en.y; ++q) {
+    const int e = r.nb[en.x + q];
+    if (!(e & kOwnBit)) continue;
+    if (r.state[p] & kResMemory) {
+      const PairMemory<R> m = res_load_memory(r.mem + p, (size_t)r.pair_cap, true);
+      if (cnt < a.hist_cap) {
+        HistEntry<R> x;
+        x.other = a.cur.meta[entry_slot(e)].x;
+        x.flags = 0;
+        x.kd[0] = m.kdelta.x; x.kd[1] = m.kdelta.y; x.kd[2] = m.kdelta.z;
+        x.n[0] = m.prev_normal.x; x.n[1] = m.prev_normal.y; x.n[2] = m.prev_normal.z;
+        x.sp[0] = m.spring.x; x.sp[1] = m.spring.y; x.sp[2] = m.spring.z;
+        h[cnt] = x;
+        ++cnt;
+      } else {
+        set_status(a.stats, GRAINS_GPU_HISTORY_FULL);
+      }
+    }
+    ++p;
+  }
+  a.hist_n_prev[row] = cnt;
+  return cnt;
+}
+
+// One cooperative launch: the cell lists, the pair lists, the memory.  Every
+// barrier wait is bounded (grid_barrier); a build that gave up leaves kResValid
+// at -1, on which the other kernels do nothing, and the status bit.
+template <typename R>
+__global__ void __launch_bounds__(256) res_rebuild_kernel(StepArgs<R> a, ResArgs<R> r, int parity) {
+  const int request = *(volatile int*)(r.ctl + kResRequest);
+  if (request == 0 || (*(volatile int*)&a.stats->status & GRAINS_GPU_TIMEOUT)) return;
+  const int nthreads = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = a.n, C = a.n_cells;
+  int* status = &a.stats->status;
+  const int* count = r.count[parity];
+  __shared__ int offset_s;
+  if (request == 1)
+    for (int s = tid; s < n; s += nthreads) res_flush_pairs(a, r, s);
+  // exclusive scan of the cell counts: a chunk per block, then the offsets
+  const int chunk = (C + gridDim.x - 1) / gridDim.x;
+  const int c0 = min(C, (int)blockIdx.x * chunk), c1 = min(C, c0 + chunk);
+  int run = 0;
+  for (int base = c0; base < c1; base += blockDim.x) {
+    const int i = base + threadIdx.x;
+    const int v = i < c1 ? count[i] : 0;
+    int total;
+    const int pre = block_exclusive_scan(v, &total);
+    if (i < c1) a.cell_start[i] = run + pre;
+    run += total;
+  }
+  if (threadIdx.x == 0) r.block_sums[blockIdx.x] = run;
+  if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+  if (tid == 0) {
+    r.ctl[kResValid] = -1;
+    r.ctl[kResEntries] = r.ctl[kResPairs] = 0;
+  }
+  int part = 0;
+  for (int b = threadIdx.x; b < (int)blockIdx.x; b += blockDim.x) part += r.block_sums[b];
+  int before;
+  block_exclusive_scan(part, &before);
+  if (threadIdx.x == 0) {
+    offset_s = before;
+    if (blockIdx.x == gridDim.x - 1) a.cell_start[C] = before + run;
+  }
+  __syncthreads();
+  for (int i = c0 + threadIdx.x; i < c1; i += blockDim.x) {
+    const int v = a.cell_start[i] + offset_s;
+    a.cell_start[i] = v;
+    a.cell_cursor[i] = v;
+  }
+  if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+  for (int s = tid; s < n; s += nthreads) scatter_one(a, s);
+  if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+  for (int c = tid; c < C; c += nthreads) cell_order(a, a.cell_start[c], a.cell_start[c + 1]);
+  if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+  // the lists, with half the skin again when they do not fit
+  double skin = r.skin0;
+  for (;;) {
+    const int padded = (n + nthreads - 1) / nthreads * nthreads;
+    for (int s = tid; s < padded; s += nthreads) {
+      int cnt = 0, own = 0;
+      if (s < n) res_walk(a, r, s, skin, [&](int, bool o) { ++cnt; own += o ? 1 : 0; });
+      const int e0 = warp_reserve(r.ctl + kResEntries, cnt), p0 = warp_reserve(r.ctl + kResPairs, own);
+      if (s >= n) continue;
+      const bool fits = (long long)e0 + cnt <= r.ent_cap && (long long)p0 + own <= r.pair_cap;
+      r.ent[s] = make_int2(fits ? e0 : 0, fits ? cnt : 0);
+      r.pair_first[s] = p0;
+      const double4 x = a.cur.xr[s];
+      r.x0[s] = x;
+      if (!fits) continue;
+      int q = e0, p = p0;
+      res_walk(a, r, s, skin, [&](int t, bool o) {
+        r.nb[q] = t | (o ? kOwnBit : 0);
+        r.res[q].f.w = R(0);
+        if (o) r.pair[p++] = make_int4(s, t, q, -1);
+        ++q;
+      });
+    }
+    if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+    const int ne = *(volatile int*)(r.ctl + kResEntries), np = *(volatile int*)(r.ctl + kResPairs);
+    if (ne <= r.ent_cap && np <= r.pair_cap) break;
+    if (skin < 1.e-3 * r.skin0) {  // more contacts than the lists hold
+      if (tid == 0) set_status(a.stats, GRAINS_GPU_PAIR_OVERFLOW);
+      return;
+    }
+    if (!grid_barrier(r.bar, status, a.barrier_polls)) return;  // every block has read the totals
+    if (tid == 0) r.ctl[kResEntries] = r.ctl[kResPairs] = 0;
+    if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+    skin *= 0.5;
+  }
+  // each pair's entry in the partner's list, and its memory from the owner's row
+  for (int s = tid; s < n; s += nthreads) {
+    const int2 en = r.ent[s];
+    const int row = a.cur.orig[s];
+    const HistEntry<R>* h = a.hist_prev + (size_t)row * a.hist_cap;
+    const int hn = a.hist_n_prev[row];
+    int p = r.pair_first[s];
+    for (int q = 0; q < en.y; ++q) {
+      const int e = r.nb[en.x + q];
+      if (!(e & kOwnBit)) continue;
+      const int t = entry_slot(e);
+      const int2 te = r.ent[t];
+      int other = -1;
+      for (int k = 0; k < te.y; ++k)
+        if (r.nb[te.x + k] == s) other = te.x + k;
+      r.pair[p].w = other;
+      const int id = a.cur.meta[t].x;
+      unsigned char st = 0;
+      for (int k = 0; k < hn; ++k)
+        if (h[k].other == id && h[k].flags == 0) {
+          PairMemory<R> m;
+          m.kdelta = v3<R>(h[k].kd[0], h[k].kd[1], h[k].kd[2]);
+          m.prev_normal = v3<R>(h[k].n[0], h[k].n[1], h[k].n[2]);
+          m.spring = v3<R>(h[k].sp[0], h[k].sp[1], h[k].sp[2]);
+          res_store_memory(r.mem + p, (size_t)r.pair_cap, m, true);
+          st = kResContact | kResMemory;
+          break;
+        }
+      r.state[p] = st;
+      ++p;
+    }
+  }
+  if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+  if (tid == 0) {
+    *r.skin = skin;
+    r.ctl[kResValid] = r.ctl[kResPairs];
+    r.ctl[kResRequest] = 0;
+  }
+}
+
+// ---- obstacles ------------------------------------------------------------------
+// The obstacles linked to the particle's cell whose box meets its sphere's box
+// (the candidates of contacts_one): bit o for the system's obstacle o.
+template <typename R>
+__device__ __forceinline__ unsigned res_obstacle_candidates(const StepArgs<R>& a, const SysDev& S, unsigned key, D3 X,
+                                                            double radius) {
+  unsigned mask = 0;
+  const int b = a.cell_obs_start[key], e = a.cell_obs_start[key + 1];
+  for (int u = b; u < e; ++u) {
+    const int o = a.cell_obs_idx[u];
+    const ObstacleDev& O = a.obs[o];
+    if (in_zone(d3(O.bbc[0], O.bbc[1], O.bbc[2]), d3(O.bbe[0], O.bbe[1], O.bbe[2]), X, radius, radius, radius))
+      mask |= 1u << (o - S.obs_offset);
+  }
+  return mask;
+}
+
+// candidates `mask` of particle s (every lane of the warp calls it, a lane
+// without a particle with an empty mask): items for the evaluation of parity
+// `parity`; returns the state word, in which obstacles that are no candidates
+// have lost their contact
+template <typename R>
+__device__ __forceinline__ unsigned long long res_emit_obstacles(const ResArgs<R>& r, int s, unsigned mask,
+                                                                 unsigned long long state, int parity) {
+  const int base = warp_reserve(r.ctl + kResObs + parity, __popc(mask));
+  unsigned long long next = 0;
+  int k = base;
+  for (unsigned m = mask; m; m &= m - 1) {
+    const int o = __ffs(m) - 1;
+    next |= (((state >> (8 * o)) & (kResContact | kResMemory)) | kResCandidate) << (8 * o);
+    r.obs_item[parity][k++] = s * kResObsMax + o;
+  }
+  return next;
+}
+
+// the start of a run: the obstacle candidates of the current positions and
+// their memory from the rows
+template <typename R>
+__global__ void __launch_bounds__(256) res_begin_kernel(StepArgs<R> a, ResArgs<R> r) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool active = s < a.n;
+  unsigned mask = 0;
+  unsigned long long state = 0;
+  if (active) {
+    const double4 x = a.cur.xr[s];
+    const SysDev& S = a.sys[a.cur.meta[s].w];
+    mask = res_obstacle_candidates(a, S, a.cur.key[s], d3(x.x, x.y, x.z), x.w);
+    const int row = a.cur.orig[s];
+    const HistEntry<R>* h = a.hist_prev + (size_t)row * a.hist_cap;
+    for (int k = a.hist_n_prev[row] - 1; k >= 0; --k) {  // the first of equal entries counts
+      const int o = h[k].other;
+      if (h[k].flags != 1 || o < 0 || o >= S.n_obs || !((mask >> o) & 1)) continue;
+      PairMemory<R> m;
+      m.kdelta = v3<R>(h[k].kd[0], h[k].kd[1], h[k].kd[2]);
+      m.prev_normal = v3<R>(h[k].n[0], h[k].n[1], h[k].n[2]);
+      m.spring = v3<R>(h[k].sp[0], h[k].sp[1], h[k].sp[2]);
+      res_store_memory(r.obs_mem + 9 * ((size_t)s * r.obs_stride + o), 1, m, true);
+      state |= (unsigned long long)(kResContact | kResMemory) << (8 * o);
+    }
+  }
+  const unsigned long long next = res_emit_obstacles(r, s, mask, state, 0);
+  if (active) r.obs_state[s] = next;
+}
+
+// the end of a run: every memory back into the rows, pairs then obstacles
+template <typename R>
+__global__ void __launch_bounds__(256) res_end_kernel(StepArgs<R> a, ResArgs<R> r) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= a.n || *(volatile int*)(r.ctl + kResValid) < 0) return;
+  // before the first build of a run the rows still hold everything
+  int cnt = res_flush_pairs(a, r, s);
+  const int row = a.cur.orig[s];
+  HistEntry<R>* h = a.hist_prev + (size_t)row * a.hist_cap;
+  const unsigned long long state = r.obs_state[s];
+  for (int o = 0; o < kResObsMax; ++o) {
+    if (!((state >> (8 * o)) & kResMemory)) continue;
+    const PairMemory<R> m = res_load_memory(r.obs_mem + 9 * ((size_t)s * r.obs_stride + o), 1, true);
+    if (cnt >= a.hist_cap) {
+      set_status(a.stats, GRAINS_GPU_HISTORY_FULL);
+      break;
+    }
+    HistEntry<R> x;
+    x.other = o;
+    x.flags = 1;
+    x.kd[0] = m.kdelta.x; x.kd[1] = m.kdelta.y; x.kd[2] = m.kdelta.z;
+    x.n[0] = m.prev_normal.x; x.n[1] = m.prev_normal.y; x.n[2] = m.prev_normal.z;
+    x.sp[0] = m.spring.x; x.sp[1] = m.spring.y; x.sp[2] = m.spring.z;
+    h[cnt++] = x;
+  }
+  a.hist_n_prev[row] = cnt;
+}
+
+// ---- pairs ----------------------------------------------------------------------
+constexpr int kResPairThreads = 128;
+constexpr int kResPairTile = 256;
+
+template <typename R>
+__device__ __forceinline__ void res_no_contact(const ResArgs<R>& r, int p, int4 pr, unsigned char st) {
+  if (!st) return;
+  r.state[p] = 0;
+  r.res[pr.z].f.w = R(0);
+  if (pr.w >= 0) r.res[pr.w].f.w = R(0);
+}
+
+// the contact law of listed pair p (in contact: the overlap test has passed)
+template <typename R>
+__device__ __forceinline__ void res_pair_one(const StepArgs<R>& a, const ResArgs<R>& r, int p, R dt, ForceStats& fs) {
+  const ParticleArrays<R>& P = a.cur;
+  const int4 pr = r.pair[p];
+  const int s = pr.x, t = pr.y;
+  const double4 xi = P.xr[s], xj = P.xr[t];
+  const int4 mi = P.meta[s], mj = P.meta[t];
+  const double4 mdi = P.md[s], mdj = P.md[t];
+  const V3<R> vi = ld3<R>(P.v[s]), wi = ld3<R>(P.w[s]);
+  const V3<R> vj = ld3<R>(P.v[t]), wj = ld3<R>(P.w[t]);
+  const unsigned char st = r.state[p];
+  const SysDev& S = a.sys[mi.w];
+  const LawParams<R> L = a.laws[S.law_offset + mi.y * S.n_mat + mj.y];
+  const bool memory = law_has_memory(L.type);
+  PairMemory<R> mem;
+  const bool existed = memory && (st & kResMemory);
+  if (existed) mem = res_load_memory(r.mem + p, (size_t)r.pair_cap, L.rolling != 0);
+  const D3 Xi = d3(xi.x, xi.y, xi.z), Xj = d3(xj.x, xj.y, xj.z);
+  ContactGeom g;
+  if (!sphere_pair_geometry(a, Xi, xi.w, mdi.y, Xj, xj.w, mdj.y, g)) {
+    res_no_contact(r, p, pr, st);
+    return;
+  }
+  V3<R> t0, t1;
+  const LawResult<R> res = particle_pair_law(L, dt, g, Xi, Xj, mdi, mdj, vi, wi, vj, wj, existed, mem, t0, t1);
+  if (memory) res_store_memory(r.mem + p, (size_t)r.pair_cap, mem, L.rolling != 0 || !existed);
+  const int now = memory ? kResContact | kResMemory : kResContact;
+  if (st != now) r.state[p] = (unsigned char)now;
+  if (law_has_torque(L)) {
+    t0 = t0 + res.torque;
+    t1 = t1 + (-res.torque);
+  }
+  r.res[pr.z].f = st3<R>(res.force, R(memory ? 3 : 1));
+  r.res[pr.z].t = st3<R>(t0);
+  if (pr.w >= 0) {
+    r.res[pr.w].f = st3<R>(-res.force, R(1));
+    r.res[pr.w].t = st3<R>(t1);
+  }
+  ++fs.ncont_own;
+  const double o = fabs(g.overlap);
+  fs.ov_sum += o;
+  fs.ov_max = fmax(fs.ov_max, o);
+}
+
+// one obstacle candidate (pair_one's obstacle part on resident memory)
+template <typename R>
+__device__ __forceinline__ void res_obstacle_one(const StepArgs<R>& a, const ResArgs<R>& r, int item, R dt,
+                                                 ForceStats& fs) {
+  const ParticleArrays<R>& P = a.cur;
+  const int s = item / kResObsMax, o = item % kResObsMax;
+  const double4 xi = P.xr[s];
+  const int4 mi = P.meta[s];
+  const double4 mdi = P.md[s];
+  const V3<R> vi = ld3<R>(P.v[s]), wi = ld3<R>(P.w[s]);
+  unsigned char* state = reinterpret_cast<unsigned char*>(r.obs_state + s) + o;
+  const unsigned char st = *state;
+  const SysDev& S = a.sys[mi.w];
+  const ObstacleDev& O = a.obs[S.obs_offset + o];
+  const size_t at = (size_t)s * r.obs_stride + o;
+  const D3 Xi = d3(xi.x, xi.y, xi.z);
+  const ShapeDev& sho = a.shapes[O.shape];
+  M3 ob;
+  for (int k = 0; k < 9; ++k) ob.m[k] = O.b[k];
+  ContactGeom g = sphere_box(Xi, xi.w, xadd(mdi.y, O.crust), ob, d3(O.o[0], O.o[1], O.o[2]),
+                             d3(sho.ext[0], sho.ext[1], sho.ext[2]));
+  if (g.status) {
+    set_status(a.stats, GRAINS_GPU_CONTACT_ERROR);
+    g.overlap = 1.;
+  }
+  if (!(g.overlap < 0.)) {
+    if (st != kResCandidate) *state = kResCandidate;
+    return;
+  }
+  const LawParams<R> L = a.laws[S.law_offset + mi.y * S.n_mat + O.material];
+  const bool memory = law_has_memory(L.type);
+  PairMemory<R> mem;
+  const bool existed = memory && (st & kResMemory);
+  if (existed) mem = res_load_memory(r.obs_mem + 9 * at, 1, L.rolling != 0);
+  V3<R> t0, t1;
+  const LawResult<R> res = obstacle_law(L, dt, g, Xi, O, sho, mdi, vi, wi, existed, mem, t0, t1);
+  if (memory) res_store_memory(r.obs_mem + 9 * at, 1, mem, L.rolling != 0 || !existed);
+  const int now = kResCandidate | kResContact | (memory ? kResMemory : 0);
+  if (st != now) *state = (unsigned char)now;
+  if (law_has_torque(L)) t0 = t0 + res.torque;
+  r.obs_res[at].f = st3<R>(res.force, R(memory ? 3 : 1));
+  r.obs_res[at].t = st3<R>(t0);
+  ++fs.nobs_cont;
+  const double ov = fabs(g.overlap);
+  fs.ov_sum += ov;
+  fs.ov_max = fmax(fs.ov_max, ov);
+}
+
+// Blocks [0, pair_blocks): the listed pairs, a tile at a time: the exact overlap
+// test of every pair (two per thread, their loads in flight together), those in
+// contact packed in shared memory, then the law on the packed ones, so that the
+// law runs on full warps whatever share of the list is in contact.  Then
+// obs_blocks: the obstacle candidates; the other blocks: the number of candidate
+// pairs of the step (the 27 cells around every particle, as the launched
+// broadphase counts them), and the cell counts of the next step cleared.
+template <typename R>
+__global__ void __launch_bounds__(kResPairThreads, GG_PAIRS_MIN_BLOCKS)
+    res_pairs_kernel(StepArgs<R> a, ResArgs<R> r, R dt, int parity, int pair_blocks, int obs_blocks) {
+  __shared__ int list[kResPairTile];
+  __shared__ int n_list;
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  ForceStats fs{0, 0, 0, 0, 0., 0.};
+  if ((int)blockIdx.x < pair_blocks) {
+    const int n_pairs = *(volatile int*)(r.ctl + kResValid);
+    for (int base = blockIdx.x * kResPairTile; base < n_pairs; base += pair_blocks * kResPairTile) {
+      if (threadIdx.x == 0) n_list = 0;
+      __syncthreads();
+      int4 pr[2];
+      double4 xi[2], xj[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int p = base + u * kResPairThreads + threadIdx.x;
+        pr[u] = p < n_pairs ? r.pair[p] : make_int4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        xi[u] = a.cur.xr[pr[u].x];
+        xj[u] = a.cur.xr[pr[u].y];
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int p = base + u * kResPairThreads + threadIdx.x;
+        bool contact = false;
+        if (p < n_pairs) {
+          const double dx = xj[u].x - xi[u].x, dy = xj[u].y - xi[u].y, dz = xj[u].z - xi[u].z;
+          const double rs = xi[u].w + xj[u].w;
+          if (!(dx * dx + dy * dy + dz * dz > rs * rs * (1. + 1.e-12))) {  // as in contacts_one
+            D3 ab;
+            double nab;
+            contact = sphere_sphere_overlap(d3(xi[u].x, xi[u].y, xi[u].z), xi[u].w, d3(xj[u].x, xj[u].y, xj[u].z),
+                                            xj[u].w, &ab, &nab) < 0.;
+          }
+          if (!contact) res_no_contact(r, p, pr[u], r.state[p]);
+        }
+        const unsigned hit = __ballot_sync(full, contact);
+        int at = 0;
+        if (lane == 0 && hit) at = atomicAdd(&n_list, __popc(hit));
+        at = __shfl_sync(full, at, 0);
+        if (contact) list[at + __popc(hit & ((1u << lane) - 1u))] = p;
+      }
+      __syncthreads();
+      for (int k = threadIdx.x; k < n_list; k += kResPairThreads) res_pair_one(a, r, list[k], dt, fs);
+      __syncthreads();
+    }
+    flush_force_stats(a.stats, fs);
+  } else if ((int)blockIdx.x < pair_blocks + obs_blocks) {
+    const int n_items = *(volatile int*)(r.ctl + kResObs + parity);
+    const int b = blockIdx.x - pair_blocks;
+    for (int k = b * kResPairThreads + threadIdx.x; k < n_items; k += obs_blocks * kResPairThreads)
+      res_obstacle_one(a, r, r.obs_item[parity][k], dt, fs);
+    if (b == 0 && threadIdx.x == 0) {
+      if (n_items > 0) atomicAdd(&a.stats->n_obs_cand, (unsigned long long)n_items);
+      r.ctl[kResObs + 1 - parity] = 0;  // the sums kernel fills the next step's list
+    }
+    flush_force_stats(a.stats, fs);
+  } else {
+    const int* count = r.count[parity];
+    int* next = r.count[1 - parity];
+    const int blocks = gridDim.x - pair_blocks - obs_blocks;
+    unsigned long long cand = 0;
+    for (int c = (blockIdx.x - pair_blocks - obs_blocks) * kResPairThreads + threadIdx.x; c < a.n_cells;
+         c += blocks * kResPairThreads) {
+      next[c] = 0;
+      const int own = count[c];
+      if (own == 0) continue;
+      int sys = 0;
+      for (int hi = a.n_sys; hi - sys > 1;) {  // the cell's system
+        const int mid = (sys + hi) / 2;
+        if (a.sys[mid].cell_offset <= c) sys = mid;
+        else hi = mid;
+      }
+      const SysDev& S = a.sys[sys];
+      const int local = c - S.cell_offset;
+      const int i = local % S.nbi, k = (local / S.nbi) % S.nbk, j = local / (S.nbi * S.nbk);
+      int around = 0;
+#pragma unroll
+      for (int q = 0; q < 27; ++q) {
+        const int ii = i + q % 3 - 1, kk = k + (q / 3) % 3 - 1, jj = j + q / 9 - 1;
+        if (ii >= 0 && ii < S.nbi && jj >= 0 && jj < S.nbj && kk >= 0 && kk < S.nbk)
+          around += count[cell_index(S, ii, jj, kk)];
+      }
+      cand += (unsigned long long)own * (unsigned long long)(around - 1);
+    }
+    warp_add(&a.stats->n_cand, cand);
+  }
+}
+
+// ---- sums -----------------------------------------------------------------------
+// The torsor of particle s from the results of its list entries in the order of
+// (cell of the partner, id), as the launched pipeline lists them; then its
+// obstacles, the fluid, the kicks, the drift and the next step's candidates.
+template <typename R>
+__global__ void __launch_bounds__(256) res_sums_kernel(StepArgs<R> a, ResArgs<R> r, R dt_half, double dt, int parity) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool active = s < a.n && *(volatile int*)(r.ctl + kResValid) >= 0;
+  const ParticleArrays<R>& P = a.cur;
+  unsigned mask = 0;
+  unsigned long long state = 0;
+  if (active) {
+    const int4 meta = P.meta[s];
+    const double4 md = P.md[s];
+    const double mass = md.x * (1. - md.w);  // Particle::computeWeight, as in sum_one
+    const SysDev& S = a.sys[meta.w];
+    V3<R> F = v3<R>(R(S.gx * mass), R(S.gy * mass), R(S.gz * mass));
+    V3<R> T = v3<R>(R(0), R(0), R(0));
+    const int2 en = r.ent[s];
+    state = r.obs_state[s];
+    int listed = 0, owned = 0;
+    bool full = false;  // a memory beyond the row
+    auto add = [&](const ResResult<R>& x, bool own) {
+      F = F + ld3<R>(x.f);
+      T = T + ld3<R>(x.t);
+      ++listed;
+      if (own) full = full || (x.f.w == R(3) && owned >= a.hist_cap);
+      owned += own ? 1 : 0;
+    };
+    // entries keep the order of their build; a partner that has crossed into
+    // another cell since may have changed it
+    const V3<R> F0 = F;
+    unsigned last_key = 0;
+    int last_entry = 0;
+    bool ordered = true;
+    for (int q0 = 0; q0 < en.y; q0 += 4) {
+      ResResult<R> x[4];
+      int e[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (q0 + u < en.y) {
+          x[u] = r.res[en.x + q0 + u];
+          e[u] = r.nb[en.x + q0 + u];
+        }
+      unsigned key[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (q0 + u < en.y && x[u].f.w != R(0)) key[u] = P.key[entry_slot(e[u])];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (q0 + u >= en.y || x[u].f.w == R(0)) continue;
+        if (listed > 0 && key[u] <= last_key &&
+            (key[u] < last_key || P.meta[entry_slot(e[u])].x < P.meta[entry_slot(last_entry)].x))
+          ordered = false;
+        last_entry = e[u];
+        last_key = key[u];
+        add(x[u], (e[u] & kOwnBit) != 0);
+      }
+    }
+    if (!ordered) {
+      F = F0;
+      T = v3<R>(R(0), R(0), R(0));
+      listed = owned = 0;
+      full = false;
+      bool any = false;
+      unsigned long long done = 0;  // (cell, id) of the last one added
+      for (;;) {
+        unsigned long long least = ~0ull;
+        int at = -1;
+        for (int q = 0; q < en.y; ++q) {
+          if (r.res[en.x + q].f.w == R(0)) continue;
+          const int t = entry_slot(r.nb[en.x + q]);
+          const unsigned long long k = ((unsigned long long)P.key[t] << 32) | ((unsigned)P.meta[t].x ^ 0x80000000u);
+          if ((!any || k > done) && k < least) {
+            least = k;
+            at = q;
+          }
+        }
+        if (at < 0) break;
+        add(r.res[en.x + at], (r.nb[en.x + at] & kOwnBit) != 0);
+        done = least;
+        any = true;
+      }
+    }
+    int n_cand = 0;
+    for (unsigned long long m = state; m; ) {
+      const int o = (__ffsll((long long)m) - 1) / 8;
+      const unsigned b = (unsigned)(m >> (8 * o)) & 255u;
+      m &= ~(255ull << (8 * o));
+      if (!(b & kResCandidate)) continue;
+      ++n_cand;
+      if (b & kResContact) {
+        const ResResult<R> x = r.obs_res[(size_t)s * r.obs_stride + o];
+        F = F + ld3<R>(x.f);
+        T = T + ld3<R>(x.t);
+        full = full || (x.f.w == R(3) && owned >= a.hist_cap);
+      }
+      ++owned;
+    }
+    if (listed + n_cand > a.clist_cap) set_status(a.stats, GRAINS_GPU_PAIR_OVERFLOW);
+    if (full) set_status(a.stats, GRAINS_GPU_HISTORY_FULL);
+    add_hydro(a, P.orig[s], F, T);
+    D3 X;
+    unsigned key;
+    // partners still read this particle's present cell: the new one goes to the
+    // other key array
+    ParticleArrays<R> D = P;
+    D.key = a.alt.key;
+    integrate(a, P, D, s, F, T, 1, dt_half, 1, dt_half, dt, &X, &key);
+    const double4 x0 = r.x0[s];
+    const double dx = X.x - x0.x, dy = X.y - x0.y, dz = X.z - x0.z;
+    const double half = *r.skin * (0.5 * (1. - 1.e-9));
+    if (!(dx * dx + dy * dy + dz * dz < half * half)) r.ctl[kResRequest] = 1;
+    mask = res_obstacle_candidates(a, S, key, X, x0.w);
+  }
+  const unsigned long long next = res_emit_obstacles(r, s, mask, state, 1 - parity);
+  if (active && next != state) r.obs_state[s] = next;
+}
+
+// ---- launchers ------------------------------------------------------------------
+template <typename R>
+int res_rebuild_blocks(int n) {
+  int dev = 0, sms = 0, per_sm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, res_rebuild_kernel<R>, 256, 0) != cudaSuccess ||
+      per_sm < 1)
+    return 0;
+  const int need = grid_for(n, 256);
+  return std::max(1, std::min(std::min(per_sm, 2) * sms, need));
+}
+
+template <typename R>
+int launch_res_begin(const StepArgs<R>& a, const ResArgs<R>& r, cudaStream_t s) {
+  if (cudaMemsetAsync(r.ctl, 0, kResWords * sizeof(int), s) != cudaSuccess) return GRAINS_GPU_CUDA_ERROR;
+  if (cudaMemsetAsync(r.bar, 0, 2 * sizeof(unsigned), s) != cudaSuccess) return GRAINS_GPU_CUDA_ERROR;
+  if (cudaMemsetAsync(r.ctl + kResRequest, 2, sizeof(int), s) != cudaSuccess) return GRAINS_GPU_CUDA_ERROR;
+  if (cudaMemsetAsync(r.ctl + kResValid, 255, sizeof(int), s) != cudaSuccess) return GRAINS_GPU_CUDA_ERROR;
+  res_begin_kernel<R><<<grid_for(a.n, 256), 256, 0, s>>>(a, r);
+  return check_launch();
+}
+
+template <typename R>
+int launch_res_end(const StepArgs<R>& a, const ResArgs<R>& r, cudaStream_t s) {
+  res_end_kernel<R><<<grid_for(a.n, 256), 256, 0, s>>>(a, r);
+  return check_launch();
+}
+
+// phases (bits): 1 = rebuild when asked for, 2 = pairs, 4 = sums and kick.  The
+// cell keys alternate between the two particle buffers: a.cur.key holds those of
+// the step's positions, a.alt.key takes the next ones.
+template <typename R>
+int launch_res_step(const StepArgs<R>& args, const ResArgs<R>& r, cudaStream_t s, double dt, int parity, int phases) {
+  StepArgs<R> a = args;
+  if (parity) std::swap(a.cur.key, a.alt.key);
+  if (phases & 1) {
+    StepArgs<R> a0 = a;
+    ResArgs<R> r0 = r;
+    void* kargs[] = {&a0, &r0, &parity};
+    if (cudaLaunchCooperativeKernel((const void*)res_rebuild_kernel<R>, dim3(r.rebuild_blocks), dim3(256), kargs, 0,
+                                    s) != cudaSuccess)
+      return GRAINS_GPU_CUDA_ERROR;
+  }
+  if (phases & 2) {
+    // every SM filled once by the pair blocks (four per SM), fewer when the lists (about 5 pairs a particle) are
+    // short; the obstacle and count blocks follow them
+    const int pb = std::min(4 * 148, grid_for(5ll * a.n, kResPairTile));
+    const int ob = std::min(148, grid_for(a.n, 4 * kResPairThreads));
+    const int cb = std::min(2 * 148, grid_for(a.n_cells, kResPairThreads));
+    res_pairs_kernel<R><<<pb + ob + cb, kResPairThreads, 0, s>>>(a, r, R(dt), parity, pb, ob);
+  }
+  if (phases & 4) {
+    StepArgs<R> an = a;
+    an.cell_count = r.count[1 - parity];  // the drift counts the new cells for the next step
+    res_sums_kernel<R><<<grid_for(a.n, 256), 256, 0, s>>>(an, r, R(0.5 * dt), dt, parity);
+  }
+  return check_launch();
+}

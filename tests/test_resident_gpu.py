@@ -1,0 +1,124 @@
+"""Steps on resident pair lists (spheres among static obstacles) against the
+launched pipeline, which lists the contacts anew in every step: the same bits in
+every field, the same contact memory, counts and status.  A list capacity below
+24, or above twice the memory capacity (24), keeps a context on the launched
+pipeline and changes nothing else."""
+import numpy as np
+import pytest
+
+from pacific_b200 import scenarios as S
+from pacific_b200.abi import FP64, HERTZ_MEMORY, HOOKE, HOOKE_MEMORY, MIXED
+
+from helpers import make
+
+pytestmark = pytest.mark.gpu
+
+TUNING = dict(cell_factor=1.0, contacts_block=256, forces_block=128, gather_every=16)
+LAWS = {
+    "memory": None,  # the scenario's HookeMemory
+    "rolling": (HOOKE_MEMORY, [1.0e5, 0.9, -1.0, 0.5, 0.8e5, 0.05, 0.1, 0.0]),
+    "none": (HOOKE, [1.0e5, 0.9, -1.0, 0.5, 1.0e-3]),
+    "hertz": (HERTZ_MEMORY, [2.0e8, 0.9, 0.5, 6.0e7, 0.05, 0.1, 0.0]),
+}
+
+
+def with_law(sc, law):
+    if LAWS[law] is not None:
+        sc.laws = [[(a, b, *LAWS[law]) for a, b, _, _ in laws] for laws in sc.laws]
+    return sc
+
+
+def run(lib, sc, precision, steps, capacity, resident, basis=False, factor=1.0):
+    if basis:
+        sc.particles["basis"] = S.quaternion_basis(sc.particles["quaternion"])
+    sim = make(lib, sc, precision)
+    sim.set_tuning(**{**TUNING, "cell_factor": factor}, list_capacity=capacity)
+    assert (sim.launches_per_step() == 3) == resident
+    sim.initialize_leapfrog(0.0, sc.dt)
+    out, t = [], 0.0
+    for n in steps:
+        t = sim.step(n, t, sc.dt)
+        d, m = sim.download(), sim.contact_memory()
+        order = np.lexsort((m["other"], m["owner"], m["system"]))
+        out.append({**d, **{"memory " + k: v[order] for k, v in m.items()}})
+    sim.synchronize()
+    st = sim.stats()
+    sim.close()
+    return out, st
+
+
+def check(lib, sc, precision, steps, capacities=(32, 20), **kw):
+    a, sa = run(lib, sc, precision, steps, capacities[0], True, **kw)
+    b, sb = run(lib, sc, precision, steps, capacities[1], False, **kw)
+    for x, y in zip(a, b):
+        for k in x:
+            assert np.array_equal(x[k], y[k]), k
+    for k in sa:
+        if k in ("overlap_sum", "overlap_mean"):  # summed by atomics, in any order
+            assert abs(sa[k] - sb[k]) <= 1e-12 * abs(sb[k])
+        else:
+            assert sa[k] == sb[k], k
+    return a, sa
+
+
+# 7 steps: the shortest resident run; 8: an odd number of middle steps; 40: graphs and a remainder
+@pytest.mark.parametrize("precision", [FP64, MIXED])
+@pytest.mark.parametrize("law", list(LAWS))
+@pytest.mark.parametrize("n", [1, 2, 33, 257, 1000])
+def test_same_bits_as_the_launched_pipeline(gpu_lib, n, law, precision):
+    sc = with_law(S.small_box(n, seed=n, velocity_sigma=0.3, radius_range=(0.95, 1.05), spacing=2.07), law)
+    sc.dt = 5.0e-6
+    check(gpu_lib, sc, precision, (7, 8, 40))
+
+
+def test_lists_are_rebuilt_and_regathered(gpu_lib):
+    """Fast spheres cross cells and half the skin many times; a run longer than
+    the gather period."""
+    sc = S.small_box(700, seed=3, velocity_sigma=1.5, radius_range=(0.7, 1.3), spacing=2.7, jitter=0.05)
+    sc.dt = 2.0e-6
+    _, st = check(gpu_lib, sc, MIXED, (1100, 530))
+    assert st["n_contacts"] > 0
+
+
+@pytest.mark.parametrize("factor", [1.0, 1.5])
+def test_bases_systems_and_wide_cells(gpu_lib, factor):
+    """Several systems with their own laws, given bases, cells wider than the
+    largest diameter."""
+    sc = S.ensemble_512(n_systems=5, n_min=40, n_max=900)
+    rng = np.random.default_rng(1)
+    sc.particles["velocity"] = rng.normal(0.0, 0.5, sc.particles["velocity"].shape)
+    sc.particles["omega"] = rng.normal(0.0, 20.0, sc.particles["omega"].shape)
+    check(gpu_lib, sc, FP64, (200,), basis=True, factor=factor)
+
+
+def test_crowded_lists_take_a_thinner_skin(gpu_lib):
+    """A lattice so tight that every inner sphere touches 32 others (the list
+    capacity) and has 56 within the skin: the build halves the skin until the
+    lists hold the entries."""
+    rng = np.random.default_rng(2)
+    n, side, spacing = 1000, 10, 0.777e-3
+    sc = S.small_box(n, seed=1, velocity_sigma=0.01)
+    sc.laws = [[(a, b, HOOKE_MEMORY, [1.0e2, 0.9, -1.0, 0.5, 0.8e2, 0.0, 0.0, 0.0]) for a, b, _, _ in sc.laws[0]]]
+    k = np.arange(n)
+    sc.particles["radius"][:] = 0.79e-3
+    sc.particles["crust"][:] = 0.45e-3  # overlaps of 0.8 mm are no ContactError
+    sc.particles["position"] = 2.5e-3 + spacing * np.stack([k % side, k // side % side, k // side ** 2], 1)
+    sc.particles["position"] += rng.uniform(-0.5e-6, 0.5e-6, (n, 3))
+    sc.obstacles = [[]]
+    sc.domains[0]["gravity"] = (0.0, 0.0, 0.0)
+    sc.dt = 1.0e-7
+    out, _ = check(gpu_lib, sc, FP64, (12,), capacities=(32, 52))
+    assert out[0]["coordination"].max() == 32
+
+
+def test_what_does_not_run_on_resident_lists(gpu_lib):
+    """Convex bodies, moving obstacles and radii far apart stay on the launched
+    pipeline."""
+    far = S.small_box(30, seed=1, radius_range=(0.2, 1.0))
+    for sc in (S.convex_box(27, seed=1), S.pressed_box(27), far):
+        sim = make(gpu_lib, sc, FP64)
+        assert sim.launches_per_step() > 3
+        sim.initialize_leapfrog(0.0, sc.dt)
+        sim.step(9, 0.0, sc.dt)
+        sim.synchronize()
+        sim.close()
