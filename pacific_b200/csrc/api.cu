@@ -655,7 +655,7 @@ StepArgs<R> make_args(grains_gpu_ctx* c) {
 // pipeline's.
 constexpr size_t kResAlign = 256;
 constexpr int kResObsHost = 8;  // obstacles per system the state word holds
-size_t res_layout(int64_t cap, int obs_stride, int hist_cap, size_t rsize, size_t off[9]) {
+size_t res_layout(int64_t cap, int obs_stride, int hist_cap, size_t n_sys, size_t rsize, size_t off[10]) {
   size_t at = 0;
   auto put = [&](int k, size_t bytes) {
     off[k] = at;
@@ -671,6 +671,7 @@ size_t res_layout(int64_t cap, int obs_stride, int hist_cap, size_t rsize, size_
   put(6, m * 9 * rsize);
   put(7, 2 * m * sizeof(int));
   put(8, n * (size_t)hist_cap);
+  put(9, n_sys * sizeof(double));
   return at;
 }
 
@@ -683,9 +684,9 @@ int res_obs_stride(const grains_gpu_ctx* c) {
 template <typename R>
 ResArgs<R> make_res(grains_gpu_ctx* c) {
   ResArgs<R> r{};
-  size_t off[9];
+  size_t off[10];
   const int stride = res_obs_stride(c);
-  res_layout(c->cap, stride, c->hist_cap, c->rsize, off);
+  res_layout(c->cap, stride, c->hist_cap, c->sys.size(), c->rsize, off);
   char* b = c->res_buf;
   r.ctl = (int*)(b + off[0]);
   r.bar = (unsigned*)(r.ctl + 16);
@@ -694,7 +695,7 @@ ResArgs<R> make_res(grains_gpu_ctx* c) {
   // a wide skin lasts longer but lists more pairs: 0.2 r_min (a tenth of a
   // diameter) lists 8 to 9 partners a particle in a dense bed, of which 5 touch
   r.skin0 = 0.2 * c->r_min;
-  r.r_max = c->r_max;
+  r.r_max = (const double*)(b + off[9]);
   r.x0 = (double4*)(b + off[1]);
   r.ent = (int2*)(b + off[2]);
   r.pair_first = (int*)(b + off[3]);
@@ -885,8 +886,8 @@ bool res_scene(const grains_gpu_ctx* c) {
 int ensure_resident(grains_gpu_ctx* c) {
   c->res_ok = res_scene(c);
   if (!c->res_ok) return 0;
-  size_t off[9];
-  const size_t need = res_layout(c->cap, res_obs_stride(c), c->hist_cap, c->rsize, off);
+  size_t off[10];
+  const size_t need = res_layout(c->cap, res_obs_stride(c), c->hist_cap, c->sys.size(), c->rsize, off);
   if (need > c->res_bytes) {
     if (c->res_buf) cudaFree(c->res_buf);
     c->res_buf = nullptr;
@@ -896,6 +897,9 @@ int ensure_resident(grains_gpu_ctx* c) {
     c->res_buf = (char*)q;
     c->res_bytes = need;
   }
+  CK(cudaMemcpyAsync(c->res_buf + off[9], c->sys_r_max.data(), c->sys_r_max.size() * sizeof(double),
+                     cudaMemcpyHostToDevice, c->stream));
+  CK(cudaStreamSynchronize(c->stream));  // pageable host memory
   if (!c->res_blocks) {
     c->res_blocks = c->precision == GRAINS_GPU_FP64 ? res_rebuild_blocks<double>((int)c->cap)
                                                     : res_rebuild_blocks<float>((int)c->cap);

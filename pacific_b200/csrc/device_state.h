@@ -253,7 +253,8 @@ template <typename R>
 struct ResArgs {
   int* ctl;              // control words (kResRequest ...)
   double* skin;          // the skin of the present lists
-  double skin0, r_max;   // the skin asked for, the largest radius
+  double skin0;          // the skin asked for
+  const double* r_max;   // per system: the largest radius
   double4* x0;           // positions at the build
   int2* ent;             // per particle: first entry, entries
   int* pair_first;       // per particle: its first owned pair
