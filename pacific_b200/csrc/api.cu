@@ -195,6 +195,8 @@ struct grains_gpu_ctx {
   double r_min = 0, r_max = 0; // radii of the uploaded particles
   std::vector<double> sys_r_max;  // and the largest of each system
   bool res_ok = false;         // the uploaded scene can run on resident lists
+  bool hooke_memory_only = false;  // every contact law is HookeMemory without a rolling spring
+  bool hooke_memory_pairs = false; // and every pair of materials of the uploaded particles has one
   cudaGraphExec_t res_graph[4] = {nullptr, nullptr, nullptr, nullptr};  // by (cur, hcur)
   double res_graph_dt[4] = {0, 0, 0, 0};
   // reload and RawData files (io.cu): particle names by upload index, sorted
@@ -655,7 +657,7 @@ StepArgs<R> make_args(grains_gpu_ctx* c) {
 // pipeline's.
 constexpr size_t kResAlign = 256;
 constexpr int kResObsHost = 8;  // obstacles per system the state word holds
-size_t res_layout(int64_t cap, int obs_stride, int hist_cap, size_t n_sys, size_t rsize, size_t off[10]) {
+size_t res_layout(int64_t cap, int obs_stride, int hist_cap, size_t n_sys, size_t rsize, size_t off[11]) {
   size_t at = 0;
   auto put = [&](int k, size_t bytes) {
     off[k] = at;
@@ -672,6 +674,7 @@ size_t res_layout(int64_t cap, int obs_stride, int hist_cap, size_t n_sys, size_
   put(7, 2 * m * sizeof(int));
   put(8, n * (size_t)hist_cap);
   put(9, n_sys * sizeof(double));
+  put(10, n * (size_t)hist_cap * sizeof(ResConst));
   return at;
 }
 
@@ -684,7 +687,7 @@ int res_obs_stride(const grains_gpu_ctx* c) {
 template <typename R>
 ResArgs<R> make_res(grains_gpu_ctx* c) {
   ResArgs<R> r{};
-  size_t off[10];
+  size_t off[11];
   const int stride = res_obs_stride(c);
   res_layout(c->cap, stride, c->hist_cap, c->sys.size(), c->rsize, off);
   char* b = c->res_buf;
@@ -711,6 +714,7 @@ ResArgs<R> make_res(grains_gpu_ctx* c) {
   r.pair = c->work;
   r.state = (unsigned char*)(b + off[8]);
   r.mem = (R*)c->hist[1 - c->hcur];
+  r.konst = c->hooke_memory_pairs ? (ResConst*)(b + off[10]) : nullptr;
   // capacities from the buffers' sizes
   const int64_t ent = std::min<int64_t>(c->cap * (int64_t)c->clist_cap, 1ll << 30);
   r.ent_cap = (int)ent;
@@ -886,7 +890,7 @@ bool res_scene(const grains_gpu_ctx* c) {
 int ensure_resident(grains_gpu_ctx* c) {
   c->res_ok = res_scene(c);
   if (!c->res_ok) return 0;
-  size_t off[10];
+  size_t off[11];
   const size_t need = res_layout(c->cap, res_obs_stride(c), c->hist_cap, c->sys.size(), c->rsize, off);
   if (need > c->res_bytes) {
     if (c->res_buf) cudaFree(c->res_buf);
@@ -1443,6 +1447,7 @@ int build_tables(grains_gpu_ctx* c) {
   c->h_sys = hs;
   c->h_obs = ho;
   // laws
+  c->hooke_memory_only = true;
   std::vector<LawParams<double>> ld(c->sys.size() * maxmat * maxmat);
   std::vector<LawParams<float>> lf(ld.size());
   for (auto& x : ld) x.type = -1;
@@ -1453,6 +1458,7 @@ int build_tables(grains_gpu_ctx* c) {
         int a = flip ? kv.first.second : kv.first.first, b = flip ? kv.first.first : kv.first.second;
         size_t k = si * maxmat * maxmat + a * maxmat + b;
         const LawHost& L = kv.second;
+        if (L.type != GRAINS_GPU_HOOKE_MEMORY || L.p[5] != 0.) c->hooke_memory_only = false;
         LawParams<double> P{};
         P.type = L.type;
         P.kn = L.p[0];
@@ -1606,6 +1612,7 @@ int grains_gpu_upload_particles(grains_gpu_ctx* c, const grains_gpu_particles* p
     c->tables_dirty = false;
   }
   const int64_t n_before = c->n;
+  const bool pairs_before = c->hooke_memory_pairs;
   const bool basis_before = c->has_basis, convex_before = c->has_convex;
   c->has_basis = basis_needed;
   c->has_convex = nonsphere;
@@ -1775,6 +1782,17 @@ int grains_gpu_upload_particles(grains_gpu_ctx* c, const grains_gpu_particles* p
   c->sorted = false;
   c->pending_kick2 = false;
   c->uploaded = true;
+  // the resident lists' short form of the law: HookeMemory for every pair of materials that can meet
+  c->hooke_memory_pairs = c->hooke_memory_only;
+  {
+    std::vector<char> has(c->sys.size() * (size_t)maxmat, 0);
+    for (int64_t i = 0; i < n; ++i) has[(size_t)(p->system ? p->system[i] : 0) * maxmat + p->material[i]] = 1;
+    for (size_t k = 0; k < c->sys.size(); ++k)
+      for (int x = 0; x < maxmat; ++x)
+        for (int y = x; y < maxmat; ++y)
+          if (has[k * maxmat + x] && has[k * maxmat + y] && !c->sys[k].laws.count(std::make_pair(x, y)))
+            c->hooke_memory_pairs = false;
+  }
   double r_min = n > 0 ? p->radius[0] : 0., r_max = r_min;
   c->sys_r_max.assign(c->sys.size(), 0.);
   for (int64_t i = 0; i < n; ++i) {
@@ -1784,7 +1802,7 @@ int grains_gpu_upload_particles(grains_gpu_ctx* c, const grains_gpu_particles* p
     b2 = std::max(b2, p->radius[i]);
   }
   // what the step graphs hold of the last upload
-  if (n != n_before || basis_needed != basis_before || c->has_convex != convex_before || r_min != c->r_min ||
+  if (n != n_before || pairs_before != c->hooke_memory_pairs || basis_needed != basis_before || c->has_convex != convex_before || r_min != c->r_min ||
       r_max != c->r_max)
     drop_graphs(c);
   c->r_min = r_min;

@@ -96,11 +96,12 @@ GG_HD V3<R> tangential_vector(R epst, R n_t, V3<R> ut, V3<R> kd, int* branch = n
 // spring is built from (Jiang et al. 2005): constants for Hooke, functions of
 // sqrt(Req deltan) for Hertz.  'existed' tells whether a memory entry was
 // found; 'mem' holds it on entry (when existed) and the updated entry on exit.
+// may_roll = false: the caller knows that no law has a rolling spring.
 template <typename R>
 GG_HD LawResult<R> memory_tangent_rolling(const LawParams<R>& L, R dt, V3<R> normal, V3<R> v_t, V3<R> delFN,
                                           R normFN, R gammat, R kt, R kn, R gamman, const BodyAtContact<R>& b0,
                                           const BodyAtContact<R>& b1, bool existed, PairMemory<R>& mem,
-                                          int* branch) {
+                                          int* branch, bool may_roll = true) {
   V3<R> viscousFT = sc(v_t, -gammat);
   Qt<R> qrot{v3<R>(R(0), R(0), R(0)), R(0)};
   if (existed) {
@@ -127,7 +128,7 @@ GG_HD LawResult<R> memory_tangent_rolling(const LawParams<R>& L, R dt, V3<R> nor
   out.force = delFN + delFT;
   out.tangential = delFT;
   out.torque = v3<R>(R(0), R(0), R(0));
-  if (L.rolling) {
+  if (may_roll && L.rolling) {
     R Req = R(1) / (R(1) / b0.req + R(1) / b1.req);
     R kr = R(3) * kn * L.mur * L.mur * Req * Req;
     R etar = R(3) * gamman * L.mur * L.mur * Req * Req;

@@ -249,6 +249,12 @@ struct StepArgs {
 // reading.
 template <typename R>
 struct ResResult;
+// of a listed pair, when the context's only law is HookeMemory without rolling:
+// the damping coefficients, the crust sum, the law's slot
+struct ResConst {
+  double gamman, gammat, crust;
+  int law, pad;
+};
 template <typename R>
 struct ResArgs {
   int* ctl;              // control words (kResRequest ...)
@@ -263,6 +269,7 @@ struct ResArgs {
   int4* pair;            // pairs: owner's slot, partner's slot, their entries
   unsigned char* state;  // per pair: contact and memory of the last evaluation
   R* mem;                // pair memories, 9 arrays of pair_cap
+  ResConst* konst;       // per pair, or null
   int ent_cap, pair_cap;
   int obs_stride;        // obstacles of the system that has most
   unsigned long long* obs_state;  // per particle: a state byte per obstacle of its system

@@ -190,6 +190,26 @@ __device__ __forceinline__ int res_flush_pairs(const StepArgs<R>& a, const ResAr
   return cnt;
 }
 
+// what the HookeMemory law forms from the two bodies alone, with its own
+// expressions (normal_part_fp64 of the mixed path, hooke_memory of the FP64 one:
+// the same operations)
+template <typename R>
+__device__ __forceinline__ ResConst res_constants(const StepArgs<R>& a, int s, int t) {
+  const int4 mi = a.cur.meta[s], mj = a.cur.meta[t];
+  const double4 mdi = a.cur.md[s], mdj = a.cur.md[t];
+  const SysDev& S = a.sys[mi.w];
+  ResConst k;
+  k.law = S.law_offset + mi.y * S.n_mat + mj.y;
+  const LawParams<R>& L = a.laws[k.law];
+  const double avmass = 1. / (1. / mdi.x + 1. / mdj.x);
+  k.gamman = -2. * L.beta64 * std::sqrt(avmass * L.kn64);
+  const double etat = L.etat64 == -1. ? -L.beta64 * std::sqrt(L.kn64 / avmass) : L.etat64;
+  k.gammat = 2. * etat * avmass;
+  k.crust = xadd(mdi.y, mdj.y);
+  k.pad = 0;
+  return k;
+}
+
 // One cooperative launch: the cell lists, the pair lists, the memory.  Every
 // barrier wait is bounded (grid_barrier); a build that gave up leaves kResValid
 // at -1, on which the other kernels do nothing, and the status bit.
@@ -336,6 +356,7 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
       for (int k = 0; k < te.y; ++k)
         if (r.nb[te.x + k] == s) other = te.x + k;
       r.pair[mine].w = other;
+      if (r.konst) r.konst[mine] = res_constants(a, s, t);
       unsigned char st = 0;
       for (int k = 0; k < hn; ++k)
         if (h[k].other == id && h[k].flags == 0) {
@@ -455,19 +476,37 @@ __global__ void __launch_bounds__(256) res_end_kernel(StepArgs<R> a, ResArgs<R> 
 
 // ---- pairs ----------------------------------------------------------------------
 constexpr int kResPairThreads = 128;
-constexpr int kResPairTile = 256;
 
 template <typename R>
-__device__ __forceinline__ void res_no_contact(const ResArgs<R>& r, int p, int4 pr, unsigned char st) {
-  if (!st) return;
+__device__ __forceinline__ void res_no_contact(const ResArgs<R>& r, int p, int4 pr) {
+  if (!r.state[p]) return;
   r.state[p] = 0;
   r.res[pr.z].f.w = R(0);
   if (pr.w >= 0) r.res[pr.w].f.w = R(0);
 }
 
+// the results, memory and state of listed pair p after its law
+template <typename R>
+__device__ __forceinline__ void res_put_pair(const ResArgs<R>& r, int p, int4 pr, unsigned char st, bool memory,
+                                             const ContactGeom& g, V3<R> f, V3<R> t0, V3<R> t1, ForceStats& fs) {
+  const int now = memory ? kResContact | kResMemory : kResContact;
+  if (st != now) r.state[p] = (unsigned char)now;
+  r.res[pr.z].f = st3<R>(f, R(memory ? 3 : 1));
+  r.res[pr.z].t = st3<R>(t0);
+  if (pr.w >= 0) {
+    r.res[pr.w].f = st3<R>(-f, R(1));
+    r.res[pr.w].t = st3<R>(t1);
+  }
+  ++fs.ncont_own;
+  const double o = fabs(g.overlap);
+  fs.ov_sum += o;
+  fs.ov_max = fmax(fs.ov_max, o);
+}
+
 // the contact law of listed pair p (in contact: the overlap test has passed)
 template <typename R>
-__device__ __forceinline__ void res_pair_one(const StepArgs<R>& a, const ResArgs<R>& r, int p, R dt, ForceStats& fs) {
+__device__ __forceinline__ void res_pair_any_law(const StepArgs<R>& a, const ResArgs<R>& r, int p, R dt,
+                                                 ForceStats& fs) {
   const ParticleArrays<R>& P = a.cur;
   const int4 pr = r.pair[p];
   const int s = pr.x, t = pr.y;
@@ -486,28 +525,88 @@ __device__ __forceinline__ void res_pair_one(const StepArgs<R>& a, const ResArgs
   const D3 Xi = d3(xi.x, xi.y, xi.z), Xj = d3(xj.x, xj.y, xj.z);
   ContactGeom g;
   if (!sphere_pair_geometry(a, Xi, xi.w, mdi.y, Xj, xj.w, mdj.y, g)) {
-    res_no_contact(r, p, pr, st);
+    res_no_contact(r, p, pr);
     return;
   }
   V3<R> t0, t1;
   const LawResult<R> res = particle_pair_law(L, dt, g, Xi, Xj, mdi, mdj, vi, wi, vj, wj, existed, mem, t0, t1);
   if (memory) res_store_memory(r.mem + p, (size_t)r.pair_cap, mem, L.rolling != 0 || !existed);
-  const int now = memory ? kResContact | kResMemory : kResContact;
-  if (st != now) r.state[p] = (unsigned char)now;
   if (law_has_torque(L)) {
     t0 = t0 + res.torque;
     t1 = t1 + (-res.torque);
   }
-  r.res[pr.z].f = st3<R>(res.force, R(memory ? 3 : 1));
-  r.res[pr.z].t = st3<R>(t0);
-  if (pr.w >= 0) {
-    r.res[pr.w].f = st3<R>(-res.force, R(1));
-    r.res[pr.w].t = st3<R>(t1);
+  res_put_pair(r, p, pr, st, memory, g, res.force, t0, t1, fs);
+}
+
+// The same for a context whose only law is HookeMemory without a rolling spring:
+// what depends on the two bodies alone (the damping coefficients, the crust sum,
+// the law's slot) comes from the pair's constants, formed by the build with the
+// law's own expressions.  That leaves out the gathers of both bodies' masses and
+// materials, and four divisions and two square roots of the chain.
+template <typename R>
+__device__ __forceinline__ void res_pair_hooke_memory(const StepArgs<R>& a, const ResArgs<R>& r, int p, R dt,
+                                                      ForceStats& fs) {
+  const ParticleArrays<R>& P = a.cur;
+  const int4 pr = r.pair[p];
+  const ResConst k = r.konst[p];
+  const unsigned char st = r.state[p];
+  const int s = pr.x, t = pr.y;
+  const double4 xi = P.xr[s], xj = P.xr[t];
+  BodyAtContact<R> b0, b1;
+  b0.v = ld3<R>(P.v[s]);
+  b0.w = ld3<R>(P.w[s]);
+  b1.v = ld3<R>(P.v[t]);
+  b1.w = ld3<R>(P.w[t]);
+  const LawParams<R>& L = a.laws[k.law];
+  const bool existed = (st & kResMemory) != 0;
+  PairMemory<R> mem;
+  if (existed) mem = res_load_memory(r.mem + p, (size_t)r.pair_cap, false);
+  const D3 Xi = d3(xi.x, xi.y, xi.z), Xj = d3(xj.x, xj.y, xj.z);
+  D3 ab;
+  double nab;
+  const double dist = sphere_sphere_overlap(Xi, xi.w, Xj, xj.w, &ab, &nab);
+  ContactGeom g = sphere_sphere_features(Xi, xi.w, ab, nab, dist, k.crust);
+  if (g.status && !sphere_pair_geometry(a, Xi, xi.w, P.md[s].y, Xj, xj.w, P.md[t].y, g)) {
+    res_no_contact(r, p, pr);
+    return;
   }
-  ++fs.ncont_own;
-  const double o = fabs(g.overlap);
-  fs.ov_sum += o;
-  fs.ov_max = fmax(fs.ov_max, o);
+  const D3 lev0 = xsub3(g.point, Xi), lev1 = xsub3(g.point, Xj);
+  b0.lever = from_d3<R>(lev0);
+  b1.lever = from_d3<R>(lev1);
+  V3<R> f, t0, t1;
+  if constexpr (sizeof(R) == 4) {
+    // normal_part_fp64 and pair_law, with the constants
+    const V3<double> pen = v3<double>(g.overlap_vector.x, g.overlap_vector.y, g.overlap_vector.z);
+    const V3<double> l0 = dvec(lev0), l1 = dvec(lev1);
+    const V3<double> normal = round3(dv(pen, norm(pen)));
+    const V3<double> rel = (widen(b0.v) + cross(widen(b0.w), l0)) - (widen(b1.v) + cross(widen(b1.w), l1));
+    const V3<double> v_n = sc(normal, dot(rel, normal));
+    const V3<double> v_t = rel - v_n;
+    const V3<double> fn = sc(pen, L.kn64) - sc(v_n, k.gamman);
+    const LawResult<R> res = memory_tangent_rolling(
+        L, dt, v3<R>(R(normal.x), R(normal.y), R(normal.z)), v3<R>(R(v_t.x), R(v_t.y), R(v_t.z)),
+        v3<R>(R(fn.x), R(fn.y), R(fn.z)), R(norm(fn)), R(k.gammat), L.kt, R(L.kn64), R(k.gamman), b0, b1, existed, mem,
+        (int*)nullptr, false);
+    const V3<double> tn0 = cross(l0, fn), tn1 = cross(l1, -fn);
+    f = res.force;
+    t0 = v3<R>(R(tn0.x), R(tn0.y), R(tn0.z)) + cross(b0.lever, res.tangential);
+    t1 = v3<R>(R(tn1.x), R(tn1.y), R(tn1.z)) + cross(b1.lever, -res.tangential);
+  } else {
+    // hooke_memory, with the constants
+    const V3<R> pen = from_d3<R>(g.overlap_vector);
+    const V3<R> normal = round3(dv(pen, norm(pen)));
+    const V3<R> rel = velocity_at(b0) - velocity_at(b1);
+    const V3<R> v_n = sc(normal, dot(rel, normal));
+    const V3<R> v_t = rel - v_n;
+    const V3<R> fn = sc(pen, L.kn) - sc(v_n, R(k.gamman));
+    const LawResult<R> res = memory_tangent_rolling(L, dt, normal, v_t, fn, norm(fn), R(k.gammat), L.kt, L.kn,
+                                                    R(k.gamman), b0, b1, existed, mem, (int*)nullptr, false);
+    f = res.force;
+    t0 = cross(b0.lever, res.force);
+    t1 = cross(b1.lever, -res.force);
+  }
+  res_store_memory(r.mem + p, (size_t)r.pair_cap, mem, !existed);
+  res_put_pair(r, p, pr, st, true, g, f, t0, t1, fs);
 }
 
 // one obstacle candidate (pair_one's obstacle part on resident memory)
@@ -558,62 +657,87 @@ __device__ __forceinline__ void res_obstacle_one(const StepArgs<R>& a, const Res
   fs.ov_max = fmax(fs.ov_max, ov);
 }
 
-// Blocks [0, pair_blocks): the listed pairs, a tile at a time: the exact overlap
-// test of every pair (two per thread, their loads in flight together), those in
-// contact packed in shared memory, then the law on the packed ones, so that the
-// law runs on full warps whatever share of the list is in contact.  Then
-// obs_blocks: the obstacle candidates; the other blocks: the number of candidate
-// pairs of the step (the 27 cells around every particle, as the launched
-// broadphase counts them), and the cell counts of the next step cleared.
-template <typename R>
-__global__ void __launch_bounds__(kResPairThreads, GG_PAIRS_MIN_BLOCKS)
+// Blocks [0, pair_blocks): the listed pairs.  Each warp tests 32 or 64 pairs at a
+// time (the exact overlap test of every listed pair) and queues those in contact
+// in shared memory; whenever 32 are queued it runs the law on them, so that the
+// law runs on full warps whatever share of the list is in contact, without a
+// barrier.  64 at a time keeps twice the loads in flight; 32 spreads a short list
+// over more warps.  Then obs_blocks: the obstacle candidates; the other blocks:
+// the number of candidate pairs of the step (the 27 cells around every particle,
+// as the launched broadphase counts them), and the cell counts of the next step
+// cleared.
+// Bound by the latency of the gathers and by L2 (about 450 B a contact); four
+// blocks a SM at 128 registers (five at 96 spill: 67.2 against 66.5 us).  200,000
+// spheres, 460,000 contacts: 82 -> 66 us mixed, 103 -> 82 us FP64 with the pair
+// constants and without the block-wide barriers of the first form.
+constexpr int kResPairBlocks = 4;
+template <typename R, bool HOOKE_MEMORY>
+__global__ void __launch_bounds__(kResPairThreads, kResPairBlocks)
     res_pairs_kernel(StepArgs<R> a, ResArgs<R> r, R dt, int parity, int pair_blocks, int obs_blocks) {
-  __shared__ int list[kResPairTile];
-  __shared__ int n_list;
+  constexpr int kQueue = 96;
+  __shared__ int queue_s[kResPairThreads / 32][kQueue];
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   ForceStats fs{0, 0, 0, 0, 0., 0.};
   if ((int)blockIdx.x < pair_blocks) {
     const int n_pairs = *(volatile int*)(r.ctl + kResValid);
-    for (int base = blockIdx.x * kResPairTile; base < n_pairs; base += pair_blocks * kResPairTile) {
-      if (threadIdx.x == 0) n_list = 0;
-      __syncthreads();
-      int4 pr[2];
-      double4 xi[2], xj[2];
+    int* queue = queue_s[threadIdx.x / 32];
+    const int warps = pair_blocks * (kResPairThreads / 32);
+    const int warp = blockIdx.x * (kResPairThreads / 32) + threadIdx.x / 32;
+    const int per = n_pairs > 32 * warps ? 2 : 1;
+    int queued = 0;
+    auto law = [&](int p) {
+      if constexpr (HOOKE_MEMORY)
+        res_pair_hooke_memory(a, r, p, dt, fs);
+      else
+        res_pair_any_law(a, r, p, dt, fs);
+    };
+    bool more = true;
+    for (int base = warp * 32 * per; more; base += warps * 32 * per) {
+      more = base < n_pairs;
+      if (more) {
+        int4 pr[2];
+        double4 xi[2], xj[2];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int p = base + u * kResPairThreads + threadIdx.x;
-        pr[u] = p < n_pairs ? r.pair[p] : make_int4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        xi[u] = a.cur.xr[pr[u].x];
-        xj[u] = a.cur.xr[pr[u].y];
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int p = base + u * kResPairThreads + threadIdx.x;
-        bool contact = false;
-        if (p < n_pairs) {
-          const double dx = xj[u].x - xi[u].x, dy = xj[u].y - xi[u].y, dz = xj[u].z - xi[u].z;
-          const double rs = xi[u].w + xj[u].w;
-          if (!(dx * dx + dy * dy + dz * dz > rs * rs * (1. + 1.e-12))) {  // as in contacts_one
-            D3 ab;
-            double nab;
-            contact = sphere_sphere_overlap(d3(xi[u].x, xi[u].y, xi[u].z), xi[u].w, d3(xj[u].x, xj[u].y, xj[u].z),
-                                            xj[u].w, &ab, &nab) < 0.;
-          }
-          if (!contact) res_no_contact(r, p, pr[u], r.state[p]);
+        for (int u = 0; u < 2; ++u) {
+          const int p = base + 32 * u + lane;
+          pr[u] = u < per && p < n_pairs ? r.pair[p] : make_int4(0, 0, 0, 0);
         }
-        const unsigned hit = __ballot_sync(full, contact);
-        int at = 0;
-        if (lane == 0 && hit) at = atomicAdd(&n_list, __popc(hit));
-        at = __shfl_sync(full, at, 0);
-        if (contact) list[at + __popc(hit & ((1u << lane) - 1u))] = p;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          xi[u] = a.cur.xr[pr[u].x];
+          xj[u] = a.cur.xr[pr[u].y];
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int p = base + 32 * u + lane;
+          bool contact = false;
+          if (u < per && p < n_pairs) {
+            const double dx = xj[u].x - xi[u].x, dy = xj[u].y - xi[u].y, dz = xj[u].z - xi[u].z;
+            const double rs = xi[u].w + xj[u].w;
+            if (!(dx * dx + dy * dy + dz * dz > rs * rs * (1. + 1.e-12))) {  // as the broadphase tests
+              D3 ab;
+              double nab;
+              contact = sphere_sphere_overlap(d3(xi[u].x, xi[u].y, xi[u].z), xi[u].w,
+                                              d3(xj[u].x, xj[u].y, xj[u].z), xj[u].w, &ab, &nab) < 0.;
+            }
+            if (!contact) res_no_contact(r, p, pr[u]);
+          }
+          const unsigned hit = __ballot_sync(full, contact);
+          if (contact) queue[queued + __popc(hit & ((1u << lane) - 1u))] = p;
+          queued += __popc(hit);
+        }
+        __syncwarp();
       }
-      __syncthreads();
-      for (int k = threadIdx.x; k < n_list; k += kResPairThreads) res_pair_one(a, r, list[k], dt, fs);
-      __syncthreads();
+      // full warps as they come, the rest in the end
+      while (queued >= 32 || (!more && queued > 0)) {
+        const int take = min(queued, 32);
+        const int p = lane < take ? queue[queued - take + lane] : -1;
+        queued -= take;
+        __syncwarp();
+        if (p >= 0) law(p);
+        __syncwarp();
+      }
     }
     flush_force_stats(a.stats, fs);
   } else if ((int)blockIdx.x < pair_blocks + obs_blocks) {
@@ -822,12 +946,15 @@ int launch_res_step(const StepArgs<R>& args, const ResArgs<R>& r, cudaStream_t s
       return GRAINS_GPU_CUDA_ERROR;
   }
   if (phases & 2) {
-    // every SM filled once by the pair blocks (four per SM), fewer when the lists (about 5 pairs a particle) are
-    // short; the obstacle and count blocks follow them
-    const int pb = std::min(4 * 148, grid_for(5ll * a.n, kResPairTile));
+    // every SM filled once by the pair blocks, fewer when the lists (about 5 pairs a particle) are short; the
+    // obstacle and count blocks follow them
+    const int pb = std::min(kResPairBlocks * 148, grid_for(5ll * a.n, kResPairThreads));
     const int ob = std::min(148, grid_for(a.n, 4 * kResPairThreads));
     const int cb = std::min(2 * 148, grid_for(a.n_cells, kResPairThreads));
-    res_pairs_kernel<R><<<pb + ob + cb, kResPairThreads, 0, s>>>(a, r, R(dt), parity, pb, ob);
+    if (r.konst)
+      res_pairs_kernel<R, true><<<pb + ob + cb, kResPairThreads, 0, s>>>(a, r, R(dt), parity, pb, ob);
+    else
+      res_pairs_kernel<R, false><<<pb + ob + cb, kResPairThreads, 0, s>>>(a, r, R(dt), parity, pb, ob);
   }
   if (phases & 4) {
     StepArgs<R> an = a;
