@@ -657,7 +657,7 @@ StepArgs<R> make_args(grains_gpu_ctx* c) {
 // pipeline's.
 constexpr size_t kResAlign = 256;
 constexpr int kResObsHost = 8;  // obstacles per system the state word holds
-size_t res_layout(int64_t cap, int obs_stride, int hist_cap, size_t n_sys, size_t rsize, size_t off[11]) {
+size_t res_layout(int64_t cap, int obs_stride, int hist_cap, int list_cap, size_t n_sys, size_t rsize, size_t off[12]) {
   size_t at = 0;
   auto put = [&](int k, size_t bytes) {
     off[k] = at;
@@ -667,7 +667,7 @@ size_t res_layout(int64_t cap, int obs_stride, int hist_cap, size_t n_sys, size_
   put(0, 16 * sizeof(int) + 2 * sizeof(unsigned) + sizeof(double) + 4096 * sizeof(int));  // control, barrier, skin, sums
   put(1, n * sizeof(double4));
   put(2, n * sizeof(int2));
-  put(3, n * sizeof(int));
+  put(3, n * (size_t)list_cap * sizeof(int));
   put(4, n * sizeof(unsigned long long));
   put(5, m * 8 * rsize);
   put(6, m * 9 * rsize);
@@ -675,6 +675,7 @@ size_t res_layout(int64_t cap, int obs_stride, int hist_cap, size_t n_sys, size_
   put(8, n * (size_t)hist_cap);
   put(9, n_sys * sizeof(double));
   put(10, n * (size_t)hist_cap * sizeof(ResConst));
+  put(11, 2 * n);
   return at;
 }
 
@@ -687,9 +688,9 @@ int res_obs_stride(const grains_gpu_ctx* c) {
 template <typename R>
 ResArgs<R> make_res(grains_gpu_ctx* c) {
   ResArgs<R> r{};
-  size_t off[11];
+  size_t off[12];
   const int stride = res_obs_stride(c);
-  res_layout(c->cap, stride, c->hist_cap, c->sys.size(), c->rsize, off);
+  res_layout(c->cap, stride, c->hist_cap, c->clist_cap, c->sys.size(), c->rsize, off);
   char* b = c->res_buf;
   r.ctl = (int*)(b + off[0]);
   r.bar = (unsigned*)(r.ctl + 16);
@@ -701,7 +702,9 @@ ResArgs<R> make_res(grains_gpu_ctx* c) {
   r.r_max = (const double*)(b + off[9]);
   r.x0 = (double4*)(b + off[1]);
   r.ent = (int2*)(b + off[2]);
-  r.pair_first = (int*)(b + off[3]);
+  r.ent_pair = (int*)(b + off[3]);
+  r.dirty[0] = (unsigned char*)(b + off[11]);
+  r.dirty[1] = r.dirty[0] + c->cap;
   r.obs_state = (unsigned long long*)(b + off[4]);
   r.obs_res = (ResResult<R>*)(b + off[5]);
   r.obs_mem = (R*)(b + off[6]);
@@ -890,8 +893,8 @@ bool res_scene(const grains_gpu_ctx* c) {
 int ensure_resident(grains_gpu_ctx* c) {
   c->res_ok = res_scene(c);
   if (!c->res_ok) return 0;
-  size_t off[11];
-  const size_t need = res_layout(c->cap, res_obs_stride(c), c->hist_cap, c->sys.size(), c->rsize, off);
+  size_t off[12];
+  const size_t need = res_layout(c->cap, res_obs_stride(c), c->hist_cap, c->clist_cap, c->sys.size(), c->rsize, off);
   if (need > c->res_bytes) {
     if (c->res_buf) cudaFree(c->res_buf);
     c->res_buf = nullptr;

@@ -263,8 +263,9 @@ struct ResArgs {
   const double* r_max;   // per system: the largest radius
   double4* x0;           // positions at the build
   int2* ent;             // per particle: first entry, entries
-  int* pair_first;       // per particle: its first owned pair
   int* nb;               // entries: partner's slot, kOwnBit when this particle owns the pair
+  int* ent_pair;         // entries: their pair
+  unsigned char* dirty[2];  // per particle, by parity: a partner has crossed into another cell
   ResResult<R>* res;     // per entry: force and torque on this particle
   int4* pair;            // pairs: owner's slot, partner's slot, their entries
   unsigned char* state;  // per pair: contact and memory of the last evaluation

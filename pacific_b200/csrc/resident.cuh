@@ -40,7 +40,7 @@ enum { kResContact = 1, kResMemory = 2, kResCandidate = 4 };
 // force and torque of one side of a listed pair: one 32-byte sector in mixed precision
 template <typename R>
 struct ResResult {
-  typename Vec4<R>::type f;  // w: 0 no contact, 1 contact, 3 contact whose owner stored a memory
+  typename Vec4<R>::type f;  // w: 0 no contact; a contact: 1 the partner owns it, else 2, with a memory 3
   typename Vec4<R>::type t;
 };
 
@@ -155,19 +155,16 @@ __device__ __forceinline__ int res_flush_pairs(const StepArgs<R>& a, const ResAr
   const int lane = res_lane();
   const unsigned lower = (1u << lane) - 1u;
   int2 en = make_int2(0, 0);
-  int row = 0, p = 0, cnt = 0;
+  int row = 0, cnt = 0;
   if (active) {
     en = r.ent[s];
     row = a.cur.orig[s];
-    p = r.pair_first[s];
   }
   HistEntry<R>* h = a.hist_prev + (size_t)row * a.hist_cap;
   for (int q0 = 0; __any_sync(full, q0 < en.y); q0 += kResLanes) {
     const int e = q0 + lane < en.y ? r.nb[en.x + q0 + lane] : 0;
-    const bool own = (e & kOwnBit) != 0;
-    const unsigned owners = res_ballot(own);
-    const int mine = p + __popc(owners & lower);
-    const bool keep = own && (r.state[mine] & kResMemory);
+    const int mine = e & kOwnBit ? r.ent_pair[en.x + q0 + lane] : 0;
+    const bool keep = (e & kOwnBit) && (r.state[mine] & kResMemory);
     const unsigned keepers = res_ballot(keep);
     const int at = cnt + __popc(keepers & lower);
     if (keep && at < a.hist_cap) {
@@ -182,7 +179,6 @@ __device__ __forceinline__ int res_flush_pairs(const StepArgs<R>& a, const ResAr
     } else if (keep) {
       set_status(a.stats, GRAINS_GPU_HISTORY_FULL);
     }
-    p += __popc(owners);
     cnt += __popc(keepers);
   }
   cnt = min(cnt, a.hist_cap);
@@ -290,8 +286,8 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
       const bool fits = (long long)e0 + cnt <= r.ent_cap && (long long)p0 + own <= r.pair_cap;
       if (s < n && leader) {
         r.ent[s] = make_int2(fits ? e0 : 0, fits ? cnt : 0);
-        r.pair_first[s] = p0;
         r.x0[s] = a.cur.xr[s];
+        r.dirty[0][s] = r.dirty[1][s] = 0;
       }
       // entry q of the list; the pair of an owned one
       int q0 = 0, rank = 0;
@@ -302,7 +298,11 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
           const int q = e0 + q0 + __popc(ins & lower);
           r.nb[q] = e;
           r.res[q].f.w = R(0);
-          if (o) r.pair[p0 + rank + __popc(owners & lower)] = make_int4(s, entry_slot(e), q, -1);
+          if (o) {
+            const int p = p0 + rank + __popc(owners & lower);
+            r.pair[p] = make_int4(s, entry_slot(e), q, -1);
+            r.ent_pair[q] = p;
+          }
         }
         q0 += __popc(ins);
         rank += __popc(owners);
@@ -334,21 +334,17 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
   // each pair's entry in the partner's list, and its memory from the owner's row
   for (int s = group; s < padded; s += groups) {
     int2 en = make_int2(0, 0);
-    int row = 0, p = 0, hn = 0;
+    int row = 0, hn = 0;
     if (s < n) {
       en = r.ent[s];
       row = a.cur.orig[s];
-      p = r.pair_first[s];
       hn = a.hist_n_prev[row];
     }
     const HistEntry<R>* h = a.hist_prev + (size_t)row * a.hist_cap;
-    for (int q = 0; __any_sync(0xffffffffu, q < en.y); q += kResLanes) {
-      const int e = q + lane < en.y ? r.nb[en.x + q + lane] : 0;
-      const bool own = (e & kOwnBit) != 0;
-      const unsigned owners = res_ballot(own);
-      const int mine = p + __popc(owners & lower);
-      p += __popc(owners);
-      if (!own) continue;
+    for (int q = lane; q < en.y; q += kResLanes) {
+      const int e = r.nb[en.x + q];
+      if (!(e & kOwnBit)) continue;
+      const int mine = r.ent_pair[en.x + q];
       const int t = entry_slot(e);
       const int2 te = r.ent[t];
       const int id = a.cur.meta[t].x;
@@ -356,6 +352,7 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
       for (int k = 0; k < te.y; ++k)
         if (r.nb[te.x + k] == s) other = te.x + k;
       r.pair[mine].w = other;
+      if (other >= 0) r.ent_pair[other] = mine;
       if (r.konst) r.konst[mine] = res_constants(a, s, t);
       unsigned char st = 0;
       for (int k = 0; k < hn; ++k)
@@ -491,7 +488,7 @@ __device__ __forceinline__ void res_put_pair(const ResArgs<R>& r, int p, int4 pr
                                              const ContactGeom& g, V3<R> f, V3<R> t0, V3<R> t1, ForceStats& fs) {
   const int now = memory ? kResContact | kResMemory : kResContact;
   if (st != now) r.state[p] = (unsigned char)now;
-  r.res[pr.z].f = st3<R>(f, R(memory ? 3 : 1));
+  r.res[pr.z].f = st3<R>(f, R(memory ? 3 : 2));
   r.res[pr.z].t = st3<R>(t0);
   if (pr.w >= 0) {
     r.res[pr.w].f = st3<R>(-f, R(1));
@@ -783,9 +780,51 @@ __global__ void __launch_bounds__(kResPairThreads, kResPairBlocks)
 }
 
 // ---- sums -----------------------------------------------------------------------
+
+// The list of particle s back into the order of (cell, id) after partners have
+// crossed into other cells: an insertion sort of the nearly ordered entries with
+// their results; each moved entry's pair learns the new place.
+template <typename R>
+__device__ __forceinline__ void res_reorder(const StepArgs<R>& a, const ResArgs<R>& r, int2 en) {
+  auto rank = [&](int e) {
+    const int t = entry_slot(e);
+    return ((unsigned long long)a.cur.key[t] << 32) | ((unsigned)a.cur.meta[t].x ^ 0x80000000u);
+  };
+  auto place = [&](int q, int e, int p, const ResResult<R>& x) {
+    r.nb[q] = e;
+    r.ent_pair[q] = p;
+    r.res[q] = x;
+    if (e & kOwnBit)
+      r.pair[p].z = q;
+    else
+      r.pair[p].w = q;
+  };
+  unsigned long long last = 0;
+  for (int q = en.x; q < en.x + en.y; ++q) {
+    const int e = r.nb[q];
+    const unsigned long long k = rank(e);
+    if (q == en.x || k > last) {
+      last = k;
+      continue;
+    }
+    const int p = r.ent_pair[q];
+    const ResResult<R> x = r.res[q];
+    int to = q;
+    for (; to > en.x; --to) {
+      const int f = r.nb[to - 1];
+      if (rank(f) < k) break;
+      place(to, f, r.ent_pair[to - 1], r.res[to - 1]);
+    }
+    place(to, e, p, x);
+  }
+}
+
 // The torsor of particle s from the results of its list entries in the order of
 // (cell of the partner, id), as the launched pipeline lists them; then its
 // obstacles, the fluid, the kicks, the drift and the next step's candidates.
+// Lists keep that order from their build; a particle that crosses into another
+// cell marks its partners' lists for res_reorder in the next step (about one
+// list in a hundred a step), so that no step looks up the partners' cells.
 template <typename R>
 __global__ void __launch_bounds__(256) res_sums_kernel(StepArgs<R> a, ResArgs<R> r, R dt_half, double dt, int parity) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -794,76 +833,35 @@ __global__ void __launch_bounds__(256) res_sums_kernel(StepArgs<R> a, ResArgs<R>
   unsigned mask = 0;
   unsigned long long state = 0;
   if (active) {
+    const int2 en = r.ent[s];
+    const unsigned char dirty = r.dirty[parity][s];
     const int4 meta = P.meta[s];
     const double4 md = P.md[s];
+    const unsigned old_key = P.key[s];
+    state = r.obs_state[s];
     const double mass = md.x * (1. - md.w);  // Particle::computeWeight, as in sum_one
     const SysDev& S = a.sys[meta.w];
     V3<R> F = v3<R>(R(S.gx * mass), R(S.gy * mass), R(S.gz * mass));
     V3<R> T = v3<R>(R(0), R(0), R(0));
-    const int2 en = r.ent[s];
-    state = r.obs_state[s];
+    if (dirty) {
+      res_reorder(a, r, en);
+      r.dirty[parity][s] = 0;
+    }
     int listed = 0, owned = 0;
     bool full = false;  // a memory beyond the row
-    auto add = [&](const ResResult<R>& x, bool own) {
-      F = F + ld3<R>(x.f);
-      T = T + ld3<R>(x.t);
-      ++listed;
-      if (own) full = full || (x.f.w == R(3) && owned >= a.hist_cap);
-      owned += own ? 1 : 0;
-    };
-    // entries keep the order of their build; a partner that has crossed into
-    // another cell since may have changed it
-    const V3<R> F0 = F;
-    unsigned last_key = 0;
-    int last_entry = 0;
-    bool ordered = true;
     for (int q0 = 0; q0 < en.y; q0 += 4) {
       ResResult<R> x[4];
-      int e[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (q0 + u < en.y) {
-          x[u] = r.res[en.x + q0 + u];
-          e[u] = r.nb[en.x + q0 + u];
-        }
-      unsigned key[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (q0 + u < en.y && x[u].f.w != R(0)) key[u] = P.key[entry_slot(e[u])];
+        if (q0 + u < en.y) x[u] = r.res[en.x + q0 + u];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         if (q0 + u >= en.y || x[u].f.w == R(0)) continue;
-        if (listed > 0 && key[u] <= last_key &&
-            (key[u] < last_key || P.meta[entry_slot(e[u])].x < P.meta[entry_slot(last_entry)].x))
-          ordered = false;
-        last_entry = e[u];
-        last_key = key[u];
-        add(x[u], (e[u] & kOwnBit) != 0);
-      }
-    }
-    if (!ordered) {
-      F = F0;
-      T = v3<R>(R(0), R(0), R(0));
-      listed = owned = 0;
-      full = false;
-      bool any = false;
-      unsigned long long done = 0;  // (cell, id) of the last one added
-      for (;;) {
-        unsigned long long least = ~0ull;
-        int at = -1;
-        for (int q = 0; q < en.y; ++q) {
-          if (r.res[en.x + q].f.w == R(0)) continue;
-          const int t = entry_slot(r.nb[en.x + q]);
-          const unsigned long long k = ((unsigned long long)P.key[t] << 32) | ((unsigned)P.meta[t].x ^ 0x80000000u);
-          if ((!any || k > done) && k < least) {
-            least = k;
-            at = q;
-          }
-        }
-        if (at < 0) break;
-        add(r.res[en.x + at], (r.nb[en.x + at] & kOwnBit) != 0);
-        done = least;
-        any = true;
+        F = F + ld3<R>(x[u].f);
+        T = T + ld3<R>(x[u].t);
+        ++listed;
+        full = full || (x[u].f.w == R(3) && owned >= a.hist_cap);
+        owned += x[u].f.w >= R(2) ? 1 : 0;
       }
     }
     int n_cand = 0;
@@ -895,6 +893,8 @@ __global__ void __launch_bounds__(256) res_sums_kernel(StepArgs<R> a, ResArgs<R>
     const double dx = X.x - x0.x, dy = X.y - x0.y, dz = X.z - x0.z;
     const double half = *r.skin * (0.5 * (1. - 1.e-9));
     if (!(dx * dx + dy * dy + dz * dz < half * half)) r.ctl[kResRequest] = 1;
+    if (key != old_key)
+      for (int q = 0; q < en.y; ++q) r.dirty[1 - parity][entry_slot(r.nb[en.x + q])] = 1;
     mask = res_obstacle_candidates(a, S, key, X, x0.w);
   }
   const unsigned long long next = res_emit_obstacles(r, s, mask, state, 1 - parity);
