@@ -190,7 +190,7 @@ struct grains_gpu_ctx {
   // resident pair lists of the middle steps (resident.cuh)
   char* res_buf = nullptr;   // per-particle and per-obstacle arrays
   size_t res_bytes = 0;
-  int* cell_count2 = nullptr;  // cell counts of the steps of odd parity
+  int* cell_count2[2] = {nullptr, nullptr};  // cell counts of the steps 1 and 2 modulo 3 (step 0: cell_count)
   int res_blocks = 0;          // blocks of the build's cooperative launch
   double r_min = 0, r_max = 0; // radii of the uploaded particles
   std::vector<double> sys_r_max;  // and the largest of each system
@@ -664,7 +664,7 @@ size_t res_layout(int64_t cap, int obs_stride, int hist_cap, int list_cap, size_
     at += (bytes + kResAlign - 1) / kResAlign * kResAlign;
   };
   const size_t n = (size_t)cap, m = n * (size_t)std::max(1, obs_stride);
-  put(0, 16 * sizeof(int) + 2 * sizeof(unsigned) + sizeof(double) + 4096 * sizeof(int));  // control, barrier, skin, sums
+  put(0, 16 * sizeof(int) + 2 * sizeof(unsigned) + 2 * sizeof(double) + 4096 * sizeof(int));  // control, barrier, skin, candidates, sums
   put(1, n * sizeof(double4));
   put(2, n * sizeof(int2));
   put(3, n * (size_t)list_cap * sizeof(int));
@@ -695,7 +695,8 @@ ResArgs<R> make_res(grains_gpu_ctx* c) {
   r.ctl = (int*)(b + off[0]);
   r.bar = (unsigned*)(r.ctl + 16);
   r.skin = (double*)(r.bar + 2);
-  r.block_sums = (int*)(r.skin + 1);
+  r.n_cand = (unsigned long long*)(r.skin + 1);
+  r.block_sums = (int*)(r.n_cand + 1);
   // a wide skin lasts longer but lists more pairs: 0.2 r_min (a tenth of a
   // diameter) lists 8 to 9 partners a particle in a dense bed, of which 5 touch
   r.skin0 = 0.2 * c->r_min;
@@ -723,7 +724,8 @@ ResArgs<R> make_res(grains_gpu_ctx* c) {
   r.ent_cap = (int)ent;
   r.pair_cap = (int)std::min<int64_t>(ent / 2, c->cap * (int64_t)c->hist_cap);
   r.count[0] = c->cell_count;
-  r.count[1] = c->cell_count2;
+  r.count[1] = c->cell_count2[0];
+  r.count[2] = c->cell_count2[1];
   r.rebuild_blocks = c->res_blocks;
   return r;
 }
@@ -922,22 +924,22 @@ int resident_begin(grains_gpu_ctx* c) {
   return rc ? fail(c, rc, "resident lists: start failed") : 0;
 }
 
-int resident_step(grains_gpu_ctx* c, double dt, int parity, int phases = 7) {
-  const int rc = with_res(c, [&](auto a, auto r) { return launch_res_step(a, r, c->stream, dt, parity, phases); });
+int resident_step(grains_gpu_ctx* c, double dt, int step, int phases = 7) {
+  const int rc = with_res(c, [&](auto a, auto r) { return launch_res_step(a, r, c->stream, dt, step % 6, phases); });
   return rc ? fail(c, rc, "resident step launch failed") : 0;
 }
 
 // the memories back into the rows, the counts and keys of the new positions
 // where the launched pipeline expects them
-int resident_end(grains_gpu_ctx* c, int parity) {
+int resident_end(grains_gpu_ctx* c, int steps) {
   const int rc = with_res(c, [&](auto a, auto r) { return launch_res_end(a, r, c->stream); });
   if (rc) return fail(c, rc, "resident lists: end failed");
-  if (parity) {
-    CK(cudaMemcpyAsync(c->cell_count, c->cell_count2, (size_t)c->n_cells * sizeof(int), cudaMemcpyDeviceToDevice,
-                       c->stream));
+  if (steps % 3)
+    CK(cudaMemcpyAsync(c->cell_count, c->cell_count2[steps % 3 - 1], (size_t)c->n_cells * sizeof(int),
+                       cudaMemcpyDeviceToDevice, c->stream));
+  if (steps % 2)
     CK(cudaMemcpyAsync(c->buf[c->cur].key, c->buf[1 - c->cur].key, (size_t)c->n * sizeof(unsigned),
                        cudaMemcpyDeviceToDevice, c->stream));
-  }
   c->keys_valid = true;
   c->sorted = false;
   return 0;
@@ -945,8 +947,8 @@ int resident_end(grains_gpu_ctx* c, int parity) {
 
 // Steps between two gathers of the particle arrays into cell order within a
 // resident run (a gather moves the slots, so the lists are built anew)
-constexpr int kResGather = 512;
-constexpr int kResGraph = 16;  // steps of a graph (even: the parity comes back)
+constexpr int kResGather = 504;
+constexpr int kResGraph = 12;  // steps of a graph: a multiple of 6, the period of the alternating buffers
 // A resident run costs the build of its lists and the memories' way back, about
 // as much as two launched steps: shorter runs take those
 constexpr int kResMinSteps = 6;
@@ -958,7 +960,8 @@ bool use_resident(const grains_gpu_ctx* c, int middle) {
 // n middle steps on resident lists
 int resident_steps(grains_gpu_ctx* c, int n, double dt) {
   while (n > 0) {
-    int k = std::min(n, kResGather), parity = 0;
+    int k = std::min(n, kResGather), step = 0;
+    const int run = k;
     n -= k;
     if (int rc = resident_begin(c)) return rc;
     for (; k >= kResGraph; k -= kResGraph) {
@@ -971,7 +974,7 @@ int resident_steps(grains_gpu_ctx* c, int n, double dt) {
         cudaGraph_t g;
         CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
         int rc = 0;
-        for (int q = 0; q < kResGraph && !rc; ++q) rc = resident_step(c, dt, q & 1);
+        for (int q = 0; q < kResGraph && !rc; ++q) rc = resident_step(c, dt, q);
         cudaError_t e = cudaStreamEndCapture(c->stream, &g);
         if (rc) return rc;
         if (e != cudaSuccess) return cuda_fail(c, e, "cudaStreamEndCapture");
@@ -982,9 +985,9 @@ int resident_steps(grains_gpu_ctx* c, int n, double dt) {
       }
       CK(cudaGraphLaunch(c->res_graph[slot], c->stream));
     }
-    for (; k > 0; --k, parity ^= 1)
-      if (int rc = resident_step(c, dt, parity)) return rc;
-    if (int rc = resident_end(c, parity)) return rc;
+    for (; k > 0; --k, ++step)
+      if (int rc = resident_step(c, dt, step)) return rc;
+    if (int rc = resident_end(c, run)) return rc;
     if (n > 0) {  // into cell order, and the counts the next lists start from
       if (int rc = sort_now(c, 0)) return rc;
       CK(cudaMemsetAsync(c->cell_count, 0, (size_t)c->n_cells * sizeof(int), c->stream));
@@ -1559,9 +1562,11 @@ int build_tables(grains_gpu_ctx* c) {
   CK(cudaMalloc(&p, (size_t)cells * sizeof(int)));
   c->table_pool.push_back(p);
   c->cell_count = (int*)p;
-  CK(cudaMalloc(&p, (size_t)cells * sizeof(int)));
-  c->table_pool.push_back(p);
-  c->cell_count2 = (int*)p;
+  for (int k = 0; k < 2; ++k) {
+    CK(cudaMalloc(&p, (size_t)cells * sizeof(int)));
+    c->table_pool.push_back(p);
+    c->cell_count2[k] = (int*)p;
+  }
   CK(cudaMalloc(&p, ((size_t)cells + 1) * sizeof(int)));
   c->table_pool.push_back(p);
   c->cell_start = (int*)p;
@@ -2733,7 +2738,7 @@ int grains_gpu_profile_kernels(grains_gpu_ctx* c, int32_t n_steps, double* time,
       // the overlap tests and the law as the pairs
       for (int q = 0; q < 3; ++q) {
         CK(cudaEventRecord(ev[1 + q], c->stream));
-        if (int rc = resident_step(c, dt, k & 1, 1 << q)) return rc;
+        if (int rc = resident_step(c, dt, k, 1 << q)) return rc;
       }
       CK(cudaEventRecord(ev[4], c->stream));
       CK(cudaEventSynchronize(ev[4]));
@@ -2745,7 +2750,7 @@ int grains_gpu_profile_kernels(grains_gpu_ctx* c, int32_t n_steps, double* time,
         cnt[phase[q]] += 1;
       }
       if (k == n_steps - 2)
-        if (int rc = resident_end(c, (n_steps - 1) & 1)) return rc;
+        if (int rc = resident_end(c, n_steps - 1)) return rc;
       continue;
     }
     CK(cudaEventRecord(ev[1], c->stream));

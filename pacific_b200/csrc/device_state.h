@@ -277,7 +277,8 @@ struct ResArgs {
   ResResult<R>* obs_res; // per particle and obstacle
   R* obs_mem;            // per particle and obstacle: 9 numbers
   int* obs_item[2];      // obstacle candidates (particle * kResObsMax + obstacle) by the step's parity
-  int* count[2];         // cell counts of the step's positions, by parity
+  int* count[3];         // cell counts of the positions of step % 3
+  unsigned long long* n_cand;  // candidate pairs of the present positions, the particles themselves included
   int* block_sums;       // scan scratch of the build, one per block
   unsigned* bar;         // its grid barrier
   int rebuild_blocks;
@@ -347,13 +348,13 @@ int persistent_blocks(const StepArgs<R>& a);
 template <typename R>
 int launch_persistent_steps(const StepArgs<R>& a, cudaStream_t s, int n_steps, double dt, int gather_every,
                             int since_gather, int n_moving, double* clock, unsigned* bar, int* sums, int blocks);
-// steps on resident pair lists; parity: of the step within the run
+// steps on resident pair lists; step: its number within the run, modulo 6
 template <typename R>
 int res_rebuild_blocks(int n);
 template <typename R>
 int launch_res_begin(const StepArgs<R>& a, const ResArgs<R>& r, cudaStream_t s);
 template <typename R>
-int launch_res_step(const StepArgs<R>& a, const ResArgs<R>& r, cudaStream_t s, double dt, int parity, int phases);
+int launch_res_step(const StepArgs<R>& a, const ResArgs<R>& r, cudaStream_t s, double dt, int step, int phases);
 template <typename R>
 int launch_res_end(const StepArgs<R>& a, const ResArgs<R>& r, cudaStream_t s);
 // number of kernel launches issued by one middle step of grains_gpu_step

@@ -26,12 +26,15 @@
 // lists, memory rows and coordination as before.
 
 // control words
-enum { kResRequest = 0, kResEntries = 1, kResPairs = 2, kResValid = 3, kResObs = 4, kResWords = 8 };
+enum {
+  kResRequest = 0, kResEntries = 1, kResPairs = 2, kResValid = 3, kResObs = 4, kResCountAll = 6, kResWords = 8
+};
 // kResRequest: 0 lists are good, 1 a particle has moved half the skin, other
 // values: first build of a run (the memory rows are current)
 // kResEntries, kResPairs: reservations of a build; kResValid: pairs of a
 // complete build, else -1; kResObs, kResObs + 1: obstacle items of the steps of
-// even and odd parity
+// even and odd parity; kResCountAll: the step's candidate pairs are counted over
+// all cells, not from the step before
 
 constexpr int kResObsMax = 8;   // obstacles per system (a byte each in a particle's state word)
 // the state of a listed pair or of a particle's obstacle
@@ -211,13 +214,13 @@ __device__ __forceinline__ ResConst res_constants(const StepArgs<R>& a, int s, i
 // at -1, on which the other kernels do nothing, and the status bit.
 constexpr int kResHits = 64;  // a particle's listed partners kept in shared memory during its walk
 template <typename R>
-__global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResArgs<R> r, int parity) {
+__global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResArgs<R> r, int step) {
   const int request = *(volatile int*)(r.ctl + kResRequest);
   if (request == 0 || (*(volatile int*)&a.stats->status & GRAINS_GPU_TIMEOUT)) return;
   const int nthreads = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = a.n, C = a.n_cells;
   int* status = &a.stats->status;
-  const int* count = r.count[parity];
+  const int* count = r.count[step % 3];
   __shared__ int offset_s;
   __shared__ int hit_s[256 / kResLanes][kResHits];
   __shared__ int2 range_s[256 / kResLanes][kResRows];
@@ -654,15 +657,78 @@ __device__ __forceinline__ void res_obstacle_one(const StepArgs<R>& a, const Res
   fs.ov_max = fmax(fs.ov_max, ov);
 }
 
+// The number of candidate pairs of the step (the 27 cells around every particle,
+// as the launched broadphase counts them), and the cell counts of the next step
+// cleared.  With n the cells' counts and A their adjacency (27 cells), the number
+// is n.An - N; a step changes few cells, and with d = n_new - n_old the change is
+// d.(A n_old + A n_new), so only cells whose count has changed look around.
+// Counting all cells took 20 us of a step of 200,000 falling spheres and 140 us of
+// one of 500 systems (5 million cells).  The sums kernel adds the number to the
+// statistics.
+template <typename R>
+__device__ __forceinline__ void res_count_candidates(const StepArgs<R>& a, const ResArgs<R>& r, int step, int block,
+                                                     int blocks) {
+  const int* now = r.count[step % 3];
+  const int* old = r.count[(step + 2) % 3];
+  int* next = r.count[(step + 1) % 3];
+  const bool all = *(volatile int*)(r.ctl + kResCountAll) != 0;
+  long long sum = 0;
+  auto around = [&](int c) {  // the 27 cells of c: of both counts (of the new one alone when all cells are counted)
+    int sys = 0;
+    for (int hi = a.n_sys; hi - sys > 1;) {  // the cell's system
+      const int mid = (sys + hi) / 2;
+      if (a.sys[mid].cell_offset <= c) sys = mid;
+      else hi = mid;
+    }
+    const SysDev& S = a.sys[sys];
+    const int local = c - S.cell_offset;
+    const int i = local % S.nbi, k = (local / S.nbi) % S.nbk, j = local / (S.nbi * S.nbk);
+    int m = 0;
+#pragma unroll 9
+    for (int q = 0; q < 27; ++q) {
+      const int ii = i + q % 3 - 1, kk = k + (q / 3) % 3 - 1, jj = j + q / 9 - 1;
+      if (ii >= 0 && ii < S.nbi && jj >= 0 && jj < S.nbj && kk >= 0 && kk < S.nbk) {
+        const int o = cell_index(S, ii, jj, kk);
+        m += now[o];
+        if (!all) m += old[o];
+      }
+    }
+    return m;
+  };
+  const int quads = (a.n_cells + 3) / 4;
+  for (int q = block * kResPairThreads + threadIdx.x; q < quads; q += blocks * kResPairThreads) {
+    const int c = 4 * q;
+    int n4[4], o4[4];
+    if (c + 4 <= a.n_cells) {
+      const int4 x = reinterpret_cast<const int4*>(now)[q], y = reinterpret_cast<const int4*>(old)[q];
+      reinterpret_cast<int4*>(next)[q] = make_int4(0, 0, 0, 0);
+      n4[0] = x.x; n4[1] = x.y; n4[2] = x.z; n4[3] = x.w;
+      o4[0] = y.x; o4[1] = y.y; o4[2] = y.z; o4[3] = y.w;
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool in = c + u < a.n_cells;
+        n4[u] = in ? now[c + u] : 0;
+        o4[u] = in ? old[c + u] : 0;
+        if (in) next[c + u] = 0;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int d = all ? n4[u] : n4[u] - o4[u];
+      if (d != 0) sum += (long long)d * around(c + u);
+    }
+  }
+  warp_add(r.n_cand, (unsigned long long)sum);  // two's complement: changes may be negative
+}
+
 // Blocks [0, pair_blocks): the listed pairs.  Each warp tests 32 or 64 pairs at a
 // time (the exact overlap test of every listed pair) and queues those in contact
 // in shared memory; whenever 32 are queued it runs the law on them, so that the
 // law runs on full warps whatever share of the list is in contact, without a
 // barrier.  64 at a time keeps twice the loads in flight; 32 spreads a short list
 // over more warps.  Then obs_blocks: the obstacle candidates; the other blocks:
-// the number of candidate pairs of the step (the 27 cells around every particle,
-// as the launched broadphase counts them), and the cell counts of the next step
-// cleared.
+// res_count_candidates.
 // Bound by the latency of the gathers and by L2 (about 450 B a contact); four
 // blocks a SM at 128 registers (five at 96 spill: 67.2 against 66.5 us).  200,000
 // spheres, 460,000 contacts: 82 -> 66 us mixed, 103 -> 82 us FP64 with the pair
@@ -670,7 +736,8 @@ __device__ __forceinline__ void res_obstacle_one(const StepArgs<R>& a, const Res
 constexpr int kResPairBlocks = 4;
 template <typename R, bool HOOKE_MEMORY>
 __global__ void __launch_bounds__(kResPairThreads, kResPairBlocks)
-    res_pairs_kernel(StepArgs<R> a, ResArgs<R> r, R dt, int parity, int pair_blocks, int obs_blocks) {
+    res_pairs_kernel(StepArgs<R> a, ResArgs<R> r, R dt, int step, int pair_blocks, int obs_blocks) {
+  const int parity = step & 1;
   constexpr int kQueue = 96;
   __shared__ int queue_s[kResPairThreads / 32][kQueue];
   const unsigned full = 0xffffffffu;
@@ -748,34 +815,7 @@ __global__ void __launch_bounds__(kResPairThreads, kResPairBlocks)
     }
     flush_force_stats(a.stats, fs);
   } else {
-    const int* count = r.count[parity];
-    int* next = r.count[1 - parity];
-    const int blocks = gridDim.x - pair_blocks - obs_blocks;
-    unsigned long long cand = 0;
-    for (int c = (blockIdx.x - pair_blocks - obs_blocks) * kResPairThreads + threadIdx.x; c < a.n_cells;
-         c += blocks * kResPairThreads) {
-      next[c] = 0;
-      const int own = count[c];
-      if (own == 0) continue;
-      int sys = 0;
-      for (int hi = a.n_sys; hi - sys > 1;) {  // the cell's system
-        const int mid = (sys + hi) / 2;
-        if (a.sys[mid].cell_offset <= c) sys = mid;
-        else hi = mid;
-      }
-      const SysDev& S = a.sys[sys];
-      const int local = c - S.cell_offset;
-      const int i = local % S.nbi, k = (local / S.nbi) % S.nbk, j = local / (S.nbi * S.nbk);
-      int around = 0;
-#pragma unroll
-      for (int q = 0; q < 27; ++q) {
-        const int ii = i + q % 3 - 1, kk = k + (q / 3) % 3 - 1, jj = j + q / 9 - 1;
-        if (ii >= 0 && ii < S.nbi && jj >= 0 && jj < S.nbj && kk >= 0 && kk < S.nbk)
-          around += count[cell_index(S, ii, jj, kk)];
-      }
-      cand += (unsigned long long)own * (unsigned long long)(around - 1);
-    }
-    warp_add(&a.stats->n_cand, cand);
+    res_count_candidates(a, r, step, blockIdx.x - pair_blocks - obs_blocks, gridDim.x - pair_blocks - obs_blocks);
   }
 }
 
@@ -826,10 +866,15 @@ __device__ __forceinline__ void res_reorder(const StepArgs<R>& a, const ResArgs<
 // cell marks its partners' lists for res_reorder in the next step (about one
 // list in a hundred a step), so that no step looks up the partners' cells.
 template <typename R>
-__global__ void __launch_bounds__(256) res_sums_kernel(StepArgs<R> a, ResArgs<R> r, R dt_half, double dt, int parity) {
+__global__ void __launch_bounds__(256) res_sums_kernel(StepArgs<R> a, ResArgs<R> r, R dt_half, double dt, int step) {
+  const int parity = step & 1;
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = s < a.n && *(volatile int*)(r.ctl + kResValid) >= 0;
   const ParticleArrays<R>& P = a.cur;
+  if (s == 0) {
+    a.stats->n_cand += *r.n_cand - (unsigned long long)a.n;  // less the particles themselves
+    r.ctl[kResCountAll] = 0;
+  }
   unsigned mask = 0;
   unsigned long long state = 0;
   if (active) {
@@ -920,6 +965,8 @@ int launch_res_begin(const StepArgs<R>& a, const ResArgs<R>& r, cudaStream_t s) 
   if (cudaMemsetAsync(r.bar, 0, 2 * sizeof(unsigned), s) != cudaSuccess) return GRAINS_GPU_CUDA_ERROR;
   if (cudaMemsetAsync(r.ctl + kResRequest, 2, sizeof(int), s) != cudaSuccess) return GRAINS_GPU_CUDA_ERROR;
   if (cudaMemsetAsync(r.ctl + kResValid, 255, sizeof(int), s) != cudaSuccess) return GRAINS_GPU_CUDA_ERROR;
+  if (cudaMemsetAsync(r.ctl + kResCountAll, 1, sizeof(int), s) != cudaSuccess) return GRAINS_GPU_CUDA_ERROR;
+  if (cudaMemsetAsync(r.n_cand, 0, sizeof(unsigned long long), s) != cudaSuccess) return GRAINS_GPU_CUDA_ERROR;
   res_begin_kernel<R><<<grid_for(a.n, 256), 256, 0, s>>>(a, r);
   return check_launch();
 }
@@ -934,13 +981,13 @@ int launch_res_end(const StepArgs<R>& a, const ResArgs<R>& r, cudaStream_t s) {
 // cell keys alternate between the two particle buffers: a.cur.key holds those of
 // the step's positions, a.alt.key takes the next ones.
 template <typename R>
-int launch_res_step(const StepArgs<R>& args, const ResArgs<R>& r, cudaStream_t s, double dt, int parity, int phases) {
+int launch_res_step(const StepArgs<R>& args, const ResArgs<R>& r, cudaStream_t s, double dt, int step, int phases) {
   StepArgs<R> a = args;
-  if (parity) std::swap(a.cur.key, a.alt.key);
+  if (step & 1) std::swap(a.cur.key, a.alt.key);
   if (phases & 1) {
     StepArgs<R> a0 = a;
     ResArgs<R> r0 = r;
-    void* kargs[] = {&a0, &r0, &parity};
+    void* kargs[] = {&a0, &r0, &step};
     if (cudaLaunchCooperativeKernel((const void*)res_rebuild_kernel<R>, dim3(r.rebuild_blocks), dim3(256), kargs, 0,
                                     s) != cudaSuccess)
       return GRAINS_GPU_CUDA_ERROR;
@@ -950,16 +997,16 @@ int launch_res_step(const StepArgs<R>& args, const ResArgs<R>& r, cudaStream_t s
     // obstacle and count blocks follow them
     const int pb = std::min(kResPairBlocks * 148, grid_for(5ll * a.n, kResPairThreads));
     const int ob = std::min(148, grid_for(a.n, 4 * kResPairThreads));
-    const int cb = std::min(2 * 148, grid_for(a.n_cells, kResPairThreads));
+    const int cb = std::min(2 * 148, grid_for(a.n_cells, 4 * kResPairThreads));
     if (r.konst)
-      res_pairs_kernel<R, true><<<pb + ob + cb, kResPairThreads, 0, s>>>(a, r, R(dt), parity, pb, ob);
+      res_pairs_kernel<R, true><<<pb + ob + cb, kResPairThreads, 0, s>>>(a, r, R(dt), step, pb, ob);
     else
-      res_pairs_kernel<R, false><<<pb + ob + cb, kResPairThreads, 0, s>>>(a, r, R(dt), parity, pb, ob);
+      res_pairs_kernel<R, false><<<pb + ob + cb, kResPairThreads, 0, s>>>(a, r, R(dt), step, pb, ob);
   }
   if (phases & 4) {
     StepArgs<R> an = a;
-    an.cell_count = r.count[1 - parity];  // the drift counts the new cells for the next step
-    res_sums_kernel<R><<<grid_for(a.n, 256), 256, 0, s>>>(an, r, R(0.5 * dt), dt, parity);
+    an.cell_count = r.count[(step + 1) % 3];  // the drift counts the new cells for the next step
+    res_sums_kernel<R><<<grid_for(a.n, 256), 256, 0, s>>>(an, r, R(0.5 * dt), dt, step);
   }
   return check_launch();
 }
