@@ -1406,6 +1406,9 @@ int build_tables(grains_gpu_ctx* c) {
     d.ex = s.ex;
     d.ey = s.ey;
     d.ez = s.ez;
+    d.ix = 1. / s.ex;
+    d.iy = 1. / s.ey;
+    d.iz = 1. / s.ez;
     d.gx = s.dom.gravity[0];
     d.gy = s.dom.gravity[1];
     d.gz = s.dom.gravity[2];

@@ -82,6 +82,7 @@ struct ShapeDev {
 struct SysDev {
   double ox, oy, oz;  // grid origin
   double ex, ey, ez;  // cell edges
+  double ix, iy, iz;  // 1 / cell edges (of a cell index that an exact division confirms near a face)
   double gx, gy, gz;  // gravity
   int nbi, nbj, nbk;
   int cell_offset;

@@ -1137,7 +1137,10 @@ __device__ __forceinline__ LawResult<R> obstacle_law(const LawParams<R>& L, R dt
   b1.lever = from_d3<R>(olev);
   b1.pos_minus_contact = from_d3<R>(xsub3(oo, g.point));
   b1.mass = R(kObstacleMass);
-  b1.req = R(pow((0.75 / kPi) * sho.volume, 1. / 3.));
+  // the equivalent radius enters the Hertz laws and the rolling terms only
+  const bool uses_req = L.rolling || L.kr != R(0) || L.type == GRAINS_GPU_HERTZ || L.type == GRAINS_GPU_HERTZ_MEMORY;
+  const double req = uses_req ? pow((0.75 / kPi) * sho.volume, 1. / 3.) : 0.;
+  b1.req = R(req);
   PairFp64 pd;
   if constexpr (sizeof(R) == 4) {
     pd.v0 = widen(vi);
@@ -1149,7 +1152,7 @@ __device__ __forceinline__ LawResult<R> obstacle_law(const LawParams<R>& L, R dt
     pd.m0 = mdi.x;
     pd.m1 = kObstacleMass;
     pd.req0 = mdi.z;
-    pd.req1 = pow((0.75 / kPi) * sho.volume, 1. / 3.);
+    pd.req1 = req;
   }
   return pair_law(L, dt, g, b0, b1, pd, existed, mem, t0, t1);
 }
