@@ -864,25 +864,6 @@ __device__ __forceinline__ void res_reorder(const StepArgs<R>& a, const ResArgs<
   }
 }
 
-// x / d for three numbers, correctly rounded like the division itself.  For
-// floats by one double reciprocal: the double product is within 2^-52 of the
-// quotient, a quotient of two 24-bit numbers is no midpoint of two floats (an odd
-// 25-bit number times a 24-bit one needs more than 24 bits) and lies at least
-// 2^-49 from any, so rounding the product rounds the quotient.
-__device__ __forceinline__ V3<float> res_div(V3<float> x, float d) {
-  const double q = 1. / (double)d;
-  return v3<float>((float)((double)x.x * q), (float)((double)x.y * q), (float)((double)x.z * q));
-}
-__device__ __forceinline__ V3<double> res_div(V3<double> x, double d) { return dv(x, d); }
-
-// the cell index floor((x - o) / e) of the exact division: by the reciprocal
-// (within a few 2^-53 of it), and by the division itself near a cell's face
-__device__ __forceinline__ int res_cell(double x, double o, double e, double inv) {
-  const double d = xsub(x, o), t = d * inv, f = floor(t);
-  const double r = t - f;
-  return r > 1.e-6 && r < 1. - 1.e-6 && fabs(t) < 1.e6 ? int(f) : int(floor(xdiv(d, e)));
-}
-
 // `integrate` for a sphere whose torsor (F, T) is final: the second half kick,
 // the next first half kick, the drift and the cell of the new position.  The same
 // operations; what both kicks share is formed once, since the angular
@@ -904,9 +885,10 @@ __device__ __forceinline__ void res_drift(const StepArgs<R>& a, const SysDev& S,
   Qt<double> q{v3<double>(qd.x, qd.y, qd.z), qd.w};
   const Qt<R> qr{v3<R>(R(qd.x), R(qd.y), R(qd.z)), R(qd.w)};
   const V3<R> Tbf = q_to_body(qr, T);
-  const V3<R> dvel = sc(res_div(F, mass * cf), dt_half);
-  const V3<R> K = sc(v3<R>(Tbf.x / (cf * I.x), Tbf.y / (cf * I.y), Tbf.z / (cf * I.z)), dt_half);
-  const V3<R> dw = res_div((K + K) + sc(K, R(4)), R(6));  // rk3
+  const V3<R> dvel = sc(div3(F, mass * cf), dt_half);
+  const V3<R> at = v3<R>(Divisor<R>(cf * I.x)(Tbf.x), Divisor<R>(cf * I.y)(Tbf.y), Divisor<R>(cf * I.z)(Tbf.z));
+  const V3<R> K = sc(at, dt_half);
+  const V3<R> dw = div3((K + K) + sc(K, R(4)), R(6));  // rk3
   v = v + dvel;
   v = v + dvel;
   wbf = wbf + dw;
@@ -930,17 +912,9 @@ __device__ __forceinline__ void res_drift(const StepArgs<R>& a, const SysDev& S,
     mrotate_left(b, dq);
     for (int t = 0; t < 9; ++t) P.basis[9 * (size_t)s + t] = b.m[t];
   }
-  // |tm| > crust: the square root only near the limit
-  const double far = norm2(tm), lim = md.y * md.y;
-  if ((md.y < 0. || !(far < lim * (1. - 1.e-12))) && norm(tm) > md.y) set_status(a.stats, GRAINS_GPU_MOTION_ERROR);
-  int ci = res_cell(xr.x, S.ox, S.ex, S.ix), cj = res_cell(xr.y, S.oy, S.ey, S.iy),
-      ck = res_cell(xr.z, S.oz, S.ez, S.iz);
-  if (!(-1 < ci && ci < S.nbi && -1 < cj && cj < S.nbj && -1 < ck && ck < S.nbk)) {
-    set_status(a.stats, GRAINS_GPU_OUT_OF_GRID);
-    ci = min(max(ci, 0), S.nbi - 1);
-    cj = min(max(cj, 0), S.nbj - 1);
-    ck = min(max(ck, 0), S.nbk - 1);
-  }
+  if (longer(tm, md.y)) set_status(a.stats, GRAINS_GPU_MOTION_ERROR);
+  int ci, cj, ck;
+  if (!cell_of(S, xr.x, xr.y, xr.z, ci, cj, ck)) set_status(a.stats, GRAINS_GPU_OUT_OF_GRID);
   key = (unsigned)cell_index(S, ci, cj, ck);
   key_out[s] = key;
   atomicAdd(&a.cell_count[key], 1);
