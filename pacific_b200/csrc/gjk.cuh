@@ -126,15 +126,24 @@ GG_HD V3<T> support_local(const LocalBody<T>& B, V3<T> v) {
         for (int moves = 0; moves < B.nverts; ++moves) {
           int next = -1;
           T dn = T(0);
-          for (int k = B.adj_start[cur]; k < B.adj_start[cur + 1]; ++k) {
-            const int c = B.adj[k];
-            if (c == last) continue;
-            const T d = dot(v3<T>(T(B.verts[3 * c]), T(B.verts[3 * c + 1]), T(B.verts[3 * c + 2])), v);
-            if (!(d - h < T(1.e-16))) {
-              next = c;
-              dn = d;
-              break;
+          // four neighbours at a time, so that their loads and products overlap:
+          // one by one, each waited for two loads and a product (pair phase of
+          // 40,000 convex bodies 331 -> 281 us, of 11,111 168 -> 132)
+          const int end = B.adj_start[cur + 1];
+          for (int k = B.adj_start[cur]; k < end && next < 0; k += 4) {
+            int c[4];
+            T d[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              c[j] = B.adj[k + j < end ? k + j : end - 1];
+              d[j] = dot(v3<T>(T(B.verts[3 * c[j]]), T(B.verts[3 * c[j] + 1]), T(B.verts[3 * c[j] + 2])), v);
             }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              if (next < 0 && k + j < end && c[j] != last && !(d[j] - h < T(1.e-16))) {
+                next = c[j];
+                dn = d[j];
+              }
           }
           if (next < 0) break;
           last = cur;
