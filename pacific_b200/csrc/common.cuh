@@ -147,6 +147,46 @@ GG_HD V3<R> round3(V3<R> a) {  // Group3::round(EPSILON), Group3.cpp:390-395
   const R tol = R(kEpsilon);
   return v3<R>(gabs(a.x) < tol ? R(0) : a.x, gabs(a.y) < tol ? R(0) : a.y, gabs(a.z) < tol ? R(0) : a.z);
 }
+// Division by d, correctly rounded like the operator itself.  For floats by one
+// double reciprocal: the double product is within 2^-52 of the quotient, a quotient
+// of two 24-bit numbers is no midpoint of two floats (an odd 25-bit number times a
+// 24-bit one needs more than 24 bits) and lies at least 2^-49 from any, so rounding
+// the product rounds the quotient (below the normal range, 1e-38, to within one
+// unit).
+template <typename R>
+struct Divisor;
+template <>
+struct Divisor<float> {
+  double q;
+  GG_HD explicit Divisor(float d) : q(1. / (double)d) {}
+  GG_HD float operator()(float x) const { return (float)((double)x * q); }
+};
+template <>
+struct Divisor<double> {
+  double d;
+  GG_HD explicit Divisor(double d_) : d(d_) {}
+  GG_HD double operator()(double x) const { return x / d; }
+};
+template <typename R>
+GG_HD V3<R> div3(V3<R> x, R d) {
+  const Divisor<R> by(d);
+  return v3<R>(by(x.x), by(x.y), by(x.z));
+}
+
+// |t| > most: the square root only near the limit
+GG_HD bool longer(V3<double> t, double most) {
+  const double far = norm2(t), lim = most * most;
+  return (most < 0. || !(far < lim * (1. - 1.e-12))) && norm(t) > most;
+}
+
+// the cell index floor((x - o) / e) of the exact division: by the reciprocal
+// (within a few 2^-53 of it), and by the division itself near a cell's face
+GG_HD int cell_coord(double x, double o, double e, double inv) {
+  const double d = xsub(x, o), t = d * inv, f = floor(t);
+  const double r = t - f;
+  return r > 1.e-6 && r < 1. - 1.e-6 && fabs(t) < 1.e6 ? int(f) : int(floor(xdiv(d, e)));
+}
+
 template <typename R>
 GG_HD V3<R> from_d3(D3 a) {
   return v3<R>(R(a.x), R(a.y), R(a.z));

@@ -54,46 +54,6 @@ __device__ __forceinline__ R4<R> st3(V3<R> a, R wv = R(0)) {
 
 __device__ __forceinline__ void set_status(StatsDev* st, int bits) { atomicOr(&st->status, bits); }
 
-// Division by d, correctly rounded like the operator itself.  For floats by one
-// double reciprocal: the double product is within 2^-52 of the quotient, a quotient
-// of two 24-bit numbers is no midpoint of two floats (an odd 25-bit number times a
-// 24-bit one needs more than 24 bits) and lies at least 2^-49 from any, so rounding
-// the product rounds the quotient (below the normal range, 1e-38, to within one
-// unit).
-template <typename R>
-struct Divisor;
-template <>
-struct Divisor<float> {
-  double q;
-  __device__ __forceinline__ explicit Divisor(float d) : q(1. / (double)d) {}
-  __device__ __forceinline__ float operator()(float x) const { return (float)((double)x * q); }
-};
-template <>
-struct Divisor<double> {
-  double d;
-  __device__ __forceinline__ explicit Divisor(double d_) : d(d_) {}
-  __device__ __forceinline__ double operator()(double x) const { return x / d; }
-};
-template <typename R>
-__device__ __forceinline__ V3<R> div3(V3<R> x, R d) {
-  const Divisor<R> by(d);
-  return v3<R>(by(x.x), by(x.y), by(x.z));
-}
-
-// |t| > most: the square root only near the limit
-__device__ __forceinline__ bool longer(V3<double> t, double most) {
-  const double far = norm2(t), lim = most * most;
-  return (most < 0. || !(far < lim * (1. - 1.e-12))) && norm(t) > most;
-}
-
-// the cell index floor((x - o) / e) of the exact division: by the reciprocal
-// (within a few 2^-53 of it), and by the division itself near a cell's face
-__device__ __forceinline__ int cell_coord(double x, double o, double e, double inv) {
-  const double d = xsub(x, o), t = d * inv, f = floor(t);
-  const double r = t - f;
-  return r > 1.e-6 && r < 1. - 1.e-6 && fabs(t) < 1.e6 ? int(f) : int(floor(xdiv(d, e)));
-}
-
 // Cell::GetCell (Base/src/Cell.cpp:172-184) + LinkedCell::getCell validity
 __device__ __forceinline__ bool cell_of(const SysDev& S, double x, double y, double z, int& i, int& j, int& k) {
   i = cell_coord(x, S.ox, S.ex, S.ix);
@@ -2441,9 +2401,13 @@ int launch_forces(const StepArgs<R>& a, cudaStream_t s, double dt, int diag, int
     sums();
     return check_launch();
   }
-  // about two work items per thread in a settled packing; the grid-stride
-  // loop takes any count
-  const int g = (int)std::min<long long>(grid_for(2ll * a.n, fb), 1ll << 20);
+  // about two work items per thread in a settled packing, and one where the
+  // blocks of all of them still run at once, since an item's latency is the time
+  // there (pair phase of 300 convex bodies 103 -> 92 us, 2,000 in FP64 120 -> 107,
+  // 11,111 145 -> 127; a step of 8,000 FP64 spheres by the per-phase calls 203 ->
+  // 183 us); the grid-stride loop takes any count
+  const int all = 148 * GG_PAIRS_MIN_BLOCKS * 128 / fb;
+  const int g = (int)std::min<long long>(std::max(grid_for(2ll * a.n, fb), std::min(grid_for(8ll * a.n, fb), all)), 1ll << 20);
   if (a.has_convex) {  // the GJK items grouped by shape pair, the GJK kernel, the law
     cudaMemsetAsync(a.gjk_bins, 0, 2 * kGjkBins * sizeof(int), s);
     const int gb = 2 * 148;
