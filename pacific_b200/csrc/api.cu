@@ -902,7 +902,13 @@ int ensure_resident(grains_gpu_ctx* c) {
     c->res_buf = nullptr;
     c->res_bytes = 0;
     void* q = nullptr;
-    CK(cudaMalloc(&q, need));
+    const cudaError_t e = cudaMalloc(&q, need);
+    if (e == cudaErrorMemoryAllocation) {  // no room for the lists: the launched pipeline needs none
+      cudaGetLastError();
+      c->res_ok = false;
+      return 0;
+    }
+    CK(e);
     c->res_buf = (char*)q;
     c->res_bytes = need;
   }
