@@ -44,6 +44,10 @@ sys.path.insert(0, ROOT)
 # the list entries of the force evaluation; R4 = 16 B in mixed precision, 32 B
 # in FP64; a contact-memory entry is 44 B / 80 B; a pair's two list entries and
 # its work item count once per particle on average):
+# The formulas are those of the launched pipeline (moving obstacles, convex
+# bodies).  Steps on resident pair lists (spheres) do the same work in
+# res_pairs_kernel and res_sums_kernel; their list walk runs only where a list is
+# rebuilt, so that phase has no fixed bytes there.
 #  contacts_kernel: own position+radius (32), meta (16) and cell key (4), the
 #   9 cell-row ranges (72), list length (4) in/out; z list entries (4 z) and
 #   z/2 work items (8 z/2) out.  Neighbour positions are re-read from L1/L2
@@ -371,9 +375,10 @@ def profile_run(sim, sc, n_steps, t):
     return tp, {k: v[0] / n_steps for k, v in prof.items()}, {k: v for k, v in prof.items()}
 
 
-def roofline(prof_tot, sc, precision, z, peak, peak_kind, traffic_of):
+def roofline(prof_tot, sc, precision, z, peak, peak_kind, traffic_of, resident):
     from pacific_b200 import scenarios as S
-    dom = max([k for k in ["contacts", "pairs", "sums", "sums_kick", "kick_move"] if k in prof_tot],
+    phases = ["pairs", "sums_kick"] if resident else ["contacts", "pairs", "sums", "sums_kick", "kick_move"]
+    dom = max([k for k in phases if k in prof_tot],
               key=lambda k: prof_tot[k][0])
     k_ms, k_n = prof_tot[dom]
     basis = any(sc.shapes[k][0] != S.SPHERE for k in set(np.asarray(sc.particles["shape"]).tolist()))
@@ -382,9 +387,16 @@ def roofline(prof_tot, sc, precision, z, peak, peak_kind, traffic_of):
     # with convex bodies the pair phase also holds the GJK kernels (their runs
     # are bound by divergence and FP64 latency, not by these bytes)
     kernel = "pair phase: gjk_count, gjk_place, gjk_kernel, pairs_kernel" if basis and dom == "pairs" else dom + "_kernel"
+    if resident:
+        kernel = {"pairs": "res_pairs_kernel", "sums_kick": "res_sums_kernel"}[dom]
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": traffic_of(dom), "kernel": kernel, "peak_source": peak_kind,
+            "traffic": traffic_of(kernel[:-len("_kernel")] if resident else dom), "kernel": kernel, "peak_source": peak_kind,
             "algorithmic_bytes_per_launch": alg, "mean_coordination": z, "launch_ms": k_ms / k_n}
+
+
+def on_resident_lists(sim):
+    """Steps on resident pair lists take three launches, all others at least six."""
+    return sim.launches_per_step() == 3
 
 
 def mean_coordination(sim, sc, t):
@@ -477,6 +489,7 @@ def settled_leg(args, lib, sc, local, flush, peak, peak_kind):
     gst = sm.stats()  # of that one force evaluation
     with nvtx("settled_kernels"):
         _, per_step, tot = profile_run(sm, sc, 500, tm)
+    lists = on_resident_lists(sm)
     sm.close()
     s64, _, ms_64 = run(FP64)
     s64.close()
@@ -487,7 +500,7 @@ def settled_leg(args, lib, sc, local, flush, peak, peak_kind):
                 "fp64": {"value": v_64, "ms_per_dem_step": ms_64 / steps, "mixed_over_fp64": v_m / v_64},
                 "kernels_ms_per_dem_step": per_step,
                 "roofline": roofline(tot, sc, "mixed", z, peak, peak_kind,
-                                     lambda k: profiled_traffic(k, sc.name + "_settled", "mixed")),
+                                     lambda k: profiled_traffic(k, sc.name + "_settled", "mixed"), lists),
                 "contact_force_error": contact_force_error(lib, sc, sc2.particles, mem, local,
                                                            "the settled bed read back from its reload file")})
     if gst["n_gjk_calls"]:
@@ -672,8 +685,11 @@ def main():
     h2d = sum(host[kk].nbytes for kk in ["position", "quaternion", "velocity", "omega"])
     d2h = sum(v.nbytes for v in host.values())
     e2e_value = total_particles * args.chunk / e2e_s
-    gather_every = sim.tuning()["gather_every"]
-    launches = sim.launches_per_step() * args.chunk * args.steps + (args.chunk * args.steps) // gather_every
+    # per middle step; the launched pipeline's permutations on top (the starts and
+    # ends of resident runs are not counted)
+    launches = sim.launches_per_step() * args.chunk * args.steps
+    if not on_resident_lists(sim):
+        launches += (args.chunk * args.steps) // sim.tuning()["gather_every"]
 
     line = {
         "metric": "particle-steps/s", "value": value, "unit": "particle-steps/s", "n_gpus": world,
@@ -687,7 +703,7 @@ def main():
                    "l2": "flushed (256 MiB write) between timed steps"},
         "gpu_launches": int(launches),
         "roofline": roofline(prof_tot, sc, args.precision, z, peak, peak_kind,
-                             lambda k: profiled_traffic(k, sc.name, args.precision)),
+                             lambda k: profiled_traffic(k, sc.name, args.precision), on_resident_lists(sim)),
         "e2e": {"value": e2e_value, "unit": "particle-steps/s", "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h), "host_buffers": "pinned", "over_device": e2e_value / value},
         "kernels_ms_per_dem_step": {k: v[0] / n_prof for k, v in prof_tot.items()},

@@ -440,13 +440,15 @@ int grains_gpu_reset_stats(grains_gpu_ctx* ctx);
  *   gather_every   steps between two permutations of the particle arrays
  *                  into cell order (1 .. 64); in between the cell lists are
  *                  rebuilt every step and reached through a permutation.
+ *                  Steps on resident pair lists (below) are permuted every
+ *                  504 steps whatever the period.
  *                  Results do not depend on it: every sum runs in cell order,
  *                  then id order inside a cell.
  *   persistent     1: the middle steps of grains_gpu_step run in one
  *                  cooperative launch (every block resident, the phases
  *                  separated by a grid barrier with a bounded wait) instead of
- *                  6 launches per step replayed from graphs; same results.
- *                  Pays where launch gaps dominate (small systems). */
+ *                  launches replayed from graphs; same results.  Slower
+ *                  than these at every size measured. */
 typedef struct grains_gpu_tuning {
   double  cell_factor;
   int32_t contacts_block;
@@ -473,7 +475,9 @@ int grains_gpu_autotune(grains_gpu_ctx* ctx, double time, double dt, int32_t tri
  * context stream: first_move, sort_gather, contacts, pairs (with the GJK
  * kernel of convex scenarios), sums_kick (the per-particle sums with the
  * second half kick and the next step's first half kick, drift and binning),
- * obstacle_move (the moving obstacles' kernel).
+ * obstacle_move (the moving obstacles' kernel).  Steps on resident pair lists:
+ * sort_gather holds the start of a run and its permutations, contacts the
+ * rebuild of the lists (a launch of every step, early exits included).
  * names: '\n'-separated phase names (cap bytes); ms[k]: total milliseconds of
  * phase k; launches[k]: its kernel launches. */
 int grains_gpu_profile_kernels(grains_gpu_ctx* ctx, int32_t n_steps, double* time, double dt,
@@ -486,9 +490,12 @@ int grains_gpu_profile_kernels(grains_gpu_ctx* ctx, int32_t n_steps, double* tim
  * run out: they set GRAINS_GPU_TIMEOUT and return, and the context stays
  * usable (upload the state again before stepping on). */
 int grains_gpu_set_barrier_test(grains_gpu_ctx* ctx, int64_t polls, int32_t skip_block);
-/* Kernel launches of one middle step of grains_gpu_step: the cell sort (3:
+/* Kernel launches of one middle step of grains_gpu_step.  Spheres among
+ * obstacles that do not move step on resident pair lists: 3 (the rebuild of the
+ * lists, which returns at once in most steps, the pairs, the sums with the
+ * kick).  Otherwise: the cell sort (3:
  * the tile-local scan, the scatter, the cell sort), contacts, the GJK phase of
- * convex scenarios with Johnson's GJK (two kernels grouping the GJK items by
+ * convex scenarios (two kernels grouping the GJK items by
  * shape pair, the GJK kernel), pairs, the sums with the kick, the contact
  * forces on force-driven obstacles when there are some, and the obstacle
  * move when obstacles move.  The permutation of the arrays into cell order
