@@ -664,7 +664,7 @@ size_t res_layout(int64_t cap, int obs_stride, int hist_cap, int list_cap, size_
     at += (bytes + kResAlign - 1) / kResAlign * kResAlign;
   };
   const size_t n = (size_t)cap, m = n * (size_t)std::max(1, obs_stride);
-  put(0, 16 * sizeof(int) + 2 * sizeof(unsigned) + 2 * sizeof(double) + 4096 * sizeof(int));  // control, barrier, skin, candidates, sums
+  put(0, 16 * sizeof(int) + 2 * sizeof(unsigned) + 4 * sizeof(double) + 4096 * sizeof(int));  // control, barrier, skin, candidates, totals, sums
   put(1, n * sizeof(double4));
   put(2, n * sizeof(int2));
   put(3, n * (size_t)list_cap * sizeof(int));
@@ -696,7 +696,8 @@ ResArgs<R> make_res(grains_gpu_ctx* c) {
   r.bar = (unsigned*)(r.ctl + 16);
   r.skin = (double*)(r.bar + 2);
   r.n_cand = (unsigned long long*)(r.skin + 1);
-  r.block_sums = (int*)(r.n_cand + 1);
+  r.total = r.n_cand + 1;
+  r.block_sums = (int*)(r.total + 2);
   // a wide skin lasts longer but lists more pairs: 0.2 r_min (a tenth of a
   // diameter) lists 8 to 9 partners a particle in a dense bed, of which 5 touch
   r.skin0 = 0.2 * c->r_min;

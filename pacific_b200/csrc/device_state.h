@@ -259,6 +259,7 @@ struct ResConst {
 template <typename R>
 struct ResArgs {
   int* ctl;              // control words (kResRequest ...)
+  unsigned long long* total;  // entries and pairs that a build has counted
   double* skin;          // the skin of the present lists
   double skin0;          // the skin asked for
   const double* r_max;   // per system: the largest radius

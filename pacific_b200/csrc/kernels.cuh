@@ -782,17 +782,18 @@ __device__ __forceinline__ void warp_add(unsigned long long* dst, unsigned long 
 
 // one warp-aggregated reservation of work-item slots for every lane's count
 // (every lane of the warp calls it); returns the lane's first slot
-__device__ __forceinline__ int warp_reserve(int* counter, int count) {
+template <typename C>
+__device__ __forceinline__ C warp_reserve(C* counter, C count) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  int incl = count;
+  C incl = count;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(full, incl, o);
+    const C y = __shfl_up_sync(full, incl, o);
     if (lane >= o) incl += y;
   }
-  const int total = __shfl_sync(full, incl, 31);
-  int base = 0;
+  const C total = __shfl_sync(full, incl, 31);
+  C base = 0;
   if (lane == 31 && total > 0) base = atomicAdd(counter, total);
   base = __shfl_sync(full, base, 31);
   return base + incl - count;

@@ -27,11 +27,11 @@
 
 // control words
 enum {
-  kResRequest = 0, kResEntries = 1, kResPairs = 2, kResValid = 3, kResObs = 4, kResCountAll = 6, kResWords = 8
+  kResRequest = 0, kResValid = 3, kResObs = 4, kResCountAll = 6, kResWords = 8
 };
 // kResRequest: 0 lists are good, 1 a particle has moved half the skin, other
 // values: first build of a run (the memory rows are current)
-// kResEntries, kResPairs: reservations of a build; kResValid: pairs of a
+// kResValid: pairs of a
 // complete build, else -1; kResObs, kResObs + 1: obstacle items of the steps of
 // even and odd parity; kResCountAll: the step's candidate pairs are counted over
 // all cells, not from the step before
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
   if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
   if (tid == 0) {
     r.ctl[kResValid] = -1;
-    r.ctl[kResEntries] = r.ctl[kResPairs] = 0;
+    r.total[0] = r.total[1] = 0;
   }
   int part = 0;
   for (int b = threadIdx.x; b < (int)blockIdx.x; b += blockDim.x) part += r.block_sums[b];
@@ -283,12 +283,15 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
       });
       __syncwarp();
       const bool leader = lane == 0;
-      int e0 = warp_reserve(r.ctl + kResEntries, leader ? cnt : 0), p0 = warp_reserve(r.ctl + kResPairs, leader ? own : 0);
-      e0 = __shfl_sync(0xffffffffu, e0, res_group_shift());
-      p0 = __shfl_sync(0xffffffffu, p0, res_group_shift());
-      const bool fits = (long long)e0 + cnt <= r.ent_cap && (long long)p0 + own <= r.pair_cap;
+      // in 64 bits: particles piled up count more than 2^31 entries before the lists are known not to fit
+      unsigned long long e64 = warp_reserve(r.total, leader ? (unsigned long long)cnt : 0ull),
+                         p64 = warp_reserve(r.total + 1, leader ? (unsigned long long)own : 0ull);
+      e64 = __shfl_sync(0xffffffffu, e64, res_group_shift());
+      p64 = __shfl_sync(0xffffffffu, p64, res_group_shift());
+      const bool fits = e64 + cnt <= (unsigned long long)r.ent_cap && p64 + own <= (unsigned long long)r.pair_cap;
+      const int e0 = fits ? (int)e64 : 0, p0 = fits ? (int)p64 : 0;
       if (s < n && leader) {
-        r.ent[s] = make_int2(fits ? e0 : 0, fits ? cnt : 0);
+        r.ent[s] = make_int2(e0, fits ? cnt : 0);
         r.x0[s] = a.cur.xr[s];
         r.dirty[0][s] = r.dirty[1][s] = 0;
       }
@@ -297,7 +300,7 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
       auto enter = [&](bool in, int e) {
         const bool o = in && (e & kOwnBit);
         const unsigned ins = res_ballot(in), owners = res_ballot(o);
-        if (in && fits) {
+        if (in) {
           const int q = e0 + q0 + __popc(ins & lower);
           r.nb[q] = e;
           r.res[q].f.w = R(0);
@@ -310,9 +313,9 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
         q0 += __popc(ins);
         rank += __popc(owners);
       };
-      const bool kept = cnt <= kResHits;
-      for (int q = 0; __any_sync(0xffffffffu, kept && q < cnt); q += kResLanes) {
-        const bool in = kept && q + lane < cnt;
+      const bool kept = cnt <= kResHits || !fits;  // nothing is entered when it does not fit
+      for (int q = 0; __any_sync(0xffffffffu, kept && fits && q < cnt); q += kResLanes) {
+        const bool in = kept && fits && q + lane < cnt;
         enter(in, in ? hits[q + lane] : 0);
       }
       if (__any_sync(0xffffffffu, !kept)) {  // more than shared memory holds: walked again
@@ -323,14 +326,14 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
       __syncwarp();
     }
     if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
-    const int ne = *(volatile int*)(r.ctl + kResEntries), np = *(volatile int*)(r.ctl + kResPairs);
-    if (ne <= r.ent_cap && np <= r.pair_cap) break;
+    const unsigned long long ne = *(volatile unsigned long long*)r.total, np = *(volatile unsigned long long*)(r.total + 1);
+    if (ne <= (unsigned long long)r.ent_cap && np <= (unsigned long long)r.pair_cap) break;
     if (skin < 1.e-3 * r.skin0) {  // more contacts than the lists hold
       if (tid == 0) set_status(a.stats, GRAINS_GPU_PAIR_OVERFLOW);
       return;
     }
     if (!grid_barrier(r.bar, status, a.barrier_polls)) return;  // every block has read the totals
-    if (tid == 0) r.ctl[kResEntries] = r.ctl[kResPairs] = 0;
+    if (tid == 0) r.total[0] = r.total[1] = 0;
     if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
     skin *= 0.5;
   }
@@ -374,7 +377,7 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
   if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
   if (tid == 0) {
     *r.skin = skin;
-    r.ctl[kResValid] = r.ctl[kResPairs];
+    r.ctl[kResValid] = (int)r.total[1];
     r.ctl[kResRequest] = 0;
   }
 }
