@@ -436,7 +436,9 @@ int grains_gpu_reset_stats(grains_gpu_ctx* ctx);
  *                  of 4; 0 = 32 for spheres, 64 when other shapes are
  *                  present): contacting particles and candidate obstacles of
  *                  a force evaluation; a particle with more fails the step
- *                  with GRAINS_GPU_PAIR_OVERFLOW
+ *                  with GRAINS_GPU_PAIR_OVERFLOW (resident pair lists that
+ *                  no longer fit leave the state at the last step whose
+ *                  lists did)
  *   gather_every   steps between two permutations of the particle arrays
  *                  into cell order (1 .. 64); in between the cell lists are
  *                  rebuilt every step and reached through a permutation.

@@ -27,10 +27,13 @@
 
 // control words
 enum {
-  kResRequest = 0, kResValid = 3, kResObs = 4, kResCountAll = 6, kResWords = 8
+  kResRequest = 0, kResFailed = 1, kResRowPairs = 2, kResValid = 3, kResObs = 4, kResCountAll = 6, kResWords = 8
 };
 // kResRequest: 0 lists are good, 1 a particle has moved half the skin, other
 // values: first build of a run (the memory rows are current)
+// kResFailed: the contacts did not fit in the lists; the run stands still from
+// that step on.  kResRowPairs: the rows hold the pairs' memories, not the
+// obstacles' (a rebuild that has not ended)
 // kResValid: pairs of a
 // complete build, else -1; kResObs, kResObs + 1: obstacle items of the steps of
 // even and odd parity; kResCountAll: the step's candidate pairs are counted over
@@ -216,7 +219,8 @@ constexpr int kResHits = 64;  // a particle's listed partners kept in shared mem
 template <typename R>
 __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResArgs<R> r, int step) {
   const int request = *(volatile int*)(r.ctl + kResRequest);
-  if (request == 0 || (*(volatile int*)&a.stats->status & GRAINS_GPU_TIMEOUT)) return;
+  if (request == 0 || *(volatile int*)(r.ctl + kResFailed) || (*(volatile int*)&a.stats->status & GRAINS_GPU_TIMEOUT))
+    return;
   const int nthreads = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = a.n, C = a.n_cells;
   int* status = &a.stats->status;
@@ -248,6 +252,7 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
   if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
   if (tid == 0) {
     r.ctl[kResValid] = -1;
+    if (request == 1) r.ctl[kResRowPairs] = 1;
     r.total[0] = r.total[1] = 0;
   }
   int part = 0;
@@ -329,7 +334,10 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
     const unsigned long long ne = *(volatile unsigned long long*)r.total, np = *(volatile unsigned long long*)(r.total + 1);
     if (ne <= (unsigned long long)r.ent_cap && np <= (unsigned long long)r.pair_cap) break;
     if (skin < 1.e-3 * r.skin0) {  // more contacts than the lists hold
-      if (tid == 0) set_status(a.stats, GRAINS_GPU_PAIR_OVERFLOW);
+      if (tid == 0) {
+        set_status(a.stats, GRAINS_GPU_PAIR_OVERFLOW);
+        r.ctl[kResFailed] = 1;
+      }
       return;
     }
     if (!grid_barrier(r.bar, status, a.barrier_polls)) return;  // every block has read the totals
@@ -378,6 +386,7 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
   if (tid == 0) {
     *r.skin = skin;
     r.ctl[kResValid] = (int)r.total[1];
+    r.ctl[kResRowPairs] = 0;
     r.ctl[kResRequest] = 0;
   }
 }
@@ -451,18 +460,21 @@ __global__ void __launch_bounds__(256) res_begin_kernel(StepArgs<R> a, ResArgs<R
   }
 }
 
-// the end of a run: every memory back into the rows, pairs then obstacles
+// the end of a run: every memory back into the rows, pairs then obstacles.  Without
+// complete lists the rows hold everything (a first build), or the pairs' memories
+// (a rebuild that failed)
 template <typename R>
 __global__ void __launch_bounds__(256) res_end_kernel(StepArgs<R> a, ResArgs<R> r) {
-  // without a complete build the rows still hold everything
-  if (*(volatile int*)(r.ctl + kResValid) < 0) return;
+  const bool valid = *(volatile int*)(r.ctl + kResValid) >= 0;
+  if (!valid && !*(volatile int*)(r.ctl + kResRowPairs)) return;
   const int s = (blockIdx.x * blockDim.x + threadIdx.x) / kResLanes;
   const bool active = s < a.n;
-  int cnt = res_flush_pairs(a, r, s, active);
+  int cnt = valid ? res_flush_pairs(a, r, s, active) : 0;
   if (!active || res_lane() != 0) return;
   const unsigned long long state = r.obs_state[s];
   if (!state) return;
   const int row = a.cur.orig[s];
+  if (!valid) cnt = a.hist_n_prev[row];
   HistEntry<R>* h = a.hist_prev + (size_t)row * a.hist_cap;
   for (int o = 0; o < kResObsMax; ++o) {
     if (!((state >> (8 * o)) & kResMemory)) continue;
@@ -813,7 +825,8 @@ __global__ void __launch_bounds__(kResPairThreads, kResPairBlocks)
     }
     flush_force_stats(a.stats, fs);
   } else if ((int)blockIdx.x < pair_blocks + obs_blocks) {
-    const int n_items = *(volatile int*)(r.ctl + kResObs + parity);
+    // (no lists: the run stands still, its obstacles too)
+    const int n_items = *(volatile int*)(r.ctl + kResValid) >= 0 ? *(volatile int*)(r.ctl + kResObs + parity) : 0;
     const int b = blockIdx.x - pair_blocks;
     for (int k = b * kResPairThreads + threadIdx.x; k < n_items; k += obs_blocks * kResPairThreads)
       res_obstacle_one(a, r, r.obs_item[parity][k], dt, fs);
@@ -939,11 +952,16 @@ template <typename R>
 __global__ void __launch_bounds__(256, 3) res_sums_kernel(StepArgs<R> a, ResArgs<R> r, R dt_half, double dt, int step) {
   const int parity = step & 1;
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool active = s < a.n && *(volatile int*)(r.ctl + kResValid) >= 0;
+  const bool valid = *(volatile int*)(r.ctl + kResValid) >= 0, active = s < a.n && valid;
   const ParticleArrays<R>& P = a.cur;
   if (s == 0) {
-    a.stats->n_cand += *r.n_cand - (unsigned long long)a.n;  // less the particles themselves
+    if (valid) a.stats->n_cand += *r.n_cand - (unsigned long long)a.n;  // less the particles themselves
     r.ctl[kResCountAll] = 0;
+  }
+  if (s < a.n && !valid) {  // the particle stays; its key and count go on to the next step's arrays
+    const unsigned key = P.key[s];
+    a.alt.key[s] = key;
+    atomicAdd(&a.cell_count[key], 1);
   }
   unsigned mask = 0;
   unsigned long long state = 0;

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 from pacific_b200 import scenarios as S
-from pacific_b200.abi import CUDA_ERROR, MIXED, PAIR_OVERFLOW, TIMEOUT, GrainsError
+from pacific_b200.abi import CUDA_ERROR, FP64, MIXED, PAIR_OVERFLOW, TIMEOUT, GrainsError
 
 from helpers import make
 
@@ -38,3 +38,64 @@ def test_more_entries_than_32_bits_count(gpu_lib):
     code = failing_step(sim, 8, 1.0e-9)
     assert code & PAIR_OVERFLOW and not code & (TIMEOUT | CUDA_ERROR)
     sim.close()
+
+
+def memories(sim):
+    """Contact memory by (owner, other)"""
+    m = sim.contact_memory(cap=64 * sim.n)
+    values = np.concatenate([m["kdelta"], m["prev_normal"], m["spring_torque"]], axis=1)
+    return {k: v for k, v in zip(zip(m["owner"].tolist(), m["other"].tolist()), values)}
+
+
+def shrinking_lattice(precision):
+    """A cubic lattice of overlapping spheres on the floor that shrinks by 1e-4 a
+    step: an inner sphere has 26 neighbours in touch (the shells up to sqrt(3)
+    spacings), and 6 more from the step on in which two spacings are less than a
+    diameter."""
+    side, r, dt = 20, 0.8e-3, 1.0e-7
+    n, a = side ** 3, 1.00085 * r
+    sc = S.small_box(n, seed=1, velocity_sigma=0.0)
+    k = np.arange(n)
+    ijk = np.stack([k % side, k // side % side, k // side ** 2], 1)
+    x = a * ijk + np.random.default_rng(3).uniform(-1.0e-10, 1.0e-10, (n, 3))
+    sc.particles = S._spheres(n, np.full(n, r), 2500.0, x + [5.0e-3, 5.0e-3, r - 1.0e-6],
+                              -1.0e-4 / dt * (x - [9.0 * a, 10.0 * a, 0.0]), 0.5e-3)
+    sc.laws = [[(p, q, S.HOOKE_MEMORY, [1.0e2, 0.9, -1.0, 0.5, 0.8e2, 0.0, 0.0, 0.0]) for p, q, _, _ in sc.laws[0]]]
+    sc.domains[0]["gravity"] = (0.0, 0.0, 0.0)
+    sc.dt = dt
+    return sc
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED])
+def test_a_run_stands_still_where_its_lists_do_not_fit(gpu_lib, precision):
+    """The lattice outgrows a list capacity of 28 in the middle of a run: the call
+    ends in PAIR_OVERFLOW with the particles and the contact memory (of pairs and
+    of the floor) as after the last step whose lists fitted, the state that the
+    launched pipeline has after that step."""
+    sc = shrinking_lattice(precision)
+    sim = make(gpu_lib, sc, precision)
+    sim.set_tuning(list_capacity=28)
+    assert sim.launches_per_step() == 3
+    sim.initialize_leapfrog(0.0, sc.dt)
+    assert failing_step(sim, 25, sc.dt) == PAIR_OVERFLOW
+    sim.reset_stats()
+    at, memory = sim.download()["position"], memories(sim)
+    sim.close()
+    ref = make(gpu_lib, sc, precision)
+    ref.set_tuning(list_capacity=52)  # more than twice the memory's 24: the launched pipeline
+    assert ref.launches_per_step() > 3
+    ref.initialize_leapfrog(0.0, sc.dt)
+    steps, t = 0, 0.0
+    while steps < 25:
+        t = ref.step(1, t, sc.dt)
+        steps += 1
+        if np.array_equal(ref.download()["position"], at):
+            break
+    assert 4 < steps < 24
+    want = memories(ref)
+    ref.close()
+    # the force evaluation that ended the call listed at most 28 contacts a sphere
+    assert len(memory) > 0.8 * len(want) and set(memory) <= set(want)
+    assert sum(other < 0 for _, other in memory) == sum(other < 0 for _, other in want) == 400
+    for k in memory:
+        assert np.array_equal(memory[k], want[k]), k
