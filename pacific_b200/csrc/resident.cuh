@@ -140,7 +140,8 @@ __device__ __forceinline__ void res_walk(const StepArgs<R>& a, const ResArgs<R>&
         bool hit = false, own = false;
         if (t[u] >= 0 && t[u] != s) {
           const double dx = xj[u].x - xi.x, dy = xj[u].y - xi.y, dz = xj[u].z - xi.z;
-          const double rs = (xi.w + xj[u].w) + skin;  // symmetric: both sides list the pair
+          // symmetric: both sides list the pair; with the margin every contact even without a skin
+          const double rs = (xi.w + xj[u].w) * (1. + 1.e-12) + skin;
           hit = dx * dx + dy * dy + dz * dz < rs * rs;
           own = hit && id < a.cur.meta[t[u]].x;
         }
@@ -333,7 +334,7 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
     if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
     const unsigned long long ne = *(volatile unsigned long long*)r.total, np = *(volatile unsigned long long*)(r.total + 1);
     if (ne <= (unsigned long long)r.ent_cap && np <= (unsigned long long)r.pair_cap) break;
-    if (skin < 1.e-3 * r.skin0) {  // more contacts than the lists hold
+    if (skin == 0.) {  // more contacts than the lists hold
       if (tid == 0) {
         set_status(a.stats, GRAINS_GPU_PAIR_OVERFLOW);
         r.ctl[kResFailed] = 1;
@@ -343,7 +344,7 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
     if (!grid_barrier(r.bar, status, a.barrier_polls)) return;  // every block has read the totals
     if (tid == 0) r.total[0] = r.total[1] = 0;
     if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
-    skin *= 0.5;
+    skin = skin < 1.e-3 * r.skin0 ? 0. : 0.5 * skin;  // without a skin: the contacts alone, built in every step
   }
   // each pair's entry in the partner's list, and its memory from the owner's row
   for (int s = group; s < padded; s += groups) {

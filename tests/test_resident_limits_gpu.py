@@ -99,3 +99,35 @@ def test_a_run_stands_still_where_its_lists_do_not_fit(gpu_lib, precision):
     assert sum(other < 0 for _, other in memory) == sum(other < 0 for _, other in want) == 400
     for k in memory:
         assert np.array_equal(memory[k], want[k]), k
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED])
+def test_contacts_that_just_fit(gpu_lib, precision):
+    """Every inner sphere of a lattice touches 32 others, the list capacity, and
+    24 more miss it by 2e-5 of a diameter: too many for any skin, yet the contacts
+    alone fit, so the call is accepted and its results are the launched
+    pipeline's."""
+    side, a = 20, 0.7e-3
+    n, r = side ** 3, 0.5 * np.sqrt(5.0) * a * (1.0 - 2.0e-5)
+    sc = shrinking_lattice(precision)
+    k = np.arange(n)
+    x = a * np.stack([k % side, k // side % side, k // side ** 2], 1) + 5.0e-3
+    x += np.random.default_rng(4).uniform(-1.0e-10, 1.0e-10, (n, 3))
+    sc.particles = S._spheres(n, np.full(n, r), 2500.0, x, np.zeros((n, 3)), 0.5e-3)
+    sc.domains[0]["cell_size"] = 2.0 * r
+    sc.obstacles = [[]]
+    out = []
+    for capacity in (32, 52):  # resident lists, the launched pipeline
+        sim = make(gpu_lib, sc, precision)
+        sim.set_tuning(list_capacity=capacity)
+        assert (sim.launches_per_step() == 3) == (capacity == 32)
+        sim.initialize_leapfrog(0.0, 1.0e-8)
+        sim.step(9, 0.0, 1.0e-8)
+        sim.synchronize()
+        out.append((sim.download(), memories(sim), sim.stats()))
+        sim.close()
+    (a0, m0, s0), (a1, m1, s1) = out
+    assert a0["coordination"].max() == 32 and s0["status"] == s1["status"] == 0
+    for key in a0:
+        assert np.array_equal(a0[key], a1[key]), key
+    assert set(m0) == set(m1) and all(np.array_equal(m0[q], m1[q]) for q in m0)
