@@ -490,7 +490,10 @@ int grains_gpu_profile_kernels(grains_gpu_ctx* ctx, int32_t n_steps, double* tim
  * gives up (default 2^24, about a second), skip_block = a block that leaves the
  * kernel before its first barrier (-1 = none), so that the other blocks' waits
  * run out: they set GRAINS_GPU_TIMEOUT and return, and the context stays
- * usable (upload the state again before stepping on). */
+ * usable (upload the state again before stepping on).  The same for the kernel
+ * that builds the resident pair lists; there the block leaves the rebuilds within
+ * a run, not the build that starts it, and the run stands still from the step of
+ * that rebuild on. */
 int grains_gpu_set_barrier_test(grains_gpu_ctx* ctx, int64_t polls, int32_t skip_block);
 /* Kernel launches of one middle step of grains_gpu_step.  Spheres among
  * obstacles that do not move step on resident pair lists: 3 (the rebuild of the

@@ -214,17 +214,27 @@ __device__ __forceinline__ ResConst res_constants(const StepArgs<R>& a, int s, i
 }
 
 // One cooperative launch: the cell lists, the pair lists, the memory.  Every
-// barrier wait is bounded (grid_barrier); a build that gave up leaves kResValid
-// at -1, on which the other kernels do nothing, and the status bit.
+// barrier wait is bounded (grid_barrier).  A build that gives up, at whichever
+// barrier, leaves kResValid at -1, on which the other kernels do nothing, and the
+// status bit, on which no later launch builds.
 constexpr int kResHits = 64;  // a particle's listed partners kept in shared memory during its walk
 template <typename R>
 __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResArgs<R> r, int step) {
   const int request = *(volatile int*)(r.ctl + kResRequest);
-  if (request == 0 || *(volatile int*)(r.ctl + kResFailed) || (*(volatile int*)&a.stats->status & GRAINS_GPU_TIMEOUT))
-    return;
+  if (request == 0) return;
   const int nthreads = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
+  if (*(volatile int*)(r.ctl + kResFailed) || (*(volatile int*)&a.stats->status & GRAINS_GPU_TIMEOUT)) {
+    if (threadIdx.x == 0) r.ctl[kResValid] = -1;
+    return;
+  }
+  // a test of the bounded waits: this block leaves a rebuild before its first barrier
+  if (request == 1 && (int)blockIdx.x == a.barrier_skip_block) return;
+  auto meet = [&]() {
+    const bool ok = grid_barrier(r.bar, &a.stats->status, a.barrier_polls);
+    if (!ok && threadIdx.x == 0) r.ctl[kResValid] = -1;
+    return ok;
+  };
   const int n = a.n, C = a.n_cells;
-  int* status = &a.stats->status;
   const int* count = r.count[step % 3];
   __shared__ int offset_s;
   __shared__ int hit_s[256 / kResLanes][kResHits];
@@ -250,7 +260,7 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
     run += total;
   }
   if (threadIdx.x == 0) r.block_sums[blockIdx.x] = run;
-  if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+  if (!meet()) return;
   if (tid == 0) {
     r.ctl[kResValid] = -1;
     if (request == 1) r.ctl[kResRowPairs] = 1;
@@ -270,11 +280,11 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
     a.cell_start[i] = v;
     a.cell_cursor[i] = v;
   }
-  if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+  if (!meet()) return;
   for (int s = tid; s < n; s += nthreads) scatter_one(a, s);
-  if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+  if (!meet()) return;
   for (int c = tid; c < C; c += nthreads) cell_order(a, a.cell_start[c], a.cell_start[c + 1]);
-  if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+  if (!meet()) return;
   // the lists, with half the skin again when they do not fit
   double skin = r.skin0;
   for (;;) {
@@ -331,7 +341,7 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
       }
       __syncwarp();
     }
-    if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+    if (!meet()) return;
     const unsigned long long ne = *(volatile unsigned long long*)r.total, np = *(volatile unsigned long long*)(r.total + 1);
     if (ne <= (unsigned long long)r.ent_cap && np <= (unsigned long long)r.pair_cap) break;
     if (skin == 0.) {  // more contacts than the lists hold
@@ -341,9 +351,9 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
       }
       return;
     }
-    if (!grid_barrier(r.bar, status, a.barrier_polls)) return;  // every block has read the totals
+    if (!meet()) return;  // every block has read the totals
     if (tid == 0) r.total[0] = r.total[1] = 0;
-    if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+    if (!meet()) return;
     skin = skin < 1.e-3 * r.skin0 ? 0. : 0.5 * skin;  // without a skin: the contacts alone, built in every step
   }
   // each pair's entry in the partner's list, and its memory from the owner's row
@@ -383,7 +393,7 @@ __global__ void __launch_bounds__(256, 3) res_rebuild_kernel(StepArgs<R> a, ResA
       r.state[mine] = st;
     }
   }
-  if (!grid_barrier(r.bar, status, a.barrier_polls)) return;
+  if (!meet()) return;
   if (tid == 0) {
     *r.skin = skin;
     r.ctl[kResValid] = (int)r.total[1];

@@ -131,3 +131,38 @@ def test_contacts_that_just_fit(gpu_lib, precision):
     for key in a0:
         assert np.array_equal(a0[key], a1[key]), key
     assert set(m0) == set(m1) and all(np.array_equal(m0[q], m1[q]) for q in m0)
+
+
+@pytest.mark.parametrize("polls,skip", [(20000, 0), (20000, 3), (1, -1)])
+def test_a_build_whose_waits_run_out(gpu_lib, polls, skip):
+    """A block that leaves a rebuild before its first barrier, or waits of one
+    poll: TIMEOUT comes back, the particles stand where the last step with
+    complete lists left them, and the context runs on after a new upload."""
+    sc = S.small_box(1000, seed=3, velocity_sigma=1.0, radius_range=(0.9, 1.1), spacing=2.3, jitter=0.02)
+    sc.dt = 2.0e-6
+    sim, ref = make(gpu_lib, sc, FP64), make(gpu_lib, sc, FP64)
+    sim.set_barrier_test(polls=polls, skip_block=skip)
+    sim.initialize_leapfrog(0.0, sc.dt)
+    assert failing_step(sim, 400, sc.dt) & TIMEOUT
+    sim.reset_stats()
+    at = sim.download()["position"]
+    ref.set_tuning(list_capacity=20)  # the launched pipeline
+    ref.initialize_leapfrog(0.0, sc.dt)
+    steps, t, found = 0, 0.0, False
+    while steps < 399 and not found:
+        t = ref.step(1, t, sc.dt)
+        steps += 1
+        found = np.array_equal(ref.download()["position"], at)
+    # the first build of the run gives up, or one that particles have asked for
+    assert found and (steps == 1 if skip < 0 else steps > 1)
+    sim.set_barrier_test()
+    sim.upload(sc.particles)
+    sim.initialize_leapfrog(0.0, sc.dt)
+    sim.step(steps + 20, 0.0, sc.dt)
+    sim.synchronize()
+    ref.step(20, t, sc.dt)
+    a, b = sim.download(), ref.download()
+    for key in a:
+        assert np.array_equal(a[key], b[key]), key
+    sim.close()
+    ref.close()
