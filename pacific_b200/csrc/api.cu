@@ -1789,6 +1789,7 @@ int grains_gpu_upload_particles(grains_gpu_ctx* c, const grains_gpu_particles* p
     CK(cudaStreamSynchronize(c->stream));  // the host vectors above are pageable
   }
   c->moved = 0;
+  if (c->hydro_on || c->fluid_corrected) drop_graphs(c);  // they hold both
   c->fluid_corrected = 0;  // md.w (rho_f / rho_p) was uploaded as 0
   c->hydro_on = false;
   c->obs_force_valid = false;  // no force evaluation of these particles yet

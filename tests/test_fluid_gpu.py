@@ -174,3 +174,28 @@ def test_basilisk_interface_drives_the_attached_context(gpu_lib):
     assert np.array_equal(a.download()["position"], b.download()["position"])
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("capacity", [32, 20])  # resident lists, the launched pipeline
+def test_an_upload_ends_the_fluid_forces(gpu_lib, capacity):
+    """Steps replayed from graphs with the fluid's forces; particles uploaded
+    anew are dry, in the steps after it too."""
+    sc = S.small_box(200, seed=2, velocity_sigma=0.05, spacing=2.3)
+    n = len(sc.particles["id"])
+    out = []
+    for wet in (True, False):
+        sim = make(gpu_lib, sc, FP64)
+        sim.set_tuning(list_capacity=capacity)
+        if wet:
+            sim.set_fluid(1000.0, True, np.full(n, 2500.0))
+            sim.set_hydro_forces(np.full((n, 3), 1.0e-3), None)
+            sim.initialize_leapfrog(0.0, sc.dt)
+            sim.step(70, 0.0, sc.dt)
+            sim.upload(sc.particles)
+        sim.initialize_leapfrog(0.0, sc.dt)
+        sim.step(70, 0.0, sc.dt)
+        sim.synchronize()
+        out.append(sim.download())
+        sim.close()
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k]), k
