@@ -498,7 +498,14 @@ int grains_gpu_set_barrier_test(grains_gpu_ctx* ctx, int64_t polls, int32_t skip
 /* Kernel launches of one middle step of grains_gpu_step.  Spheres among
  * obstacles that do not move step on resident pair lists: 3 (the rebuild of the
  * lists, which returns at once in most steps, the pairs, the sums with the
- * kick).  Otherwise: the cell sort (3:
+ * kick).  That holds for calls of at least 7 steps, at most 8 obstacles a system,
+ * cells no smaller than the system's largest diameter, radii within a factor of 4,
+ * a list capacity of 24 to twice the history capacity, and persistent = 0; and
+ * while the fastest sphere takes at least 3 steps (above 30,000 particles 4, few
+ * contacts: up to 8) for a tenth of the smallest radius, by the speeds that the last
+ * call before (other than grains_gpu_step, which does not wait) has seen.  Beyond that the launched steps are the faster ones;
+ * the results are the same, and this count does not look at the speeds.
+ * Otherwise: the cell sort (3:
  * the tile-local scan, the scatter, the cell sort), contacts, the GJK phase of
  * convex scenarios (two kernels grouping the GJK items by
  * shape pair, the GJK kernel), pairs, the sums with the kick, the contact

@@ -195,6 +195,9 @@ struct grains_gpu_ctx {
   double r_min = 0, r_max = 0; // radii of the uploaded particles
   std::vector<double> sys_r_max;  // and the largest of each system
   bool res_ok = false;         // the uploaded scene can run on resident lists
+  unsigned* pace = nullptr;    // the largest squared speed that gathers have met (float bits)
+  float speed2 = 0.f;          // and that of the last force evaluation read with a status
+  unsigned items = 0;          // with its work items
   bool hooke_memory_only = false;  // every contact law is HookeMemory without a rolling spring
   bool hooke_memory_pairs = false; // and every pair of materials of the uploaded particles has one
   cudaGraphExec_t res_graph[4] = {nullptr, nullptr, nullptr, nullptr};  // by (cur, hcur)
@@ -644,6 +647,7 @@ StepArgs<R> make_args(grains_gpu_ctx* c) {
   a.gdir_next = c->gdir[1 - c->hcur];
   a.gdir_n_next = c->gdir_n[1 - c->hcur];
   a.barrier_polls = c->barrier_polls;
+  a.pace = c->res_ok ? c->pace : nullptr;
   a.barrier_skip_block = c->barrier_skip_block;
   a.contacts_block = c->contacts_block;
   a.forces_block = c->forces_block;
@@ -768,10 +772,15 @@ int sort_now(grains_gpu_ctx* c, int gather_forces, bool gather = true) {
 int sort_for_step(grains_gpu_ctx* c) { return sort_now(c, 0, c->since_gather + 1 >= c->gather_every); }
 
 int read_status(grains_gpu_ctx* c) {
-  int st = 0;
-  CK(cudaMemcpyAsync(&st, &c->stats->status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  StatsDev w;
+  CK(cudaMemcpyAsync(&w.status, &c->stats->status, 3 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  return st;
+  if (w.speed) {
+    w.speed &= 0x7fffffffu;
+    std::memcpy(&c->speed2, &w.speed, sizeof(c->speed2));
+    c->items = w.items;
+  }
+  return w.status;
 }
 
 std::string status_message(int st) {
@@ -962,6 +971,27 @@ constexpr int kResMinSteps = 6;
 
 bool use_resident(const grains_gpu_ctx* c, int middle) {
   return c->res_ok && !c->persistent && middle >= kResMinSteps;
+}
+
+// Fast spheres: one that has moved half the skin (0.1 r_min) makes all lists be
+// built anew, so the fastest sphere's steps per build decide between the
+// pipelines.  us a step (mixed) launched | resident at 10, 7, 5, 4, 3 steps per build:
+//   200,000 apart          58 |  48  60  75  88 111    100,000 apart   36 | 31 37 44 50 63
+//   200,000 in pairs       72 |  58  70  87 101 123     60,000 apart   32 | 24 28 32 36 44
+//   200,000 in chains     129 |  73  83 100 115 146     40,000 apart   34 | 23 24 28 30 36
+//   200,000 cubic lattice 210 | 133 146 167 184 220     60,000 cubic   76 | 53 57 62 67 74
+//   200,000, 12 neighbours 293 | 168   - 214   - 267    27,000 apart   30 | 18 20 23 25 29
+// and at 2 steps 333 against 293 for 200,000 with 12 neighbours, 37 against 30 for
+// 27,000 apart, 31 against 26 for 1,000.  So the lists need 3 steps per build, 4 above
+// 30,000 spheres, and where these have few contacts (work items of a force
+// evaluation below 3/4 a particle) up to 8 from 100,000 on.  The speed is the
+// one that came with the last status read (every call but grains_gpu_step reads it).
+// Either pipeline gives the same bits.
+bool too_fast(const grains_gpu_ctx* c, double dt) {
+  const double large = std::min(1., std::max(0., ((double)c->n - 30000.) / 70000.));
+  const bool apart = (double)c->items < 0.75 * (double)c->n;
+  const double least = apart ? 3. + 5. * large : (large > 0. ? 4. : 3.);
+  return !(std::ceil(0.1 * c->r_min / (std::sqrt((double)c->speed2) * dt)) >= least);
 }
 
 // n middle steps on resident lists
@@ -1185,6 +1215,10 @@ int grains_gpu_create(const grains_gpu_config* cfg, grains_gpu_ctx** out) {
     ok = c->coord && c->perm && c->stats && c->pairs && c->pairs_n && c->pair_force && c->pair_sys && c->clock &&
          c->work_n && c->gjk_next && c->gjk_bins;
   }
+  if (ok) {
+    c->pace = dalloc<unsigned>(1, c->pool);
+    ok = c->pace;
+  }
   if (!ok) {
     c->err = "cudaMalloc failed for the requested capacity";
     *out = c;
@@ -1195,6 +1229,7 @@ int grains_gpu_create(const grains_gpu_config* cfg, grains_gpu_ctx** out) {
   cudaMemsetAsync(c->stats, 0, sizeof(StatsDev), c->stream);
   cudaMemsetAsync(c->work_n, 0, sizeof(int), c->stream);
   cudaMemsetAsync(c->gjk_next, 0, sizeof(int), c->stream);
+  cudaMemsetAsync(c->pace, 0, sizeof(unsigned), c->stream);
   cudaStreamSynchronize(c->stream);
   *out = c;
   return 0;
@@ -2491,7 +2526,7 @@ int grains_gpu_step(grains_gpu_ctx* c, int32_t n_steps, double* time, double dt)
   // evaluation and leaves its second half kick pending
   if (int rc = first_move(c, dt, *time)) return rc;
   int middle = n_steps - 1;
-  if (use_resident(c, middle)) {
+  if (use_resident(c, middle) && !too_fast(c, dt)) {
     if (int rc = resident_steps(c, middle, dt)) return rc;
     middle = 0;
   }
@@ -2739,7 +2774,7 @@ int grains_gpu_profile_kernels(grains_gpu_ctx* c, int32_t n_steps, double* time,
   cudaEventElapsedTime(&m, ev[0], ev[1]);
   acc[0] += m;
   cnt[0] += 1;
-  const bool resident = use_resident(c, n_steps - 1);
+  const bool resident = use_resident(c, n_steps - 1) && !too_fast(c, dt);
   if (resident)
     if (int rc = resident_begin(c)) return rc;
   for (int k = 0; k < n_steps; ++k) {

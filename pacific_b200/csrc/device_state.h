@@ -156,7 +156,11 @@ struct StatsDev {
   unsigned long long overlap_max_bits;
   double overlap_sum;
   int status;
-  int pad;
+  // of the last force evaluation that ended a call, read with the status: the bits
+  // of the largest squared speed with the sign bit set (0: none yet), the work items
+  unsigned speed;
+  unsigned items;
+  unsigned pad;
 };
 
 template <typename R>
@@ -242,6 +246,7 @@ struct StepArgs {
   int barrier_skip_block;   // persistent kernel: a block that leaves at once (a test of the bounded wait), or -1
   int contacts_block;    // threads per block of contacts_kernel (<= 256)
   int forces_block;      // threads per block of forces_kernel (<= 128)
+  unsigned* pace;        // bits of the largest squared speed that gathers have met, or null
 };
 
 // Resident pair lists (resident.cuh): the state of a run of middle steps of

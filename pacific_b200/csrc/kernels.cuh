@@ -406,6 +406,17 @@ template <typename R>
 __global__ void __launch_bounds__(256) gather_kernel(StepArgs<R> a, int gather_forces) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < a.n) gather_one(a, t, gather_forces);
+  if (!a.pace) return;
+  float fast = 0.f;
+  if (t < a.n) {
+    const float v2 = (float)norm2(ld3<R>(a.alt.v[t]));
+    fast = v2 <= 3.e38f ? v2 : INFINITY;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) fast = fmaxf(fast, __shfl_xor_sync(0xffffffffu, fast, o));
+  // few warps exceed what others have found: no queue of atomics
+  if ((threadIdx.x & 31) == 0 && __float_as_uint(fast) > *(volatile unsigned*)a.pace)
+    atomicMax(a.pace, __float_as_uint(fast));
 }
 
 // ---------------------------------------------------------------------------
@@ -1856,6 +1867,11 @@ template <typename R, bool KICK = false>
 __global__ void __launch_bounds__(256) sums_kernel(StepArgs<R> a, R dt_half, double dt) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s == 0) {
+    if (!KICK && a.pace) {
+      a.stats->speed = *a.pace | 0x80000000u;
+      a.stats->items = (unsigned)*a.work_n;
+      *a.pace = 0;
+    }
     *a.work_n = 0;
     if (a.gjk_next) *a.gjk_next = 0;
   }

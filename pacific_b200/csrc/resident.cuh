@@ -837,7 +837,8 @@ __global__ void __launch_bounds__(kResPairThreads, kResPairBlocks)
     flush_force_stats(a.stats, fs);
   } else if ((int)blockIdx.x < pair_blocks + obs_blocks) {
     // (no lists: the run stands still, its obstacles too)
-    const int n_items = *(volatile int*)(r.ctl + kResValid) >= 0 ? *(volatile int*)(r.ctl + kResObs + parity) : 0;
+    const int valid = *(volatile int*)(r.ctl + kResValid), listed = *(volatile int*)(r.ctl + kResObs + parity);
+    const int n_items = valid >= 0 ? listed : 0;
     const int b = blockIdx.x - pair_blocks;
     for (int k = b * kResPairThreads + threadIdx.x; k < n_items; k += obs_blocks * kResPairThreads)
       res_obstacle_one(a, r, r.obs_item[parity][k], dt, fs);

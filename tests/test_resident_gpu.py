@@ -122,3 +122,50 @@ def test_what_does_not_run_on_resident_lists(gpu_lib):
         sim.step(9, 0.0, sc.dt)
         sim.synchronize()
         sim.close()
+
+
+def moving_lattice(n, share, contacts, overlap=1.0e-3):
+    """Spheres on a cubic lattice, each in touch with its x neighbours (or none),
+    that move together by `share` of a radius per step."""
+    r, dt, side = 1.0e-3, 1.0e-6, int(np.ceil(n ** (1.0 / 3.0)))
+    k = np.arange(n)
+    gap = np.array([(2.0 - overlap) * r if contacts else 2.6 * r, 2.6 * r, 2.6 * r])
+    x = 5.0e-3 + gap * np.stack([k % side, k // side % side, k // side ** 2], 1)
+    sc = S.small_box(8, seed=1)
+    v = np.tile([share * r / dt, 0.0, 0.0], (n, 1))
+    v += np.random.default_rng(5).normal(0.0, 1.0e-5 * r / dt, (n, 3))
+    sc.particles = S._spheres(n, np.full(n, r), 2500.0, x, v, 0.1 * r)
+    sc.obstacles = [[]]
+    sc.domains = [dict(origin=(0.0,) * 3, size=tuple(x.max(0) + 10.0e-3), cell_size=2.0 * r, gravity=(0.0,) * 3)]
+    sc.dt = dt
+    return sc
+
+
+@pytest.mark.parametrize("n,contacts,share,resident", [
+    (1000, False, 0.045, True), (1000, False, 0.055, False), (1000, True, 0.045, True), (1000, True, 0.055, False),
+    (65000, False, 0.018, True), (65000, False, 0.021, False),
+    (110000, False, 0.013, True), (110000, False, 0.0145, False), (110000, True, 0.03, True),
+    (110000, True, 0.036, False)])
+def test_fast_spheres_take_the_launched_pipeline(gpu_lib, n, contacts, share, resident):
+    """Both sides of the rule on the steps between two builds, and the same bits
+    on both pipelines; a call that starts slowly goes
+    back to the lists."""
+    sc = moving_lattice(n, share, contacts)
+    out = []
+    for capacity in (32, 20):
+        sim = make(gpu_lib, sc, MIXED)
+        sim.set_tuning(list_capacity=capacity)
+        sim.initialize_leapfrog(0.0, sc.dt)
+        t, phases = sim.profile_kernels(12, 0.0, sc.dt)
+        launches = {k: v[1] for k, v in phases.items()}
+        assert (launches["contacts"] == 1) == (resident and capacity == 32)
+        sim.step(9, t, sc.dt)
+        sim.synchronize()
+        out.append(sim.download())
+        sim.update({**sc.particles, "velocity": 0.1 * sc.particles["velocity"]})
+        sim.initialize_leapfrog(0.0, sc.dt)
+        _, phases = sim.profile_kernels(12, 0.0, sc.dt)
+        assert (phases["contacts"][1] == 1) == (capacity == 32)
+        sim.close()
+    for k in out[0]:
+        assert np.array_equal(out[0][k], out[1][k]), k
