@@ -853,8 +853,13 @@ __global__ void __launch_bounds__(256, GG_CONTACTS_MIN_BLOCKS) contacts_kernel(S
 // loads, which is all the time there is while the chip is nearly idle; with more
 // particles than threads the lanes' extra instructions cost more than the chain.
 // B200, per launch, thread against lanes: 2,000 convex bodies 39 against 17 us,
-// 20,000 among 66 moving obstacles 53 against 35, a bed of 30,000 spheres 36
-// against 25, of 60,000 41 against 51, of 200,000 75 against 139 us.
+// 20,000 among 66 moving obstacles 53 against 35, 32,000 51 against 45, 40,000 54
+// against 47; beds of spheres: 24,000 35 against 25, 32,000 35 against 33, 40,000
+// 35 against 34, 60,000 41 against 51, 200,000 75 against 139 us.  On lattices, whose
+// particles lie in the order of their cells, the threads win from 16,000 on: cubic,
+// 24,000 19 against 22, 40,000 18 against 30 us; falling, 8,000 15 against 12, 16,000
+// 17 against 18, 40,000 17 against 25.  So the line for spheres lies between the two,
+// and for convex bodies at the largest size that was measured in favour.
 constexpr int kContactLanes = 8;
 
 // the particle's list; cnt: entries listed, owned: those that become work items
@@ -1008,7 +1013,8 @@ __device__ __forceinline__ void emit_work_group(const StepArgs<R>& a, int s, int
   }
 }
 
-constexpr int kContactLanesMax = 40000;  // particles up to which the lanes are no slower in a dense bed
+// particles up to which the lanes build the lists
+constexpr int kContactLanesSpheres = 28000, kContactLanesConvex = 40000;
 template <typename R>
 __global__ void __launch_bounds__(256, 3) contacts_lanes_kernel(StepArgs<R> a) {
   const int s = (blockIdx.x * blockDim.x + threadIdx.x) / kContactLanes;
@@ -2402,7 +2408,7 @@ int launch_forces(const StepArgs<R>& a, cudaStream_t s, double dt, int diag, int
   const int cb = (a.contacts_block >= 32 && a.contacts_block <= 256) ? a.contacts_block : 256;
   const int fb = (a.forces_block >= 32 && a.forces_block <= 128) ? a.forces_block : 128;
   if (phases & 1) {
-    if (a.n <= kContactLanesMax)
+    if (a.n <= (a.has_convex ? kContactLanesConvex : kContactLanesSpheres))
       contacts_lanes_kernel<R><<<grid_for((long long)kContactLanes * a.n, cb), cb, 0, s>>>(a);
     else
       contacts_kernel<R><<<grid_for(a.n, cb), cb, 0, s>>>(a);

@@ -17,14 +17,18 @@ def first(p, n):
     return {k: (None if v is None else v[:n]) for k, v in p.items()}
 
 
+@pytest.mark.parametrize("convex", [False, True])
 @pytest.mark.parametrize("precision", [FP64, MIXED])
-def test_contact_lists_by_eight_lanes_and_by_one_thread(gpu_lib, precision):
-    """Lists are built by eight lanes per particle up to 40,000 particles and by
-    one thread above: one particle more leaves the forces on all particles out
-    of its reach as they were."""
-    sc = S.small_box(40001, seed=2, velocity_sigma=0.1, radius_range=(0.95, 1.05), spacing=2.0)
+def test_contact_lists_by_eight_lanes_and_by_one_thread(gpu_lib, precision, convex):
+    """Lists are built by eight lanes per particle up to 28,000 spheres (40,000
+    convex bodies) and by one thread above: one particle more leaves the forces
+    on all particles out of its reach as they were."""
+    if convex:
+        m, sc = 40000, S.convex_box(40001, seed=2, spacing=3.4)
+    else:
+        m, sc = 28000, S.small_box(28001, seed=2, velocity_sigma=0.1, radius_range=(0.95, 1.05), spacing=2.0)
     out = []
-    for n in (40001, 40000):
+    for n in (m + 1, m):
         few = S.Scenario(**{**sc.__dict__, "particles": first(sc.particles, n)})
         sim = make(gpu_lib, few, precision)
         sim.initialize_leapfrog(0.0, sc.dt)
@@ -32,10 +36,11 @@ def test_contact_lists_by_eight_lanes_and_by_one_thread(gpu_lib, precision):
         out.append((d, sim.stats()))
         sim.close()
     x = sc.particles["position"]
-    apart = np.linalg.norm(x[:40000] - x[40000], axis=1) > 5.0e-3
-    assert apart.sum() > 39000 and out[0][0]["coordination"].max() >= 4
+    apart = np.linalg.norm(x[:m] - x[m], axis=1) > (8.0e-3 if convex else 5.0e-3)
+    assert apart.sum() > 0.97 * m and (convex or out[0][0]["coordination"].max() >= 4)
+    assert not convex or out[1][1]["n_gjk_calls"] > 10000  # pairs listed and tested
     for k in STATE:
-        assert np.array_equal(out[0][0][k][:40000][apart], out[1][0][k][apart]), k
+        assert np.array_equal(out[0][0][k][:m][apart], out[1][0][k][apart]), k
     assert out[0][1]["status"] == out[1][1]["status"]
 
 
