@@ -467,7 +467,11 @@ int grains_gpu_set_tuning(grains_gpu_ctx* ctx, const grains_gpu_tuning* tuning);
  * broadphase block, cell factor), keeps the fastest that completed without
  * error, applies it and restores the state exactly (particles, contact
  * memory, obstacle poses).  The candidates cover the list capacity, the two
- * block shapes, the gather period and the cell factor (coordinate descent).
+ * block shapes, the gather period, the persistent launch and the cell factor.  A
+ * context whose steps run on resident pair lists (grains_gpu_launches_per_step)
+ * keeps the block shapes and the gather period, which these do not use, and with
+ * fewer than 7 trial_steps, which would not run on the lists, every tuning that
+ * keeps it on them.
  * time = the current simulation time. */
 int grains_gpu_autotune(grains_gpu_ctx* ctx, double time, double dt, int32_t trial_steps,
                         grains_gpu_tuning* best, double* best_ms);

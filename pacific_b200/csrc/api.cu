@@ -887,10 +887,9 @@ int with_res(grains_gpu_ctx* c, F f) {
 // cells, as the launched broadphase needs); radii within a factor of 4 (the skin
 // is a share of the smallest); list and memory capacities no smaller than a dense
 // packing needs.
+bool res_capacity(const grains_gpu_ctx* c, int clist_cap) { return clist_cap >= 24 && 2 * c->hist_cap >= clist_cap; }
 bool res_scene(const grains_gpu_ctx* c) {
-  if (c->n < 1 || c->has_convex || c->n_moving > 0 || c->n_force_obs > 0 || c->clist_cap < 24 ||
-      2 * c->hist_cap < c->clist_cap)
-    return false;
+  if (c->n < 1 || c->has_convex || c->n_moving > 0 || c->n_force_obs > 0 || !res_capacity(c, c->clist_cap)) return false;
   if (!(c->r_min > 0) || c->r_max > 4. * c->r_min) return false;
   for (size_t k = 0; k < c->sys.size(); ++k) {
     const SysHost& s = c->sys[k];
@@ -2939,6 +2938,8 @@ struct Snapshot {
   bool pending = false;
   double pending_dt = 0.;
   int64_t steps_done = 0;
+  float speed2 = 0.f;
+  unsigned items = 0;
 };
 
 std::vector<std::pair<void*, size_t>> snapshot_fields(grains_gpu_ctx* c, int cur, int hcur) {
@@ -2969,6 +2970,8 @@ int take_snapshot(grains_gpu_ctx* c, Snapshot& s) {
   s.pending = c->pending_kick2;
   s.pending_dt = c->pending_dt;
   s.steps_done = c->steps_done;
+  s.speed2 = c->speed2;
+  s.items = c->items;
   for (auto& f : snapshot_fields(c, c->cur, c->hcur)) {
     void* q = nullptr;
     if (cudaMalloc(&q, f.second) != cudaSuccess) return GRAINS_GPU_CUDA_ERROR;
@@ -2991,6 +2994,8 @@ int restore_snapshot(grains_gpu_ctx* c, const Snapshot& s) {
   c->pending_kick2 = s.pending;
   c->pending_dt = s.pending_dt;
   c->steps_done = s.steps_done;
+  c->speed2 = s.speed2;
+  c->items = s.items;
   c->sorted = false;
   c->keys_valid = false;
   if (cudaMemsetAsync(c->stats, 0, sizeof(StatsDev), c->stream) != cudaSuccess) return GRAINS_GPU_CUDA_ERROR;
@@ -3039,6 +3044,13 @@ int grains_gpu_autotune(grains_gpu_ctx* c, double time, double dt, int32_t trial
   };
   double t_best = trial(cur);
   grains_gpu_tuning b = cur;
+  // A scene of resident lists: trials of fewer steps than those start with would
+  // choose among launched steps for runs that take the lists, so the tunings that
+  // leave the lists are not tried then; and the launch shapes and the gather
+  // period, which the lists' steps do not use, are left as they are.
+  const bool scene = c->res_ok, short_trials = trial_steps <= kResMinSteps;
+  auto lists = [&](const grains_gpu_tuning& t) { return scene && res_capacity(c, t.list_capacity) && !t.persistent; };
+  auto leaves = [&](const grains_gpu_tuning& t) { return short_trials && lists(b) && !lists(t); };
   // coordinate descent: list capacity, force block, broadphase block, cell factor
   const int caps_sphere[] = {16, 24, 32}, caps_convex[] = {32, 48, 64};
   const int* caps = c->has_convex ? caps_convex : caps_sphere;
@@ -3046,34 +3058,35 @@ int grains_gpu_autotune(grains_gpu_ctx* c, double time, double dt, int32_t trial
     grains_gpu_tuning t = b;
     t.list_capacity = caps[k];
     if (t.list_capacity == b.list_capacity) continue;
+    if (leaves(t)) continue;
     const double ms = trial(t);
     if (ms > 0. && (t_best < 0. || ms < t_best)) { t_best = ms; b = t; }
   }
   for (int fb : {64, 128}) {
     grains_gpu_tuning t = b;
     t.forces_block = fb;
-    if (fb == b.forces_block) continue;
+    if (lists(b) || fb == b.forces_block) continue;
     const double ms = trial(t);
     if (ms > 0. && (t_best < 0. || ms < t_best)) { t_best = ms; b = t; }
   }
   for (int cb : {128, 256}) {
     grains_gpu_tuning t = b;
     t.contacts_block = cb;
-    if (cb == b.contacts_block) continue;
+    if (lists(b) || cb == b.contacts_block) continue;
     const double ms = trial(t);
     if (ms > 0. && (t_best < 0. || ms < t_best)) { t_best = ms; b = t; }
   }
   for (int ge : {1, 2, 4, 8, 16}) {
     grains_gpu_tuning t = b;
     t.gather_every = ge;
-    if (ge == b.gather_every) continue;
+    if (lists(b) || ge == b.gather_every) continue;
     const double ms = trial(t);
     if (ms > 0. && (t_best < 0. || ms < t_best)) { t_best = ms; b = t; }
   }
   for (int ps : {0, 1}) {
     grains_gpu_tuning t = b;
     t.persistent = ps;
-    if (ps == b.persistent) continue;
+    if (ps == b.persistent || leaves(t)) continue;
     const double ms = trial(t);
     if (ms > 0. && (t_best < 0. || ms < t_best)) { t_best = ms; b = t; }
   }

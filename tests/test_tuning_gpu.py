@@ -135,3 +135,19 @@ def test_persistent_barrier_wait_runs_out_and_the_context_recovers(gpu_lib):
     a, b = s.download(), fresh.download()
     for k in ["position", "velocity", "omega"]:
         assert np.array_equal(a[k], b[k]), k
+
+
+@pytest.mark.parametrize("trial_steps", [1, 3, 6, 7, 40])
+def test_autotune_keeps_a_context_on_its_lists(gpu_lib, trial_steps):
+    """Trials too short for resident lists do not choose a tuning that leaves
+    them, and no trial chooses the launch shapes that their steps do not use."""
+    sim = make(gpu_lib, evolved_box(), MIXED)
+    assert sim.launches_per_step() == 3
+    sim.initialize_leapfrog(0.0, 1.0e-6)
+    before = sim.tuning()
+    best, _ = sim.autotune(0.0, 1.0e-6, trial_steps=trial_steps)
+    if trial_steps < 7:
+        assert sim.launches_per_step() == 3 and not best["persistent"]
+    if sim.launches_per_step() == 3:
+        assert all(best[k] == before[k] for k in ("contacts_block", "forces_block", "gather_every"))
+    sim.close()
