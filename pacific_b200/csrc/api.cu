@@ -3036,6 +3036,7 @@ int grains_gpu_autotune(grains_gpu_ctx* c, double time, double dt, int32_t trial
       int rc = grains_gpu_step(c, trial_steps, &tt, dt);
       cudaEventRecord(e1, c->stream);
       if (rc || cudaEventSynchronize(e1) != cudaSuccess) return -1.;
+      if (finish_call(c)) return -1.;  // the errors of the steps themselves: a list that overflowed
       float ms = 0.f;
       cudaEventElapsedTime(&ms, e0, e1);
       if (rep == 1) ms_best = ms;

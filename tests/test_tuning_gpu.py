@@ -151,3 +151,25 @@ def test_autotune_keeps_a_context_on_its_lists(gpu_lib, trial_steps):
     if sim.launches_per_step() == 3:
         assert all(best[k] == before[k] for k in ("contacts_block", "forces_block", "gather_every"))
     sim.close()
+
+
+@pytest.mark.parametrize("trial_steps", [3, 20])
+def test_autotune_rejects_lists_that_overflow(gpu_lib, trial_steps):
+    """Inner spheres of a tight lattice touch 26 others: capacities of 16 and 24
+    fail their trials, however fast their shortened lists are."""
+    side, a = 16, 0.9e-3
+    n, r = side ** 3, 0.88e-3
+    sc = S.small_box(n, seed=1)
+    k = np.arange(n)
+    x = a * np.stack([k % side, k // side % side, k // side ** 2], 1) + 5.0e-3
+    sc.particles = S._spheres(n, np.full(n, r), 2500.0, x, np.zeros((n, 3)), 0.5e-3)
+    sc.laws = [[(p, q, S.HOOKE_MEMORY, [1.0e2, 0.9, -1.0, 0.5, 0.8e2, 0.0, 0.0, 0.0]) for p, q, _, _ in sc.laws[0]]]
+    sc.obstacles = [[]]
+    sim = make(gpu_lib, sc, MIXED)
+    sim.initialize_leapfrog(0.0, 1.0e-8)
+    assert sim.download()["coordination"].max() == 26
+    best, _ = sim.autotune(0.0, 1.0e-8, trial_steps=trial_steps)
+    assert best["list_capacity"] == 32
+    sim.step(20, 0.0, 1.0e-8)
+    sim.synchronize()
+    sim.close()
