@@ -483,7 +483,7 @@ int grains_gpu_autotune(grains_gpu_ctx* ctx, double time, double dt, int32_t tri
  * second half kick and the next step's first half kick, drift and binning),
  * obstacle_move (the moving obstacles' kernel).  Steps on resident pair lists:
  * sort_gather holds the rebuild of the lists (a launch of every step, early
- * exits included), the start of a run and its permutations.
+ * exits included), the start and the end of a run and its permutations.
  * names: '\n'-separated phase names (cap bytes); ms[k]: total milliseconds of
  * phase k; launches[k]: its kernel launches. */
 int grains_gpu_profile_kernels(grains_gpu_ctx* ctx, int32_t n_steps, double* time, double dt,

@@ -993,6 +993,14 @@ bool too_fast(const grains_gpu_ctx* c, double dt) {
   return !(std::ceil(0.1 * c->r_min / (std::sqrt((double)c->speed2) * dt)) >= least);
 }
 
+// between two runs: the arrays into cell order, and the counts the next lists start from
+int resident_permute(grains_gpu_ctx* c) {
+  if (int rc = sort_now(c, 0)) return rc;
+  CK(cudaMemsetAsync(c->cell_count, 0, (size_t)c->n_cells * sizeof(int), c->stream));
+  const int rc = with_args(c, [&](auto& a) { return launch_bin(a, c->stream); });
+  return rc ? fail(c, rc, "bin kernel launch failed") : 0;
+}
+
 // n middle steps on resident lists
 int resident_steps(grains_gpu_ctx* c, int n, double dt) {
   while (n > 0) {
@@ -1024,12 +1032,8 @@ int resident_steps(grains_gpu_ctx* c, int n, double dt) {
     for (; k > 0; --k, ++step)
       if (int rc = resident_step(c, dt, step)) return rc;
     if (int rc = resident_end(c, run)) return rc;
-    if (n > 0) {  // into cell order, and the counts the next lists start from
-      if (int rc = sort_now(c, 0)) return rc;
-      CK(cudaMemsetAsync(c->cell_count, 0, (size_t)c->n_cells * sizeof(int), c->stream));
-      const int rc = with_args(c, [&](auto& a) { return launch_bin(a, c->stream); });
-      if (rc) return fail(c, rc, "bin kernel launch failed");
-    }
+    if (n > 0)
+      if (int rc = resident_permute(c)) return rc;
   }
   return 0;
 }
@@ -2774,28 +2778,35 @@ int grains_gpu_profile_kernels(grains_gpu_ctx* c, int32_t n_steps, double* time,
   acc[0] += m;
   cnt[0] += 1;
   const bool resident = use_resident(c, n_steps - 1) && !too_fast(c, dt);
-  if (resident)
-    if (int rc = resident_begin(c)) return rc;
   for (int k = 0; k < n_steps; ++k) {
     const bool last = (k == n_steps - 1);
     if (resident && !last) {
-      // a step on resident lists: the rebuild (or its check) counts as the sort,
-      // the overlap tests and the law as the pairs
+      // a step on resident lists: the rebuild (or its check), the start and the end
+      // of a run and the permutation between two count as the sort, the overlap
+      // tests and the law as the pairs
+      const int at = k % kResGather, middle_left = n_steps - 2 - k;
+      const bool ends = at == kResGather - 1 || middle_left == 0;
+      CK(cudaEventRecord(ev[1], c->stream));
+      if (at == 0)
+        if (int rc = resident_begin(c)) return rc;
       for (int q = 0; q < 3; ++q) {
-        CK(cudaEventRecord(ev[1 + q], c->stream));
-        if (int rc = resident_step(c, dt, k, 1 << q)) return rc;
+        if (int rc = resident_step(c, dt, at, 1 << q)) return rc;
+        CK(cudaEventRecord(ev[2 + q], c->stream));
       }
-      CK(cudaEventRecord(ev[4], c->stream));
-      CK(cudaEventSynchronize(ev[4]));
-      const int phase[3] = {1, 3, 4};
-      for (int q = 0; q < 3; ++q) {
+      if (ends)
+        if (int rc = resident_end(c, at + 1)) return rc;
+      if (ends && middle_left > 0)
+        if (int rc = resident_permute(c)) return rc;
+      CK(cudaEventRecord(ev[5], c->stream));
+      CK(cudaEventSynchronize(ev[5]));
+      const int phase[4] = {1, 3, 4, 1};
+      for (int q = 0; q < 4; ++q) {
         float t = 0;
         cudaEventElapsedTime(&t, ev[1 + q], ev[2 + q]);
         acc[phase[q]] += t;
-        cnt[phase[q]] += 1;
+        if (q < 3) cnt[phase[q]] += 1;
       }
-      if (k == n_steps - 2)
-        if (int rc = resident_end(c, n_steps - 1)) return rc;
+      cnt[1] += (at == 0 ? 1 : 0) + (ends ? 1 : 0) + (ends && middle_left > 0 ? 5 : 0);
       continue;
     }
     CK(cudaEventRecord(ev[1], c->stream));

@@ -169,3 +169,29 @@ def test_fast_spheres_take_the_launched_pipeline(gpu_lib, n, contacts, share, re
         sim.close()
     for k in out[0]:
         assert np.array_equal(out[0][k], out[1][k]), k
+
+
+@pytest.mark.parametrize("steps", [7, 520])
+def test_profiled_steps_are_those_of_a_step_call(gpu_lib, steps):
+    """The profile runs the schedule of grains_gpu_step, the permutation after 504
+    steps included, and counts its launches."""
+    sc = S.small_box(300, seed=6, velocity_sigma=0.5, spacing=2.2)
+    sc.dt = 2.0e-6
+    out = []
+    for profiled in (True, False):
+        sim = make(gpu_lib, sc, MIXED)
+        sim.initialize_leapfrog(0.0, sc.dt)
+        if profiled:
+            _, phases = sim.profile_kernels(steps, 0.0, sc.dt)
+        else:
+            sim.step(steps, 0.0, sc.dt)
+            sim.synchronize()
+        out.append((sim.download(), sim.stats()))
+        sim.close()
+    runs = 2 if steps > 504 else 1
+    # rebuilds, starts and ends, five per permutation, the sort of the last step
+    assert phases["sort_gather"][1] == steps - 1 + 2 * runs + 5 * (runs - 1) + 3
+    assert phases["pairs"][1] == phases["sums_kick"][1] == steps
+    for k in out[0][0]:
+        assert np.array_equal(out[0][0][k], out[1][0][k]), k
+    assert out[0][1]["n_candidate_pairs"] == out[1][1]["n_candidate_pairs"]
