@@ -989,6 +989,7 @@ class AdjEngineT : public AdjointEngine {
 
  public:
   AdjEngineT(const ContextView& v, int checkpoint_every) {
+    view_ = v;
     n_ = v.n;
     cap_ = std::min(std::max(v.hist_cap, 1), kAdjMaxCap);
     S_ = std::max(checkpoint_every, 1);
@@ -1183,7 +1184,7 @@ class AdjEngineT : public AdjointEngine {
   T* alloc(size_t count) {
     void* p = nullptr;
     const size_t b = std::max<size_t>(count, 1) * sizeof(T);
-    if (cudaMalloc(&p, b) != cudaSuccess) {
+    if (view_.alloc(&p, b) != cudaSuccess) {
       ok_ = false;
       return nullptr;
     }
@@ -1274,7 +1275,7 @@ class AdjEngineT : public AdjointEngine {
     const size_t b[6] = {nck * N * sizeof(double4), nck * N * sizeof(R4), nck * N * sizeof(R4), nck * N * sizeof(int),
                          nck * cn * sizeof(int), nck * 9 * cn * sizeof(R)};
     for (int k = 0; k < 6; ++k) {
-      if (cudaMalloc(&p[k], b[k]) != cudaSuccess) {
+      if (view_.alloc(&p[k], b[k]) != cudaSuccess) {
         err = "adjoint: not enough device memory for the checkpoints";
         return GRAINS_GPU_CUDA_ERROR;
       }

@@ -3,6 +3,7 @@
 // adjoint_mixed.cu).
 #pragma once
 
+#include <functional>
 #include <string>
 
 #include <cuda_runtime.h>
@@ -16,6 +17,7 @@ namespace gg {
 // What the adjoint engine reads of a context: set-up tables and the current
 // particle arrays (any order; orig maps a slot to its upload index).
 struct ContextView {
+  std::function<cudaError_t(void**, size_t)> alloc;  // device memory, the context's spare room included
   int precision;
   int device;
   cudaStream_t stream;

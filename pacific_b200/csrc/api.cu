@@ -231,6 +231,38 @@ int cuda_fail(grains_gpu_ctx* c, cudaError_t e, const char* where) {
     if (e_ != cudaSuccess) return cuda_fail(c, e_, #call);       \
   } while (0)
 
+// the step graphs: they hold buffer pointers, counts and options
+void drop_graphs(grains_gpu_ctx* c) {
+  for (cudaGraphExec_t* g : {c->graph, c->res_graph})
+    for (int k = 0; k < 4; ++k)
+      if (g[k]) {
+        cudaGraphExecDestroy(g[k]);
+        g[k] = nullptr;
+      }
+}
+
+// The buffer of the resident lists is the one allocation a context can do without:
+// where another one finds no room it is given back, and the steps are launched
+// until an upload or a change of the tuning finds room for it again.
+bool give_lists_back(grains_gpu_ctx* c) {
+  if (!c->res_buf) return false;
+  cudaGetLastError();
+  cudaStreamSynchronize(c->stream);
+  drop_graphs(c);
+  cudaFree(c->res_buf);
+  c->res_buf = nullptr;
+  c->res_bytes = 0;
+  c->res_ok = false;
+  return true;
+}
+
+cudaError_t device_alloc(grains_gpu_ctx* c, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation && give_lists_back(c)) e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) cudaGetLastError();  // the caller reports it; no later launch does
+  return e;
+}
+
 // ---- shapes ------------------------------------------------------------------
 // Tetrahedron (0, a, b, c) volume and second moments (F. Tonon, "Explicit exact
 // formulas for the 3-D tetrahedron inertia tensor in terms of its vertex
@@ -661,24 +693,30 @@ StepArgs<R> make_args(grains_gpu_ctx* c) {
 // pipeline's.
 constexpr size_t kResAlign = 256;
 constexpr int kResObsHost = 8;  // obstacles per system the state word holds
-size_t res_layout(int64_t cap, int obs_stride, int hist_cap, int list_cap, size_t n_sys, size_t rsize, size_t off[12]) {
+size_t res_pair_cap(const grains_gpu_ctx* c) {
+  const int64_t ent = std::min<int64_t>(c->cap * (int64_t)c->clist_cap, 1ll << 30);
+  return (size_t)std::min<int64_t>(ent / 2, c->cap * (int64_t)c->hist_cap);
+}
+
+// offsets of the arrays; the pair constants only where the pair kernel reads them
+size_t res_layout(const grains_gpu_ctx* c, int obs_stride, size_t off[12]) {
   size_t at = 0;
   auto put = [&](int k, size_t bytes) {
     off[k] = at;
     at += (bytes + kResAlign - 1) / kResAlign * kResAlign;
   };
-  const size_t n = (size_t)cap, m = n * (size_t)std::max(1, obs_stride);
+  const size_t n = (size_t)c->cap, m = n * (size_t)std::max(1, obs_stride), rsize = c->rsize, pairs = res_pair_cap(c);
   put(0, 16 * sizeof(int) + 2 * sizeof(unsigned) + 4 * sizeof(double) + 4096 * sizeof(int));  // control, barrier, skin, candidates, totals, sums
   put(1, n * sizeof(double4));
   put(2, n * sizeof(int2));
-  put(3, n * (size_t)list_cap * sizeof(int));
+  put(3, n * (size_t)c->clist_cap * sizeof(int));
   put(4, n * sizeof(unsigned long long));
   put(5, m * 8 * rsize);
   put(6, m * 9 * rsize);
   put(7, 2 * m * sizeof(int));
-  put(8, n * (size_t)hist_cap);
-  put(9, n_sys * sizeof(double));
-  put(10, n * (size_t)hist_cap * sizeof(ResConst));
+  put(8, pairs);
+  put(9, c->sys.size() * sizeof(double));
+  put(10, c->hooke_memory_pairs ? pairs * sizeof(ResConst) : 0);
   put(11, 2 * n);
   return at;
 }
@@ -694,7 +732,7 @@ ResArgs<R> make_res(grains_gpu_ctx* c) {
   ResArgs<R> r{};
   size_t off[12];
   const int stride = res_obs_stride(c);
-  res_layout(c->cap, stride, c->hist_cap, c->clist_cap, c->sys.size(), c->rsize, off);
+  res_layout(c, stride, off);
   char* b = c->res_buf;
   r.ctl = (int*)(b + off[0]);
   r.bar = (unsigned*)(r.ctl + 16);
@@ -725,9 +763,8 @@ ResArgs<R> make_res(grains_gpu_ctx* c) {
   r.mem = (R*)c->hist[1 - c->hcur];
   r.konst = c->hooke_memory_pairs ? (ResConst*)(b + off[10]) : nullptr;
   // capacities from the buffers' sizes
-  const int64_t ent = std::min<int64_t>(c->cap * (int64_t)c->clist_cap, 1ll << 30);
-  r.ent_cap = (int)ent;
-  r.pair_cap = (int)std::min<int64_t>(ent / 2, c->cap * (int64_t)c->hist_cap);
+  r.ent_cap = (int)std::min<int64_t>(c->cap * (int64_t)c->clist_cap, 1ll << 30);
+  r.pair_cap = (int)res_pair_cap(c);
   r.count[0] = c->cell_count;
   r.count[1] = c->cell_count2[0];
   r.count[2] = c->cell_count2[1];
@@ -905,11 +942,9 @@ int ensure_resident(grains_gpu_ctx* c) {
   c->res_ok = res_scene(c);
   if (!c->res_ok) return 0;
   size_t off[12];
-  const size_t need = res_layout(c->cap, res_obs_stride(c), c->hist_cap, c->clist_cap, c->sys.size(), c->rsize, off);
+  const size_t need = res_layout(c, res_obs_stride(c), off);
   if (need > c->res_bytes) {
-    if (c->res_buf) cudaFree(c->res_buf);
-    c->res_buf = nullptr;
-    c->res_bytes = 0;
+    give_lists_back(c);
     void* q = nullptr;
     const cudaError_t e = cudaMalloc(&q, need);
     if (e == cudaErrorMemoryAllocation) {  // no room for the lists: the launched pipeline needs none
@@ -920,6 +955,7 @@ int ensure_resident(grains_gpu_ctx* c) {
     CK(e);
     c->res_buf = (char*)q;
     c->res_bytes = need;
+    c->res_ok = true;
   }
   CK(cudaMemcpyAsync(c->res_buf + off[9], c->sys_r_max.data(), c->sys_r_max.size() * sizeof(double),
                      cudaMemcpyHostToDevice, c->stream));
@@ -1043,14 +1079,14 @@ int resident_steps(grains_gpu_ctx* c, int n, double dt) {
 int persistent_middle_steps(grains_gpu_ctx* c, int n, double dt) {
   if (!c->pbar) {
     void* q = nullptr;
-    CK(cudaMalloc(&q, 2 * sizeof(unsigned)));
+    CK(device_alloc(c, &q, 2 * sizeof(unsigned)));
     c->pbar = (unsigned*)q;
   }
   if (!c->pblocks) {
     c->pblocks = with_args(c, [&](auto& a) { return persistent_blocks(a); });
     if (c->pblocks <= 0) return fail(c, GRAINS_GPU_CUDA_ERROR, "persistent launch: occupancy query failed");
     void* q = nullptr;
-    CK(cudaMalloc(&q, (size_t)c->pblocks * sizeof(int)));
+    CK(device_alloc(c, &q, (size_t)c->pblocks * sizeof(int)));
     c->psums = (int*)q;
   }
   CK(cudaMemsetAsync(c->pbar, 0, 2 * sizeof(unsigned), c->stream));
@@ -1082,16 +1118,6 @@ int last_step(grains_gpu_ctx* c, double dt) {
   return 0;
 }
 
-// the step graphs: they hold buffer pointers, counts and options
-void drop_graphs(grains_gpu_ctx* c) {
-  for (cudaGraphExec_t* g : {c->graph, c->res_graph})
-    for (int k = 0; k < 4; ++k)
-      if (g[k]) {
-        cudaGraphExecDestroy(g[k]);
-        g[k] = nullptr;
-      }
-}
-
 // Contact-list scratch for cap_per entries per particle: the lists, the
 // result of each entry (two R4) and the work items; grown, never shrunk.
 int ensure_lists(grains_gpu_ctx* c, int cap_per) {
@@ -1107,17 +1133,17 @@ int ensure_lists(grains_gpu_ctx* c, int cap_per) {
     c->obs_force_valid = false;  // the new lists hold no force evaluation yet
     const size_t r4 = 4 * c->rsize;
     void* q = nullptr;
-    CK(cudaMalloc(&q, (size_t)need * sizeof(int)));
+    CK(device_alloc(c, &q, (size_t)need * sizeof(int)));
     c->clist = (int*)q;
-    CK(cudaMalloc(&q, 2 * (size_t)need * r4));
+    CK(device_alloc(c, &q, 2 * (size_t)need * r4));
     c->res_f = q;
     c->res_t = (char*)q + (size_t)need * r4;
-    CK(cudaMalloc(&q, (size_t)need * sizeof(int4)));
+    CK(device_alloc(c, &q, (size_t)need * sizeof(int4)));
     c->work = (int4*)q;
     if (c->has_convex) {  // one narrowphase result per possible work item, their order
-      CK(cudaMalloc(&q, (size_t)need * sizeof(GjkOut)));
+      CK(device_alloc(c, &q, (size_t)need * sizeof(GjkOut)));
       c->gjk_out = (GjkOut*)q;
-      CK(cudaMalloc(&q, (size_t)need * sizeof(int)));
+      CK(device_alloc(c, &q, (size_t)need * sizeof(int)));
       c->gjk_order = (int*)q;
     }
     c->clist_alloc = need;
@@ -1218,6 +1244,7 @@ int grains_gpu_create(const grains_gpu_config* cfg, grains_gpu_ctx** out) {
     ok = c->coord && c->perm && c->stats && c->pairs && c->pairs_n && c->pair_force && c->pair_sys && c->clock &&
          c->work_n && c->gjk_next && c->gjk_bins;
   }
+  c->io.alloc = [c](void** p, size_t bytes) { return device_alloc(c, p, bytes); };
   if (ok) {
     c->pace = dalloc<unsigned>(1, c->pool);
     ok = c->pace;
@@ -1385,9 +1412,12 @@ int grains_gpu_set_collision_options(grains_gpu_ctx* c, double tolerance, int32_
   if (history && !c->gdir[0]) {
     const size_t N = (size_t)c->cap;
     for (int k = 0; k < 2; ++k) {
-      c->gdir[k] = dalloc<GjkDir>(N * c->hist_cap, c->pool);
-      c->gdir_n[k] = dalloc<int>(N, c->pool);
-      if (!c->gdir[k] || !c->gdir_n[k]) return fail(c, GRAINS_GPU_CUDA_ERROR, "collision history allocation failed");
+      void *d = nullptr, *m = nullptr;
+      if (device_alloc(c, &d, N * c->hist_cap * sizeof(GjkDir)) == cudaSuccess) c->pool.push_back(d);
+      if (device_alloc(c, &m, N * sizeof(int)) == cudaSuccess) c->pool.push_back(m);
+      if (!d || !m) return fail(c, GRAINS_GPU_CUDA_ERROR, "collision history allocation failed");
+      c->gdir[k] = (GjkDir*)d;
+      c->gdir_n[k] = (int*)m;
     }
   }
   if (history && !c->gjk_history)  // a history starts empty
@@ -1561,7 +1591,7 @@ int build_tables(grains_gpu_ctx* c) {
   adj_start.push_back((int)adj.size());
   auto up = [&](const void* src, size_t bytes, void** dst) -> int {
     void* p = nullptr;
-    CK(cudaMalloc(&p, bytes ? bytes : 16));
+    CK(device_alloc(c, &p, bytes ? bytes : 16));
     c->table_pool.push_back(p);
     if (bytes) CK(cudaMemcpyAsync(p, src, bytes, cudaMemcpyHostToDevice, c->stream));
     *dst = p;
@@ -1607,21 +1637,21 @@ int build_tables(grains_gpu_ctx* c) {
   if (rc) return rc;
   // cell arrays
   void* p = nullptr;
-  CK(cudaMalloc(&p, (size_t)cells * sizeof(int)));
+  CK(device_alloc(c, &p, (size_t)cells * sizeof(int)));
   c->table_pool.push_back(p);
   c->cell_count = (int*)p;
   for (int k = 0; k < 2; ++k) {
-    CK(cudaMalloc(&p, (size_t)cells * sizeof(int)));
+    CK(device_alloc(c, &p, (size_t)cells * sizeof(int)));
     c->table_pool.push_back(p);
     c->cell_count2[k] = (int*)p;
   }
-  CK(cudaMalloc(&p, ((size_t)cells + 1) * sizeof(int)));
+  CK(device_alloc(c, &p, ((size_t)cells + 1) * sizeof(int)));
   c->table_pool.push_back(p);
   c->cell_start = (int*)p;
-  CK(cudaMalloc(&p, ((size_t)cells + 1) * sizeof(int)));
+  CK(device_alloc(c, &p, ((size_t)cells + 1) * sizeof(int)));
   c->table_pool.push_back(p);
   c->cell_cursor = (int*)p;
-  CK(cudaMalloc(&p, ((size_t)cells / 4096 + 2) * sizeof(int)));
+  CK(device_alloc(c, &p, ((size_t)cells / 4096 + 2) * sizeof(int)));
   c->table_pool.push_back(p);
   c->block_sums = (int*)p;
   CK(cudaMemsetAsync(c->cell_count, 0, (size_t)cells * sizeof(int), c->stream));
@@ -1682,7 +1712,7 @@ int grains_gpu_upload_particles(grains_gpu_ctx* c, const grains_gpu_particles* p
     const int cap_per = c->list_capacity > 0 ? c->list_capacity : (c->has_convex ? 64 : 32);
     if (!c->ccount) {
       void* q = nullptr;
-      CK(cudaMalloc(&q, (size_t)c->cap * sizeof(int)));
+      CK(device_alloc(c, &q, (size_t)c->cap * sizeof(int)));
       c->ccount = (int*)q;
     }
     if (int rc = ensure_lists(c, cap_per)) return rc;
@@ -1691,7 +1721,7 @@ int grains_gpu_upload_particles(grains_gpu_ctx* c, const grains_gpu_particles* p
     for (int k = 0; k < 2; ++k)
       if (!c->buf[k].basis) {
         void* q = nullptr;
-        CK(cudaMalloc(&q, (size_t)c->cap * 9 * sizeof(double)));
+        CK(device_alloc(c, &q, (size_t)c->cap * 9 * sizeof(double)));
         c->buf[k].basis = (double*)q;
       }
   }
@@ -1795,15 +1825,15 @@ int grains_gpu_upload_particles(grains_gpu_ctx* c, const grains_gpu_particles* p
   // tables of the reload and RawData writers
   if (!c->d_row_id) {
     void* q0 = nullptr;
-    CK(cudaMalloc(&q0, (size_t)c->cap * sizeof(int)));
+    CK(device_alloc(c, &q0, (size_t)c->cap * sizeof(int)));
     c->d_row_id = (int*)q0;
-    CK(cudaMalloc(&q0, (size_t)c->cap * sizeof(int)));
+    CK(device_alloc(c, &q0, (size_t)c->cap * sizeof(int)));
     c->d_row_sys = (int*)q0;
-    CK(cudaMalloc(&q0, (size_t)c->cap * sizeof(unsigned long long)));
+    CK(device_alloc(c, &q0, (size_t)c->cap * sizeof(unsigned long long)));
     c->d_row_keys = (unsigned long long*)q0;
-    CK(cudaMalloc(&q0, (size_t)c->cap * sizeof(int)));
+    CK(device_alloc(c, &q0, (size_t)c->cap * sizeof(int)));
     c->d_key_rows = (int*)q0;
-    CK(cudaMalloc(&q0, (size_t)c->cap * sizeof(RecordAttr)));
+    CK(device_alloc(c, &q0, (size_t)c->cap * sizeof(RecordAttr)));
     c->d_attr = (RecordAttr*)q0;
   }
   {
@@ -1874,7 +1904,7 @@ namespace {
 int ensure_stage(grains_gpu_ctx* c) {
   if (c->stage) return 0;
   void* q = nullptr;
-  CK(cudaMalloc(&q, (size_t)c->cap * 30 * sizeof(double)));
+  CK(device_alloc(c, &q, (size_t)c->cap * 30 * sizeof(double)));
   c->stage = (char*)q;
   return 0;
 }
@@ -1966,7 +1996,7 @@ int grains_gpu_update_particle_rows(grains_gpu_ctx* c, int64_t n_rows, const int
   if (int rc = ensure_stage(c)) return rc;
   if (!c->row_scratch) {  // the rows and the slot of every upload index
     void* q = nullptr;
-    CK(cudaMalloc(&q, (size_t)c->cap * (sizeof(long long) + sizeof(int))));
+    CK(device_alloc(c, &q, (size_t)c->cap * (sizeof(long long) + sizeof(int))));
     c->row_scratch = (char*)q;
   }
   if (int rc = flush_kick(c)) return rc;
@@ -2180,7 +2210,7 @@ int grains_gpu_set_hydro_forces(grains_gpu_ctx* c, const double* force, const do
   if (on) {
     if (!c->d_hydro) {
       void* q = nullptr;
-      CK(cudaMalloc(&q, (size_t)c->cap * 6 * sizeof(double)));
+      CK(device_alloc(c, &q, (size_t)c->cap * 6 * sizeof(double)));
       c->d_hydro = (double*)q;
     }
     const int64_t n = c->n;
@@ -2608,9 +2638,9 @@ int grains_gpu_get_candidate_pairs(grains_gpu_ctx* c, int32_t system, int32_t in
   if (!c->cand) {
     void* q = nullptr;
     c->cand_cap = (int)std::min<int64_t>(48 * c->cap + 4096, (int64_t)1 << 30);
-    CK(cudaMalloc(&q, 2 * (size_t)c->cand_cap * sizeof(int)));
+    CK(device_alloc(c, &q, 2 * (size_t)c->cand_cap * sizeof(int)));
     c->cand = (int*)q;
-    CK(cudaMalloc(&q, sizeof(unsigned long long)));
+    CK(device_alloc(c, &q, sizeof(unsigned long long)));
     c->cand_n = (unsigned long long*)q;
   }
   CK(cudaMemsetAsync(c->cand_n, 0, sizeof(unsigned long long), c->stream));
@@ -2985,7 +3015,7 @@ int take_snapshot(grains_gpu_ctx* c, Snapshot& s) {
   s.items = c->items;
   for (auto& f : snapshot_fields(c, c->cur, c->hcur)) {
     void* q = nullptr;
-    if (cudaMalloc(&q, f.second) != cudaSuccess) return GRAINS_GPU_CUDA_ERROR;
+    if (device_alloc(c, &q, f.second) != cudaSuccess) return GRAINS_GPU_CUDA_ERROR;
     s.bufs.push_back({q, f.second});
     if (cudaMemcpyAsync(q, f.first, f.second, cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess)
       return GRAINS_GPU_CUDA_ERROR;
@@ -3138,6 +3168,7 @@ int context_view(grains_gpu_ctx* c, ContextView* v, std::string& err) {
   }
   const int maxmat = c->cfg.max_materials > 0 ? c->cfg.max_materials : 4;
   *v = ContextView{};
+  v->alloc = [c](void** p, size_t bytes) { return device_alloc(c, p, bytes); };
   v->precision = c->precision;
   v->device = c->cfg.device;
   v->stream = c->stream;

@@ -45,7 +45,7 @@ char* IoScratch::work(size_t bytes, size_t keep, cudaStream_t st, std::string& e
   if (bytes > dev_bytes) {
     void* p = nullptr;
     const size_t want = bytes + bytes / 4;
-    if (cudaMalloc(&p, want) != cudaSuccess) {
+    if (alloc(&p, want) != cudaSuccess) {
       err = "device scratch allocation failed";
       return nullptr;
     }
@@ -66,7 +66,7 @@ char* IoScratch::output(size_t bytes, std::string& err) {
     out = nullptr;
     out_bytes = 0;
     const size_t want = bytes + bytes / 4 + 4096;
-    if (cudaMalloc(&out, want) != cudaSuccess) {
+    if (alloc(&out, want) != cudaSuccess) {
       err = "device output allocation failed";
       return nullptr;
     }

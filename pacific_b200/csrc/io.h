@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -61,6 +62,7 @@ struct IoScratch {
   void* pinned[2] = {nullptr, nullptr};
   size_t pinned_bytes = 0;
   cudaEvent_t ev[2] = {nullptr, nullptr};
+  std::function<cudaError_t(void**, size_t)> alloc;  // the context's
   ~IoScratch();
   // at least `bytes` of work space; the first `keep` bytes survive a regrowth
   char* work(size_t bytes, size_t keep, cudaStream_t st, std::string& err);

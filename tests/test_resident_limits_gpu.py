@@ -166,3 +166,111 @@ def test_a_build_whose_waits_run_out(gpu_lib, polls, skip):
         assert np.array_equal(a[key], b[key]), key
     sim.close()
     ref.close()
+
+
+def free_bytes():
+    import torch
+    return torch.cuda.mem_get_info()[0]
+
+
+class Filled:
+    """Device memory taken until about `left` bytes are free"""
+
+    def __init__(self, left):
+        import torch
+        torch.cuda.empty_cache()
+        self.block = torch.empty(max(0, free_bytes() - left), dtype=torch.uint8, device="cuda")
+
+    def release(self):
+        import torch
+        del self.block
+        torch.cuda.empty_cache()
+
+
+def sized(gpu_lib, sc):
+    sim = make(gpu_lib, sc, FP64)
+    sim.set_tuning(list_capacity=28)
+    return sim
+
+
+def run_out(sim, sc):
+    sim.initialize_leapfrog(0.0, sc.dt)
+    sim.step(20, 0.0, sc.dt)
+    sim.synchronize()
+    return sim.download()
+
+
+def large_box():
+    sc = S.small_box(60000, seed=9, velocity_sigma=0.2, spacing=2.03)
+    sc.dt = 2.0e-6
+    return sc
+
+
+def test_without_room_for_the_lists_steps_are_launched(gpu_lib):
+    """Device memory that holds the context but not the lists' buffer: the upload
+    succeeds, the steps are launched, the bits are the same; an upload that finds
+    room brings the lists back."""
+    sc = large_box()
+    free = free_bytes()
+    sim = sized(gpu_lib, sc)
+    assert sim.launches_per_step() == 3
+    with_lists = free - free_bytes()
+    want = run_out(sim, sc)
+    sim.close()
+    free = free_bytes()
+    sim = sized(gpu_lib, S.small_box(60000, seed=9, spacing=2.03, radius_range=(0.2, 1.0)))  # radii apart: no lists
+    assert sim.launches_per_step() > 3
+    lists = with_lists - (free - free_bytes())
+    assert lists > (64 << 20)
+    # room for less than the lists' buffer
+    full = Filled(lists // 2)
+    try:
+        sim.upload(sc.particles)
+        assert sim.launches_per_step() > 3
+        got = run_out(sim, sc)
+    finally:
+        full.release()
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k
+    sim.upload(sc.particles)
+    assert sim.launches_per_step() == 3
+    got = run_out(sim, sc)
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k
+    sim.close()
+
+
+def test_lists_give_their_room_to_other_allocations(gpu_lib):
+    """An adjoint that fits only in the room of the resident lists: it gets it,
+    and the context runs on without the lists, the same bits."""
+    from pacific_b200.abi import Adjoint
+    sc = large_box()
+    sim = sized(gpu_lib, sc)
+    want = run_out(sim, sc)
+    sim.upload(sc.particles)
+    none = np.zeros((sc.n, 3))
+
+    def gradient():
+        adj = Adjoint(sim, checkpoint_every=2)
+        out = adj.forward(2, sc.dt)
+        adj.backward(none, none, none)
+        need = free - free_bytes()
+        adj.close()
+        return out, need
+    free = 0
+    gradient()  # the first one loads its kernels
+    free = free_bytes()
+    final, need = gradient()
+    assert sim.launches_per_step() == 3 and need > (128 << 20)
+    full = Filled(need - (24 << 20))
+    try:
+        again, _ = gradient()
+        assert sim.launches_per_step() > 3
+        got = run_out(sim, sc)
+    finally:
+        full.release()
+    for k in final:
+        assert np.array_equal(final[k], again[k]), k
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k
+    sim.close()
