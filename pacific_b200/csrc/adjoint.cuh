@@ -1270,6 +1270,8 @@ class AdjEngineT : public AdjointEngine {
     if (n_seg_ <= ck_count_) return 0;
     for (void* p : ck_pool_) cudaFree(p);
     ck_pool_.clear();
+    ck_count_ = 0;
+    have_forward_ = false;  // its checkpoints are gone
     const size_t N = (size_t)n_, cn = (size_t)cap_ * n_, nck = (size_t)n_seg_;
     void* p[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     const size_t b[6] = {nck * N * sizeof(double4), nck * N * sizeof(R4), nck * N * sizeof(R4), nck * N * sizeof(int),

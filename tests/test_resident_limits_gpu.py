@@ -274,3 +274,27 @@ def test_lists_give_their_room_to_other_allocations(gpu_lib):
     for k in want:
         assert np.array_equal(got[k], want[k]), k
     sim.close()
+
+
+def test_an_adjoint_whose_checkpoints_do_not_fit(gpu_lib):
+    """A run too long for the device memory fails; a shorter one after it works as
+    before, and no backward run uses what the failed one gave back."""
+    from pacific_b200.abi import Adjoint
+    sc = S.small_box(1000, seed=4, velocity_sigma=0.1)
+    sim = make(gpu_lib, sc, FP64)
+    adj = Adjoint(sim, checkpoint_every=1)
+    one = np.ones((sc.n, 3))
+
+    def both():
+        return adj.forward(6, 1.0e-6), adj.backward(one, one, one)
+    first = both()
+    with pytest.raises(GrainsError):
+        adj.forward(10_000_000, 1.0e-6)
+    with pytest.raises(GrainsError):
+        adj.backward(one, one, one)
+    second = both()
+    for a, b in zip(first, second):
+        for k in a:
+            assert np.array_equal(a[k], b[k]), k
+    adj.close()
+    sim.close()
