@@ -692,7 +692,6 @@ StepArgs<R> make_args(grains_gpu_ctx* c) {
 // rest in res_buf.  So the lists hold as many entries in all as the launched
 // pipeline's.
 constexpr size_t kResAlign = 256;
-constexpr int kResObsHost = 8;  // obstacles per system the state word holds
 size_t res_pair_cap(const grains_gpu_ctx* c) {
   const int64_t ent = std::min<int64_t>(c->cap * (int64_t)c->clist_cap, 1ll << 30);
   return (size_t)std::min<int64_t>(ent / 2, c->cap * (int64_t)c->hist_cap);
@@ -930,7 +929,7 @@ bool res_scene(const grains_gpu_ctx* c) {
   if (!(c->r_min > 0) || c->r_max > 4. * c->r_min) return false;
   for (size_t k = 0; k < c->sys.size(); ++k) {
     const SysHost& s = c->sys[k];
-    if (s.obs.size() > (size_t)kResObsHost) return false;
+    if (s.obs.size() > (size_t)kResObsMax) return false;
     if (2. * c->sys_r_max[k] > std::min(s.ex, std::min(s.ey, s.ez))) return false;
   }
   return true;

@@ -253,6 +253,7 @@ struct StepArgs {
 // spheres among static obstacles.  Lists, results and pair memories use the
 // buffers of the launched pipeline's lists and of the memory rows it is not
 // reading.
+constexpr int kResObsMax = 8;  // obstacles per system (a byte each in a particle's state word)
 template <typename R>
 struct ResResult;
 // of a listed pair, when the context's only law is HookeMemory without rolling:

@@ -108,8 +108,7 @@ __device__ __forceinline__ V3<R> rk3(bool sphere, V3<R> I, V3<R> Tbf, V3<R> wbf,
 template <typename R>
 __device__ __forceinline__ void integrate(const StepArgs<R>& a, const ParticleArrays<R>& src,
                                           const ParticleArrays<R>& dst, int s, V3<R> F, V3<R> T, int do_kick2,
-                                          R dt_kick2, int do_move, R dt_v, double dt_x, D3* x_out = nullptr,
-                                          unsigned* key_out = nullptr) {
+                                          R dt_kick2, int do_move, R dt_v, double dt_x) {
   double4 xr = src.xr[s];
   const double4 qd = src.q[s];
   const int4 meta = src.meta[s];
@@ -161,8 +160,6 @@ __device__ __forceinline__ void integrate(const StepArgs<R>& a, const ParticleAr
     unsigned key = (unsigned)cell_index(S, ci, cj, ck);
     dst.key[s] = key;
     atomicAdd(&a.cell_count[key], 1);  // result unused: a fire-and-forget reduction
-    if (x_out) *x_out = d3(xr.x, xr.y, xr.z);
-    if (key_out) *key_out = key;
   } else if (a.has_basis && dst.basis != src.basis) {
     for (int t = 0; t < 9; ++t) dst.basis[9 * (size_t)s + t] = src.basis[9 * (size_t)s + t];
   }

@@ -39,7 +39,6 @@ enum {
 // even and odd parity; kResCountAll: the step's candidate pairs are counted over
 // all cells, not from the step before
 
-constexpr int kResObsMax = 8;   // obstacles per system (a byte each in a particle's state word)
 // the state of a listed pair or of a particle's obstacle
 enum { kResContact = 1, kResMemory = 2, kResCandidate = 4 };
 
