@@ -7,7 +7,8 @@ import numpy as np
 import pytest
 
 from pacific_b200 import scenarios as S
-from pacific_b200.abi import FP64, HERTZ_MEMORY, HOOKE, HOOKE_MEMORY, MIXED
+from pacific_b200.abi import (CONTACT_ERROR, CONTACT_HANDLED, FP64, HERTZ, HERTZ_MEMORY, HISTORY_FULL, HOOKE,
+                              HOOKE_MEMORY, MIXED, MOTION_ERROR, OUT_OF_GRID, GrainsError)
 
 from helpers import make
 
@@ -195,3 +196,134 @@ def test_profiled_steps_are_those_of_a_step_call(gpu_lib, steps):
     for k in out[0][0]:
         assert np.array_equal(out[0][0][k], out[1][0][k]), k
     assert out[0][1]["n_candidate_pairs"] == out[1][1]["n_candidate_pairs"]
+
+
+def outcome(lib, sc, precision, capacity, resident, steps=40, setup=None, history=0):
+    """Status of a run and what it leaves, errors included"""
+    sim = make(lib, sc, precision, history_capacity=history)
+    sim.set_tuning(list_capacity=capacity)
+    assert (sim.launches_per_step() == 3) == resident
+    if setup:
+        setup(sim)
+    codes = []
+    for call in (lambda: sim.initialize_leapfrog(0.0, sc.dt), lambda: sim.step(steps, 0.0, sc.dt), sim.synchronize):
+        try:
+            call()
+            codes.append(0)
+        except GrainsError as e:
+            codes.append(e.code)
+    st = sim.stats()
+    sim.reset_stats()
+    d, m = sim.download(), sim.contact_memory()
+    order = np.lexsort((m["other"], m["owner"], m["system"]))
+    sim.close()
+    return codes, st, {**d, **{"memory " + k: v[order] for k, v in m.items()}}
+
+
+def same_outcome(lib, sc, precision, capacities=(32, 20), **kw):
+    a, b = (outcome(lib, sc, precision, c, c == capacities[0], **kw) for c in capacities)
+    assert a[0] == b[0]
+    for k in a[1]:
+        if k not in ("overlap_sum", "overlap_mean"):  # summed by atomics, in any order
+            assert a[1][k] == b[1][k], k
+    for k in a[2]:
+        assert np.array_equal(a[2][k], b[2][k], equal_nan=True), k
+    return a
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED])
+@pytest.mark.parametrize("corrected", [False, True])
+def test_immersed_spheres(gpu_lib, corrected, precision):
+    """Buoyancy, the fluid's forces and torques, with and without the correction
+    of the accelerations."""
+    sc = S.small_box(300, seed=8, velocity_sigma=0.3, radius_range=(0.9, 1.1), spacing=2.25)
+    sc.dt = 5.0e-6
+    rng = np.random.default_rng(8)
+    force, torque = rng.normal(0.0, 1.0e-4, (300, 3)), rng.normal(0.0, 1.0e-7, (300, 3))
+
+    def setup(sim):
+        sim.set_fluid(1000.0, corrected, np.full(300, 2500.0))
+        sim.set_hydro_forces(force, torque)
+    codes, st, _ = same_outcome(gpu_lib, sc, precision, setup=setup)
+    assert codes == [0, 0, 0] and st["n_contacts"] > 0
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED])
+def test_hertz_without_memory(gpu_lib, precision):
+    sc = S.small_box(300, seed=9, velocity_sigma=0.3, radius_range=(0.95, 1.05), spacing=2.07)
+    sc.laws = [[(a, b, HERTZ, [2.0e8, 0.9, 0.5, 1.0e-3, 6.0e7]) for a, b, _, _ in sc.laws[0]]]
+    sc.dt = 2.0e-6
+    codes, st, d = same_outcome(gpu_lib, sc, precision)
+    assert codes == [0, 0, 0] and st["n_contacts"] > 0 and len(d["memory owner"]) == 0
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED])
+def test_materials_without_a_law(gpu_lib, precision):
+    """Pairs of materials that have no law between them meet too; the lists keep
+    no pair constants then."""
+    sc = S.small_box(300, seed=10, velocity_sigma=0.3, radius_range=(0.95, 1.05), spacing=2.0)
+    sc.dt = 2.0e-6
+    sc.particles["material"] = (np.arange(300) % 2 * 2).astype(np.int32)  # 0 and 2
+    law = sc.laws[0][0][2:]
+    sc.laws = [sc.laws[0] + [(2, 2, *law), (1, 2, *law)]]
+    codes, st, d = same_outcome(gpu_lib, sc, precision)
+    assert codes == [0, 0, 0] and len(d["memory owner"]) > 0
+
+
+def one_fast(sc, k, velocity, position=None):
+    sc.particles["velocity"][k] = velocity
+    if position is not None:
+        sc.particles["position"][k] = position
+    return sc
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED])
+@pytest.mark.parametrize("what", ["motion", "grid", "handled", "contact"])
+def test_errors_of_a_run(gpu_lib, what, precision):
+    """A displacement beyond the crust, a sphere that leaves the grid, overlaps
+    beyond the crusts that the retry with ten crusts handles or not: the status
+    and the state of the launched pipeline."""
+    sc = S.small_box(125, seed=11, velocity_sigma=0.05, radius_range=(0.95, 1.05), spacing=2.2)
+    sc.dt = 2.0e-6
+    if what == "motion":
+        sc.particles["crust"][:] = 1.0e-6
+        one_fast(sc, 7, [0.0, 0.0, 0.9])
+    elif what == "grid":
+        sc.obstacles = [[]]
+        one_fast(sc, 0, [-0.5, 0.0, 0.0], [20.0e-6, 4.0e-3, 15.0e-3])
+    else:
+        crust = 2.0e-5 if what == "handled" else 2.0e-6
+        sc.particles["crust"][:] = crust
+        for o in sc.obstacles[0]:
+            o["crust"] = crust
+        x = sc.particles["position"]
+        x[1] = x[0] + [sc.particles["radius"][0] + sc.particles["radius"][1] - 1.0e-4, 0.0, 0.0]
+    # (the handled pair flies apart: a few steps before it meets the next spheres)
+    codes, st, _ = same_outcome(gpu_lib, sc, precision, steps=9 if what == "handled" else 40)
+    bit = {"motion": MOTION_ERROR, "grid": OUT_OF_GRID, "handled": CONTACT_HANDLED, "contact": CONTACT_ERROR}[what]
+    assert st["status"] & bit
+    if what == "handled":
+        assert codes == [0, 0, 0] and st["status"] == bit
+    else:
+        assert codes[2] & bit
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED])
+def test_more_contacts_than_memory_slots(gpu_lib, precision):
+    """The sphere of the lowest id owns its 18 contacts, and a row holds 12
+    memories: both pipelines say so."""
+    side, r, a = 7, 0.7e-3, 0.975e-3  # neighbours at a and sqrt(2) a touch, at sqrt(3) a do not
+    n = side ** 3
+    sc = S.small_box(n, seed=1)
+    k = np.arange(n)
+    x = a * np.stack([k % side, k // side % side, k // side ** 2], 1) + 3.0e-3
+    sc.particles = S._spheres(n, np.full(n, r), 2500.0, x, np.zeros((n, 3)), 0.5e-3)
+    ids = np.arange(1, n + 1, dtype=np.int32)
+    ids[n // 2] = 0
+    sc.particles["id"] = ids
+    sc.laws = [[(p, q, HOOKE_MEMORY, [1.0e2, 0.9, -1.0, 0.5, 0.8e2, 0.0, 0.0, 0.0]) for p, q, _, _ in sc.laws[0]]]
+    sc.obstacles, sc.dt = [[]], 1.0e-8
+    for capacity in (24, 20):
+        codes, st, d = outcome(gpu_lib, sc, precision, capacity, capacity == 24, history=12)
+        assert d["coordination"].max() == 18
+        assert codes[0] == codes[2] == st["status"] == HISTORY_FULL
