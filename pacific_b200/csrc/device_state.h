@@ -246,7 +246,7 @@ struct StepArgs {
   int barrier_skip_block;   // persistent kernel: a block that leaves at once (a test of the bounded wait), or -1
   int contacts_block;    // threads per block of contacts_kernel (<= 256)
   int forces_block;      // threads per block of forces_kernel (<= 128)
-  unsigned* pace;        // bits of the largest squared speed that gathers have met, or null
+  unsigned* pace;        // bits of the largest squared speed that gathers have met, the sign bit set (0: none), or null
 };
 
 // Resident pair lists (resident.cuh): the state of a run of middle steps of

@@ -412,8 +412,8 @@ __global__ void __launch_bounds__(256) gather_kernel(StepArgs<R> a, int gather_f
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) fast = fmaxf(fast, __shfl_xor_sync(0xffffffffu, fast, o));
   // few warps exceed what others have found: no queue of atomics
-  if ((threadIdx.x & 31) == 0 && __float_as_uint(fast) > *(volatile unsigned*)a.pace)
-    atomicMax(a.pace, __float_as_uint(fast));
+  const unsigned word = __float_as_uint(fast) | 0x80000000u;
+  if ((threadIdx.x & 31) == 0 && word > *(volatile unsigned*)a.pace) atomicMax(a.pace, word);
 }
 
 // ---------------------------------------------------------------------------
@@ -1870,8 +1870,8 @@ template <typename R, bool KICK = false>
 __global__ void __launch_bounds__(256) sums_kernel(StepArgs<R> a, R dt_half, double dt) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s == 0) {
-    if (!KICK && a.pace) {
-      a.stats->speed = *a.pace | 0x80000000u;
+    if (!KICK && a.pace && *a.pace) {  // a permutation since the last time
+      a.stats->speed = *a.pace;
       a.stats->items = (unsigned)*a.work_n;
       *a.pace = 0;
     }

@@ -327,3 +327,27 @@ def test_more_contacts_than_memory_slots(gpu_lib, precision):
         codes, st, d = outcome(gpu_lib, sc, precision, capacity, capacity == 24, history=12)
         assert d["coordination"].max() == 18
         assert codes[0] == codes[2] == st["status"] == HISTORY_FULL
+
+
+@pytest.mark.parametrize("share", [0.04, 0.06])
+def test_the_speed_outlives_force_evaluations_and_rest(gpu_lib, share):
+    """Force evaluations that do not permute the particles leave the speed that
+    the choice of the pipeline goes by; particles put to rest are slow."""
+    sc = moving_lattice(1000, share, False)
+    sim = make(gpu_lib, sc, MIXED)
+
+    def resident():
+        t, phases = sim.profile_kernels(8, 0.0, sc.dt)
+        return phases["contacts"][1] == 1
+    sim.initialize_leapfrog(0.0, sc.dt)
+    for _ in range(3):
+        sim.compute_forces(0.0, sc.dt)
+    assert resident() == (share < 0.05)
+    sim.compute_forces(0.0, sc.dt)
+    sim.reset_stats()
+    sim.synchronize()
+    assert resident() == (share < 0.05)
+    sim.update({**sc.particles, "velocity": 0.0 * sc.particles["velocity"]})
+    sim.initialize_leapfrog(0.0, sc.dt)
+    assert resident()
+    sim.close()

@@ -298,3 +298,35 @@ def test_an_adjoint_whose_checkpoints_do_not_fit(gpu_lib):
             assert np.array_equal(a[k], b[k]), k
     adj.close()
     sim.close()
+
+
+def test_contexts_of_several_threads(gpu_lib):
+    """Four contexts step at the same time, each in a thread and on a stream of
+    its own, with lists rebuilt every few steps by launches that fill the chip: the
+    bits of each context alone, and no wait that runs out."""
+    import threading
+    sc = S.small_box(60000, seed=12, velocity_sigma=2.0, spacing=2.2)
+    sc.dt = 2.0e-6
+    sims = [make(gpu_lib, sc, MIXED) for _ in range(5)]
+
+    def run(sim):
+        sim.initialize_leapfrog(0.0, sc.dt)
+        t = 0.0
+        for _ in range(5):
+            t = sim.step(60, t, sc.dt)
+        sim.synchronize()
+        out.append(sim.download())
+    out = []
+    run(sims[0])
+    threads = [threading.Thread(target=run, args=(sim,)) for sim in sims[1:]]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert len(out) == 5 and sims[0].launches_per_step() == 3
+    for d in out[1:]:
+        for k in d:
+            assert np.array_equal(d[k], out[0][k]), k
+    for sim in sims:
+        assert sim.stats()["status"] == 0
+        sim.close()
