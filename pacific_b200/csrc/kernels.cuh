@@ -369,20 +369,22 @@ __global__ void __launch_bounds__(kCellSortThreads) cell_sort_kernel(StepArgs<R>
 }
 
 // permutes every per-particle array into cell order; the permutation then
-// becomes the identity (each thread resets its own entry after reading it)
+// becomes the identity (each thread resets its own entry after reading it).
+// Returns the particle's velocity.
 template <typename R>
-__device__ __forceinline__ void gather_one(const StepArgs<R>& a, int t, int gather_forces) {
+__device__ __forceinline__ V3<R> gather_one(const StepArgs<R>& a, int t, int gather_forces) {
   int s = a.perm[t];
   if (s < 0 || s >= a.n) {
     set_status(a.stats, GRAINS_GPU_CUDA_ERROR);
-    return;
+    return v3<R>(R(0), R(0), R(0));
   }
   a.perm[t] = t;
   const ParticleArrays<R>& C = a.cur;
   const ParticleArrays<R>& D = a.alt;
   D.xr[t] = C.xr[s];
   D.q[t] = C.q[s];
-  D.v[t] = C.v[s];
+  const auto v = C.v[s];
+  D.v[t] = v;
   D.w[t] = C.w[s];
   D.wbf[t] = C.wbf[s];
   D.inertia[t] = C.inertia[s];
@@ -397,23 +399,22 @@ __device__ __forceinline__ void gather_one(const StepArgs<R>& a, int t, int gath
   if (a.has_basis) {
     for (int k = 0; k < 9; ++k) D.basis[9 * (size_t)t + k] = C.basis[9 * (size_t)s + k];
   }
+  return ld3<R>(v);
 }
 
 template <typename R>
 __global__ void __launch_bounds__(256) gather_kernel(StepArgs<R> a, int gather_forces) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < a.n) gather_one(a, t, gather_forces);
-  if (!a.pace) return;
-  float fast = 0.f;
+  const unsigned seen = a.pace ? *(volatile unsigned*)a.pace : 0xffffffffu;
+  unsigned word = 0;
   if (t < a.n) {
-    const float v2 = (float)norm2(ld3<R>(a.alt.v[t]));
-    fast = v2 <= 3.e38f ? v2 : INFINITY;
+    const float v2 = (float)norm2(gather_one(a, t, gather_forces));
+    word = __float_as_uint(v2 <= 3.e38f ? v2 : INFINITY) | 0x80000000u;
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) fast = fmaxf(fast, __shfl_xor_sync(0xffffffffu, fast, o));
   // few warps exceed what others have found: no queue of atomics
-  const unsigned word = __float_as_uint(fast) | 0x80000000u;
-  if ((threadIdx.x & 31) == 0 && word > *(volatile unsigned*)a.pace) atomicMax(a.pace, word);
+  if (!__any_sync(0xffffffffu, word > seen)) return;
+  word = __reduce_max_sync(0xffffffffu, word);
+  if ((threadIdx.x & 31) == 0) atomicMax(a.pace, word);
 }
 
 // ---------------------------------------------------------------------------
@@ -1690,9 +1691,10 @@ __global__ void __launch_bounds__(256) gjk_place_kernel(StepArgs<R> a) {
 // run has ended wait until GG_GJK_BATCH lanes of the warp are idle (by default
 // the whole warp) and start their next runs together.
 // What bounds it: the instructions of an iteration, issued in order by few
-// warps (FP64 pipe 11 % busy, DRAM idle).  So the sub-algorithm is written out
-// with predicates (gjk_closest: 55 M instead of 85 M warp instructions for
-// 70,600 runs, 14.5 instead of 9.9 lanes active), the simplex stays in
+// warps (FP64 pipe 20 % busy, DRAM idle; 141,000 runs take 80 M warp instructions
+// with 19 of 32 lanes active, 36,800 signed-volume runs 40 M with 11).  So the sub-algorithm is written out
+// with predicates (gjk_closest: by itself 55 M instead of 85 M warp instructions
+// for 70,600 runs, 14.5 instead of 9.9 lanes), the simplex stays in
 // registers (255, 8 warps per SM), the bodies and support points, 54 numbers a
 // thread, in shared memory, and the rare retry of a ContactError runs after the
 // loop: called inside it, its spills took 5 of 6 issue slots.  141,000 runs of
@@ -1869,18 +1871,21 @@ __device__ __forceinline__ void sum_one(const StepArgs<R>& a, int s, V3<R>* f_ou
 template <typename R, bool KICK = false>
 __global__ void __launch_bounds__(256) sums_kernel(StepArgs<R> a, R dt_half, double dt) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s == 0) {
-    if (!KICK && a.pace && *a.pace) {  // a permutation since the last time
-      a.stats->speed = *a.pace;
-      a.stats->items = (unsigned)*a.work_n;
+  const bool first = s == 0, read_pace = !KICK && first && a.pace;
+  const unsigned pace = read_pace ? *a.pace : 0u;
+  const int items = read_pace ? *a.work_n : 0;
+  if (s >= a.n) return;
+  V3<R> F, T;
+  sum_one(a, s, &F, &T);
+  if (first) {
+    if (pace) {  // a permutation since the last time
+      a.stats->speed = pace;
+      a.stats->items = (unsigned)items;
       *a.pace = 0;
     }
     *a.work_n = 0;
     if (a.gjk_next) *a.gjk_next = 0;
   }
-  if (s >= a.n) return;
-  V3<R> F, T;
-  sum_one(a, s, &F, &T);
   if (KICK) integrate(a, a.cur, a.cur, s, F, T, 1, dt_half, 1, dt_half, dt);
 }
 

@@ -759,7 +759,7 @@ __device__ __forceinline__ void res_count_candidates(const StepArgs<R>& a, const
 // barrier.  64 at a time keeps twice the loads in flight; 32 spreads a short list
 // over more warps.  Then obs_blocks: the obstacle candidates; the other blocks:
 // res_count_candidates.
-// Bound by the latency of the gathers and by L2 (about 450 B a contact); four
+// Bound by the latency of the gathers and by L2 (390 B a contact); four
 // blocks a SM at 128 registers (five at 96 spill: 67.2 against 66.5 us).  200,000
 // spheres, 460,000 contacts: 82 -> 66 us mixed, 103 -> 82 us FP64 with the pair
 // constants and without the block-wide barriers of the first form.
