@@ -44,10 +44,17 @@ sys.path.insert(0, ROOT)
 # the list entries of the force evaluation; R4 = 16 B in mixed precision, 32 B
 # in FP64; a contact-memory entry is 44 B / 80 B; a pair's two list entries and
 # its work item count once per particle on average):
-# The formulas are those of the launched pipeline (moving obstacles, convex
-# bodies).  Steps on resident pair lists (spheres) do the same work in
-# res_pairs_kernel and res_sums_kernel; their list walk runs only where a list is
-# rebuilt, so that phase has no fixed bytes there.
+# Steps on resident pair lists (spheres) have kernels of their own, the others
+# those of the launched pipeline (fast spheres, moving obstacles, convex bodies):
+#  res_pairs_kernel: xr (32) and v, w (2 R4) of every particle; for each of the
+#   z/2 contacts the pair (16) and its constants (32) in, its state (1) in, six of
+#   its memory's numbers (24 B / 48 B) in and out; the results of the z entries
+#   (2 R4 each) out.  Listed pairs that do not touch, the obstacles and the cell
+#   counts come on top and are not counted.
+#  res_sums_kernel: list place, mark, meta, md, obstacle states, cell key (8 + 1 +
+#   16 + 32 + 8 + 4), xr, q, the listed position (96), v, wbf, inertia (3 R4) and
+#   the z results (2 R4 each) in; xr, q (64), v, w, wbf (3 R4), key and count (8) out.
+#   The list walk runs only where a list is rebuilt and has no fixed bytes.
 #  contacts_kernel: own position+radius (32), meta (16) and cell key (4), the
 #   9 cell-row ranges (72), list length (4) in/out; z list entries (4 z) and
 #   z/2 work items (8 z/2) out.  Neighbour positions are re-read from L1/L2
@@ -68,6 +75,10 @@ def kernel_bytes(kernel, precision, z, basis=False):
         return 32 + 16 + 4 + 72 + 4 + 4 * z + 8 * z / 2.0
     if kernel == "pairs":
         return 84 + 2 * r4 + 4 * z + 8 * z / 2.0 + 2 * (z / 2.0) * entry + 2 * r4 * z
+    if kernel == "res_pairs":
+        return 32 + 2 * r4 + (z / 2.0) * (16 + 32 + 1 + 3 * r4) + 2 * r4 * z
+    if kernel == "res_sums":
+        return 69 + 96 + 3 * r4 + 2 * r4 * z + 64 + 3 * r4 + 8
     kick = (32 + 32 + 16 + 32 + 6 * r4) + (64 + 3 * r4 + 8) + (144 if basis else 0)
     sums = 56 + 4 * z + 2 * r4 * z + 2 * r4 + 8 + (z / 2.0) * entry
     if kernel == "sums":
@@ -375,28 +386,29 @@ def profile_run(sim, sc, n_steps, t):
     return tp, {k: v[0] / n_steps for k, v in prof.items()}, {k: v for k, v in prof.items()}
 
 
-def roofline(prof_tot, sc, precision, z, peak, peak_kind, traffic_of, resident):
+def roofline(prof_tot, sc, precision, z, peak, peak_kind, traffic_of):
     from pacific_b200 import scenarios as S
+    resident = on_resident_lists(prof_tot)
     phases = ["pairs", "sums_kick"] if resident else ["contacts", "pairs", "sums", "sums_kick", "kick_move"]
     dom = max([k for k in phases if k in prof_tot],
               key=lambda k: prof_tot[k][0])
     k_ms, k_n = prof_tot[dom]
     basis = any(sc.shapes[k][0] != S.SPHERE for k in set(np.asarray(sc.particles["shape"]).tolist()))
-    alg = sc.n * kernel_bytes(dom, precision, z, basis)
+    name = {"pairs": "res_pairs", "sums_kick": "res_sums"}[dom] if resident else dom
+    alg = sc.n * kernel_bytes(name, precision, z, basis)
     achieved = alg / (k_ms / k_n / 1e3) / 1e9
     # with convex bodies the pair phase also holds the GJK kernels (their runs
     # are bound by divergence and FP64 latency, not by these bytes)
-    kernel = "pair phase: gjk_count, gjk_place, gjk_kernel, pairs_kernel" if basis and dom == "pairs" else dom + "_kernel"
-    if resident:
-        kernel = {"pairs": "res_pairs_kernel", "sums_kick": "res_sums_kernel"}[dom]
+    kernel = "pair phase: gjk_count, gjk_place, gjk_kernel, pairs_kernel" if basis and dom == "pairs" else name + "_kernel"
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-            "traffic": traffic_of(kernel[:-len("_kernel")] if resident else dom), "kernel": kernel, "peak_source": peak_kind,
+            "traffic": traffic_of(name), "kernel": kernel, "peak_source": peak_kind,
             "algorithmic_bytes_per_launch": alg, "mean_coordination": z, "launch_ms": k_ms / k_n}
 
 
-def on_resident_lists(sim):
-    """Steps on resident pair lists take three launches, all others at least six."""
-    return sim.launches_per_step() == 3
+def on_resident_lists(prof_tot):
+    """Whether the profiled steps ran on resident pair lists: only the last one
+    launches the contact lists then."""
+    return prof_tot["contacts"][1] < prof_tot["pairs"][1]
 
 
 def mean_coordination(sim, sc, t):
@@ -489,7 +501,6 @@ def settled_leg(args, lib, sc, local, flush, peak, peak_kind):
     gst = sm.stats()  # of that one force evaluation
     with nvtx("settled_kernels"):
         _, per_step, tot = profile_run(sm, sc, 500, tm)
-    lists = on_resident_lists(sm)
     sm.close()
     s64, _, ms_64 = run(FP64)
     s64.close()
@@ -500,7 +511,7 @@ def settled_leg(args, lib, sc, local, flush, peak, peak_kind):
                 "fp64": {"value": v_64, "ms_per_dem_step": ms_64 / steps, "mixed_over_fp64": v_m / v_64},
                 "kernels_ms_per_dem_step": per_step,
                 "roofline": roofline(tot, sc, "mixed", z, peak, peak_kind,
-                                     lambda k: profiled_traffic(k, sc.name + "_settled", "mixed"), lists),
+                                     lambda k: profiled_traffic(k, sc.name + "_settled", "mixed")),
                 "contact_force_error": contact_force_error(lib, sc, sc2.particles, mem, local,
                                                            "the settled bed read back from its reload file")})
     if gst["n_gjk_calls"]:
@@ -687,8 +698,11 @@ def main():
     e2e_value = total_particles * args.chunk / e2e_s
     # per middle step; the launched pipeline's permutations on top (the starts and
     # ends of resident runs are not counted)
-    launches = sim.launches_per_step() * args.chunk * args.steps
-    if not on_resident_lists(sim):
+    per_step = sim.launches_per_step()
+    if per_step == 3 and not on_resident_lists(prof_tot):
+        per_step = 6  # spheres too fast for the lists
+    launches = per_step * args.chunk * args.steps
+    if not on_resident_lists(prof_tot):
         launches += (args.chunk * args.steps) // sim.tuning()["gather_every"]
 
     line = {
@@ -703,7 +717,7 @@ def main():
                    "l2": "flushed (256 MiB write) between timed steps"},
         "gpu_launches": int(launches),
         "roofline": roofline(prof_tot, sc, args.precision, z, peak, peak_kind,
-                             lambda k: profiled_traffic(k, sc.name, args.precision), on_resident_lists(sim)),
+                             lambda k: profiled_traffic(k, sc.name, args.precision)),
         "e2e": {"value": e2e_value, "unit": "particle-steps/s", "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h), "host_buffers": "pinned", "over_device": e2e_value / value},
         "kernels_ms_per_dem_step": {k: v[0] / n_prof for k, v in prof_tot.items()},

@@ -78,7 +78,8 @@ typedef struct grains_gpu_config {
   int32_t precision;          /* enum grains_gpu_precision */
   int32_t device;             /* CUDA device ordinal */
   int32_t n_systems;          /* independent systems in one context (>=1) */
-  int32_t history_capacity;   /* contact-memory slots per particle, 0 = 24 */
+  int32_t history_capacity;   /* contact-memory slots per particle, 0 = 24 (below half the list capacity spheres
+                                 take no resident pair lists: grains_gpu_launches_per_step) */
   int64_t max_particles;      /* capacity summed over systems */
   int32_t max_obstacles;      /* capacity summed over systems, 0 = 256 */
   int32_t max_shapes;         /* shape-table capacity, 0 = 64 */
@@ -438,7 +439,8 @@ int grains_gpu_reset_stats(grains_gpu_ctx* ctx);
  *                  a force evaluation; a particle with more fails the step
  *                  with GRAINS_GPU_PAIR_OVERFLOW (resident pair lists that
  *                  no longer fit leave the state at the last step whose
- *                  lists did)
+ *                  lists did).  Spheres step on resident pair lists only
+ *                  with 24 to twice history_capacity slots
  *   gather_every   steps between two permutations of the particle arrays
  *                  into cell order (1 .. 64); in between the cell lists are
  *                  rebuilt every step and reached through a permutation.
