@@ -27,17 +27,16 @@
 
 // control words
 enum {
-  kResRequest = 0, kResFailed = 1, kResRowPairs = 2, kResValid = 3, kResObs = 4, kResCountAll = 6, kResWords = 8
+  kResRequest = 0, kResFailed = 1, kResRowPairs = 2, kResValid = 3, kResObs = 4, kResCountAll = 6
 };
 // kResRequest: 0 lists are good, 1 a particle has moved half the skin, other
 // values: first build of a run (the memory rows are current)
 // kResFailed: the contacts did not fit in the lists; the run stands still from
 // that step on.  kResRowPairs: the rows hold the pairs' memories, not the
-// obstacles' (a rebuild that has not ended)
-// kResValid: pairs of a
-// complete build, else -1; kResObs, kResObs + 1: obstacle items of the steps of
-// even and odd parity; kResCountAll: the step's candidate pairs are counted over
-// all cells, not from the step before
+// obstacles' (a rebuild that has not ended).  kResValid: pairs of a complete build,
+// else -1; kResObs, kResObs + 1: obstacle items of the steps of even and odd
+// parity; kResCountAll: the step's candidate pairs are counted over all cells, not
+// from the step before
 
 // the state of a listed pair or of a particle's obstacle
 enum { kResContact = 1, kResMemory = 2, kResCandidate = 4 };
