@@ -405,16 +405,20 @@ __device__ __forceinline__ V3<R> gather_one(const StepArgs<R>& a, int t, int gat
 template <typename R>
 __global__ void __launch_bounds__(256) gather_kernel(StepArgs<R> a, int gather_forces) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned seen = a.pace ? *(volatile unsigned*)a.pace : 0xffffffffu;
+  __shared__ unsigned most;
+  if (threadIdx.x == 0) most = 0;
   unsigned word = 0;
   if (t < a.n) {
     const float v2 = (float)norm2(gather_one(a, t, gather_forces));
     word = __float_as_uint(v2 <= 3.e38f ? v2 : INFINITY) | 0x80000000u;
   }
-  // few warps exceed what others have found: no queue of atomics
-  if (!__any_sync(0xffffffffu, word > seen)) return;
+  if (!a.pace) return;
+  // a queue of one word per block at most: few exceed what others have found
   word = __reduce_max_sync(0xffffffffu, word);
-  if ((threadIdx.x & 31) == 0) atomicMax(a.pace, word);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) atomicMax(&most, word);
+  __syncthreads();
+  if (threadIdx.x == 0 && most > *(volatile unsigned*)a.pace) atomicMax(a.pace, most);
 }
 
 // ---------------------------------------------------------------------------
