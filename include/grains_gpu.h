@@ -508,8 +508,9 @@ int grains_gpu_set_barrier_test(grains_gpu_ctx* ctx, int64_t polls, int32_t skip
  * cells no smaller than the system's largest diameter, radii within a factor of 4,
  * a list capacity of 24 to twice the history capacity, and persistent = 0; and
  * while the fastest sphere takes at least 3 steps (above 30,000 particles 4, few
- * contacts: up to 8) for a tenth of the smallest radius, by the speeds that the last
- * call before (other than grains_gpu_step, which does not wait) has seen.  Beyond that the launched steps are the faster ones;
+ * contacts: up to 8) for a tenth of the smallest radius.  The speed is that of the
+ * last upload, update or grains_gpu_step, once a call that waits for the device (any
+ * but grains_gpu_step) has read it.  Beyond that the launched steps are the faster ones;
  * the results are the same, and this count does not look at the speeds.
  * Otherwise: the cell sort (3:
  * the tile-local scan, the scatter, the cell sort), contacts, the GJK phase of

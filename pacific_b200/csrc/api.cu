@@ -783,15 +783,20 @@ int with_args(grains_gpu_ctx* c, F f) {
 }
 
 // Cell ranges and permutation of the current positions; with gather the
-// particle arrays are also permuted into cell order (other buffer).
-int sort_now(grains_gpu_ctx* c, int gather_forces, bool gather = true) {
+// particle arrays are also permuted into cell order (other buffer), and their
+// largest speed is taken along for the next step call (speed; hosts that call the
+// phases one by one take none).
+int sort_now(grains_gpu_ctx* c, int gather_forces, bool gather = true, bool speed = true) {
   int rc = 0;
   if (!c->keys_valid) {
     CK(cudaMemsetAsync(c->cell_count, 0, (size_t)c->n_cells * sizeof(int), c->stream));
     rc = with_args(c, [&](auto& a) { return launch_bin(a, c->stream); });
     if (rc) return fail(c, rc, "bin kernel launch failed");
   }
-  rc = with_args(c, [&](auto& a) { return launch_sort_and_gather(a, c->stream, gather ? 1 : 0, gather_forces); });
+  rc = with_args(c, [&](auto& a) {
+    if (!speed) a.pace = nullptr;
+    return launch_sort_and_gather(a, c->stream, gather ? 1 : 0, gather_forces);
+  });
   if (rc) return fail(c, rc, "sort kernels launch failed");
   if (gather) {
     c->cur = 1 - c->cur;
@@ -2525,7 +2530,7 @@ int grains_gpu_link_update(grains_gpu_ctx* c, double time, double dt) {
   if (!c) return GRAINS_GPU_INVALID_ARGUMENT;
   if (!c->uploaded) return fail(c, GRAINS_GPU_NOT_READY, "no particles uploaded");
   if (!c->sorted)
-    if (int rc = sort_now(c, 1)) return rc;
+    if (int rc = sort_now(c, 1, true, false)) return rc;
   return finish_call(c);
 }
 
